@@ -1188,7 +1188,7 @@ __global__ void __launch_bounds__(256) shadow_draw_kernel(ShadowArgs a)
 // a time: lane i takes the 32-row chunk's first line_inv_z and adds dy i times, which is the
 // reference's sequential row accumulation; the next chunk starts from lane 31's value plus dy.
 constexpr int SHADOW_VIEW_WARPS = 8;
-constexpr uint32_t SHADOW_VIEW_SMEM_LEAFS = 8192; // leaf starts staged in shared memory up to this many
+constexpr uint32_t SHADOW_VIEW_SMEM_LEAFS = 4096; // leaf starts staged in shared memory up to this many
 
 struct ShadowWarpShared
 {
@@ -1196,6 +1196,10 @@ struct ShadowWarpShared
 	SwVertex16 v[SW_MAX_POLYGON_VERTICES];
 	RasterPart parts[SW_RASTER_MAX_PARTS];
 };
+// Above 48 KB together the launch needs an opt-in, without which the occupancy query answers 0 CTAs per SM: the
+// grid was then one CTA for every candidate of the frame (5.3 ms for 21,557 candidates of 25 sides; 31 us with
+// the 608 CTAs that fit).
+static_assert(SHADOW_VIEW_WARPS * sizeof(ShadowWarpShared) + SHADOW_VIEW_SMEM_LEAFS * 4 <= 48 * 1024, "shared memory of shadow_view_kernel");
 
 __global__ void __launch_bounds__(SHADOW_VIEW_WARPS * 32) shadow_view_kernel(ShadowViewArgs a)
 {
@@ -1275,7 +1279,7 @@ int launch_shadow_maps(const ShadowArgs& args, cudaStream_t stream)
 int launch_shadow_view(const ShadowViewArgs& args, cudaStream_t stream)
 {
 	if (args.num_candidates == 0) return 0;
-	const size_t smem = args.num_leafs <= SHADOW_VIEW_SMEM_LEAFS ? size_t(args.num_leafs) * 4 : 0; // + 16 KB static < 48 KB
+	const size_t smem = args.num_leafs <= SHADOW_VIEW_SMEM_LEAFS ? size_t(args.num_leafs) * 4 : 0; // with the static part < 48 KB
 	// resident CTAs of the largest staging (registers bound it first), once per device; concurrent first
 	// calls compute the same value, so a relaxed atomic store is enough
 	constexpr int MAX_DEVICES = 64;
