@@ -1125,6 +1125,75 @@ __device__ __forceinline__ float depth_first_line(const RasterPart& p, float dx,
 	return fadd(fadd(fmul(float(p.y_start_int), dy), fmul(0.5f, fadd(dx, dy))), k);
 }
 
+// A part of at most this many texels (rows x widest row) is drawn by the warp that prepared it, one row per
+// lane; a larger one goes to the chunk list: a lane's row is a serial chain of as many steps as the row has
+// texels, each an atomic on a sector of its own, and one warp would run a wall that fills a 1024 x 1024 map
+// alone. With the list a 1920x1080 frame with 4 shadowed lights and a projector takes 136 us instead of 146 us;
+// lines at 256, 512, 2048 and 4096 texels measured the same within 1%.
+constexpr uint32_t SHADOW_DIRECT_TEXELS = 1024;
+
+// The parts of one depth draw, by the warp that walked its edges (the same arguments in every lane). Rows go
+// to lanes 32 at a time: lane i takes the 32-row chunk's first line_inv_z and adds dy i times, which is the
+// reference's sequential row accumulation; the next chunk starts from lane 31's value plus dy.
+__device__ __forceinline__ void emit_depth_parts(const RasterPart* parts, uint32_t np, const float eq[3], uint32_t seq, int32_t size,
+	uint64_t map_offset, unsigned long long* storage, const ShadowChunks& list)
+{
+	const uint32_t lane = threadIdx.x & 31u;
+	const float dx = eq[0], dy = eq[1], k = eq[2];
+	for (uint32_t pi = 0; pi < np; ++pi)
+	{
+		const RasterPart pt = parts[pi];
+		const uint32_t rows = uint32_t(pt.y_end_int - pt.y_start_int);
+		float chunk = depth_first_line(pt, dx, dy, k);
+		// x is linear in the row, so the widest row is the first or the last
+		const int32_t last = int32_t(rows) - 1;
+		const int32_t w0 = min(pt.x_right0 >> 16, size) - max(pt.x_left0 >> 16, 0);
+		const int32_t w1 = min(wadd(pt.x_right0, wmul(last, pt.dx_dy_right)) >> 16, size) -
+			max(wadd(pt.x_left0, wmul(last, pt.dx_dy_left)) >> 16, 0);
+		const uint32_t n = (rows + 31) / 32;
+		uint32_t at = list.capacity;
+		if (uint64_t(rows) * uint32_t(max(max(w0, w1), 0)) > SHADOW_DIRECT_TEXELS)
+		{
+			if (lane == 0) at = atomicAdd(list.count, n);
+			at = __shfl_sync(FULL_MASK, at, 0);
+			if (at + n > list.capacity || at + n < at)
+			{
+				// no room: the reserved tail of the list is left empty and the part drawn here
+				for (uint32_t i = at + lane; i < list.capacity && i < at + n; i += 32) list.items[i].rows = 0;
+				at = list.capacity;
+			}
+		}
+		for (uint32_t r0 = 0; r0 < rows; r0 += 32)
+		{
+			float line = chunk;
+			for (uint32_t i = 0; i < lane; ++i) line = fadd(line, dy);
+			if (at < list.capacity)
+			{
+				if (lane == 0)
+				{
+					ShadowChunk c;
+					c.map_offset = map_offset;
+					c.seq = seq;
+					c.size = size;
+					c.y0 = pt.y_start_int + int32_t(r0);
+					c.rows = min(rows - r0, 32u);
+					c.x_left0 = wadd(pt.x_left0, wmul(int32_t(r0), pt.dx_dy_left));
+					c.x_right0 = wadd(pt.x_right0, wmul(int32_t(r0), pt.dx_dy_right));
+					c.dx_dy_left = pt.dx_dy_left;
+					c.dx_dy_right = pt.dx_dy_right;
+					c.line = chunk;
+					c.dx = dx;
+					c.dy = dy;
+					list.items[at + r0 / 32] = c;
+				}
+			}
+			else if (r0 + lane < rows)
+				draw_depth_row(storage + map_offset, size, pt, r0 + lane, line, dx, (unsigned long long)(seq) << 32);
+			chunk = fadd(__shfl_sync(FULL_MASK, line, 31), dy);
+		}
+	}
+}
+
 } // namespace
 
 __global__ void shadow_rebase_kernel(unsigned long long* storage, uint64_t n)
@@ -1133,60 +1202,6 @@ __global__ void shadow_rebase_kernel(unsigned long long* storage, uint64_t n)
 		storage[i] &= 0xFFFFFFFFull;
 }
 
-// Host-prepared depth draws (sw_build_shadow_maps), one per CTA: thread 0 walks the edges (the colour
-// rasteriser's walk: the same parts and first-row edge positions) and accumulates each part's per-row
-// inverse depth in the reference's sequential order; then one thread per row accumulates along its span.
-__global__ void __launch_bounds__(256) shadow_draw_kernel(ShadowArgs a)
-{
-	__shared__ __align__(8) SwDrawCmd s_d;
-	__shared__ SwVertex16 s_v[SW_MAX_POLYGON_VERTICES];
-	__shared__ RasterPart s_parts[SW_RASTER_MAX_PARTS];
-	__shared__ float s_line[SW_SHADOW_MAX_SIZE];
-	__shared__ uint32_t s_np;
-	for (uint32_t di = blockIdx.x; di < a.num_draws; di += gridDim.x)
-	{
-		const SwDepthDraw dd = a.draws[di];
-		const int32_t size = int32_t(dd.map_size);
-		if (threadIdx.x == 0)
-		{
-			s_d = SwDrawCmd{};
-			s_d.vertex_count = dd.vertex_count;
-			s_d.mode = SW_RASTER_FULL_PERSPECTIVE; // no texture-coordinate edges
-		}
-		if (threadIdx.x < dd.vertex_count) s_v[threadIdx.x] = a.vertices[dd.first_vertex + threadIdx.x];
-		__syncthreads();
-		if (threadIdx.x == 0) s_np = edge_walk(s_d, s_v, size, s_parts);
-		__syncthreads();
-		const float dx = dd.depth_eq[0], dy = dd.depth_eq[1], k = dd.depth_eq[2];
-		const unsigned long long seq = (unsigned long long)(a.seq_base + di + 1u) << 32;
-		unsigned long long* map = a.storage + dd.map_offset;
-		for (uint32_t pi = 0; pi < s_np; ++pi)
-		{
-			const RasterPart p = s_parts[pi];
-			const uint32_t rows = uint32_t(p.y_end_int - p.y_start_int); // <= size <= SW_SHADOW_MAX_SIZE
-			if (threadIdx.x == 0)
-			{
-				float line = depth_first_line(p, dx, dy, k);
-				for (uint32_t r = 0; r < rows; ++r)
-				{
-					s_line[r] = line;
-					line = fadd(line, dy);
-				}
-			}
-			__syncthreads();
-			for (uint32_t r = threadIdx.x; r < rows; r += blockDim.x) draw_depth_row(map, size, p, r, s_line[r], dx, seq);
-			__syncthreads(); // s_line is reused by the next part
-		}
-	}
-}
-
-// GPU-prepared depth draws (sw_build_shadow_maps_view): every polygon of every listed leaf is one warp,
-// which prepares it (DepthRenderer::draw_polygon::<false> + draw_depth_polygon, depth_renderer.rs:
-// 199-287: the shared depth_map_equation, the view transform, the warp-cooperative
-// project_and_clip_polygon, f32_to_fixed16) and draws it at once. The candidate's index in the leaf
-// list's polygon order is its painter's-order sequence, so nothing is compacted. Rows go to lanes 32 at
-// a time: lane i takes the 32-row chunk's first line_inv_z and adds dy i times, which is the
-// reference's sequential row accumulation; the next chunk starts from lane 31's value plus dy.
 constexpr int SHADOW_VIEW_WARPS = 8;
 constexpr uint32_t SHADOW_VIEW_SMEM_LEAFS = 4096; // leaf starts staged in shared memory up to this many
 
@@ -1201,6 +1216,39 @@ struct ShadowWarpShared
 // the 608 CTAs that fit).
 static_assert(SHADOW_VIEW_WARPS * sizeof(ShadowWarpShared) + SHADOW_VIEW_SMEM_LEAFS * 4 <= 48 * 1024, "shared memory of shadow_view_kernel");
 
+// Host-prepared depth draws (sw_build_shadow_maps), one per warp: lane 0 walks the edges (the colour
+// rasteriser's walk: the same parts and first-row edge positions), then the warp draws or lists the parts.
+__global__ void __launch_bounds__(SHADOW_VIEW_WARPS * 32) shadow_draw_kernel(ShadowArgs a)
+{
+	__shared__ SwVertex16 s_v[SHADOW_VIEW_WARPS][SW_MAX_POLYGON_VERTICES];
+	__shared__ RasterPart s_parts[SHADOW_VIEW_WARPS][SW_RASTER_MAX_PARTS];
+	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+	for (uint32_t di = blockIdx.x * SHADOW_VIEW_WARPS + warp; di < a.num_draws; di += gridDim.x * SHADOW_VIEW_WARPS)
+	{
+		__syncwarp(); // the previous draw's reads are done
+		const SwDepthDraw dd = a.draws[di];
+		if (lane < dd.vertex_count) s_v[warp][lane] = a.vertices[dd.first_vertex + lane];
+		__syncwarp();
+		uint32_t np = 0;
+		if (lane == 0)
+		{
+			SwDrawCmd d{};
+			d.vertex_count = dd.vertex_count;
+			d.mode = SW_RASTER_FULL_PERSPECTIVE; // no texture-coordinate edges
+			np = edge_walk(d, s_v[warp], int32_t(dd.map_size), s_parts[warp]);
+		}
+		np = __shfl_sync(FULL_MASK, np, 0);
+		__syncwarp();
+		emit_depth_parts(s_parts[warp], np, dd.depth_eq, a.seq_base + di + 1u, int32_t(dd.map_size), dd.map_offset, a.storage, a.chunks);
+	}
+	pdl_trigger();
+}
+
+// GPU-prepared depth draws (sw_build_shadow_maps_view): every polygon of every listed leaf is one warp,
+// which prepares it (DepthRenderer::draw_polygon::<false> + draw_depth_polygon, depth_renderer.rs:
+// 199-287: the shared depth_map_equation, the view transform, the warp-cooperative
+// project_and_clip_polygon, f32_to_fixed16) and draws or lists its parts at once. The candidate's index in
+// the leaf list's polygon order is its painter's-order sequence, so nothing is compacted.
 __global__ void __launch_bounds__(SHADOW_VIEW_WARPS * 32) shadow_view_kernel(ShadowViewArgs a)
 {
 	__shared__ ShadowWarpShared s_w[SHADOW_VIEW_WARPS];
@@ -1251,29 +1299,83 @@ __global__ void __launch_bounds__(SHADOW_VIEW_WARPS * 32) shadow_view_kernel(Sha
 		}
 		np = __shfl_sync(FULL_MASK, np, 0);
 		__syncwarp();
-		const float dx = eq[0], dy = eq[1], k = eq[2];
-		const unsigned long long seq = (unsigned long long)(a.seq_base + c + 1u) << 32;
-		unsigned long long* map = a.storage + side.map_offset;
-		for (uint32_t pi = 0; pi < np; ++pi)
+		emit_depth_parts(sw.parts, np, eq, a.seq_base + c + 1u, size, side.map_offset, a.storage, a.chunks);
+	}
+	pdl_trigger();
+}
+
+// The listed chunks of large parts (up to 32 rows each), one per warp over a persistent grid. inv_z is the
+// reference's pixel-by-pixel accumulation, a serial chain along each row, so each lane runs its own row's chain
+// (32 texels at a time, into shared memory) and the warp then writes the 32 rows one after another, 32
+// neighbouring texels per atomic instruction. Bound by the atomics' rate in L2 and, for few chunks, by one
+// chunk's chain. The last CTA empties the list for the next call.
+__global__ void __launch_bounds__(SHADOW_VIEW_WARPS * 32) shadow_chunk_kernel(ShadowChunks list, unsigned long long* storage)
+{
+	__shared__ uint32_t s_tile[SHADOW_VIEW_WARPS][32][33];
+	__shared__ uint32_t s_last;
+	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+	pdl_wait(); // the chunks are listed
+	const uint32_t count = min(*list.count, list.capacity);
+	for (uint32_t i = warp * gridDim.x + blockIdx.x; i < count; i += gridDim.x * SHADOW_VIEW_WARPS)
+	{
+		const ShadowChunk& c = list.items[i];
+		const uint32_t rows = c.rows;
+		if (rows == 0) continue;
+		const float dx = c.dx, dy = c.dy;
+		float line = c.line;
+		for (uint32_t k = 0; k < lane; ++k) line = fadd(line, dy);
+		int32_t xs = INT32_MAX, xe = INT32_MIN;
+		if (lane < rows)
 		{
-			const RasterPart pt = sw.parts[pi];
-			const uint32_t rows = uint32_t(pt.y_end_int - pt.y_start_int);
-			float chunk = depth_first_line(pt, dx, dy, k);
-			for (uint32_t r0 = 0; r0 < rows; r0 += 32)
+			xs = max(wadd(c.x_left0, wmul(int32_t(lane), c.dx_dy_left)) >> 16, 0);
+			xe = min(wadd(c.x_right0, wmul(int32_t(lane), c.dx_dy_right)) >> 16, c.size);
+			if (xs >= xe) xs = INT32_MAX, xe = INT32_MIN;
+		}
+		const int32_t x_lo = __reduce_min_sync(FULL_MASK, xs), x_hi = __reduce_max_sync(FULL_MASK, xe);
+		float inv_z = xs < xe ? fadd(line, fmul(float(xs), dx)) : 0.0f;
+		const unsigned long long seq = (unsigned long long)(c.seq) << 32;
+		const uint64_t pitch = uint32_t(c.size);
+		unsigned long long* map = storage + c.map_offset + uint64_t(c.y0) * pitch;
+		for (int32_t x0 = x_lo & ~31; x0 < x_hi; x0 += 32)
+		{
+			__syncwarp(); // the tile's previous texels are written
+#pragma unroll
+			for (int j = 0; j < 32; ++j)
 			{
-				float line = chunk;
-				for (uint32_t i = 0; i < lane; ++i) line = fadd(line, dy);
-				if (r0 + lane < rows) draw_depth_row(map, size, pt, r0 + lane, line, dx, seq);
-				chunk = fadd(__shfl_sync(FULL_MASK, line, 31), dy);
+				const bool in = x0 + j >= xs && x0 + j < xe;
+				s_tile[warp][lane][j] = __float_as_uint(inv_z);
+				if (in) inv_z = fadd(inv_z, dx);
+			}
+			__syncwarp();
+			for (uint32_t r = 0; r < rows; ++r)
+			{
+				const int32_t rs = __shfl_sync(FULL_MASK, xs, int(r)), re = __shfl_sync(FULL_MASK, xe, int(r));
+				const int32_t x = x0 + int32_t(lane);
+				if (x >= rs && x < re) atomicMax(map + r * pitch + uint32_t(x), seq | s_tile[warp][r][lane]);
 			}
 		}
 	}
+	__syncthreads(); // every warp of the CTA has read the count
+	if (threadIdx.x == 0) s_last = atomicAdd(list.count + 1, 1u) == gridDim.x - 1 ? 1u : 0u;
+	__syncthreads();
+	if (s_last && threadIdx.x == 0) list.count[0] = list.count[1] = 0u;
 }
+
+namespace
+{
+int launch_shadow_chunks(const ShadowChunks& list, unsigned long long* storage, cudaStream_t stream)
+{
+	// three CTAs of eight warps per SM (34 KB of tiles each): one chunk per warp for 3,648 chunks
+	return int(launch_dependent(shadow_chunk_kernel, dim3(list.num_sms * 3), dim3(SHADOW_VIEW_WARPS * 32), 0, stream, list, storage));
+}
+} // namespace
 
 int launch_shadow_maps(const ShadowArgs& args, cudaStream_t stream)
 {
-	if (args.num_draws > 0) shadow_draw_kernel<<<std::min(args.num_draws, 65535u), 256, 0, stream>>>(args);
-	return int(cudaGetLastError());
+	if (args.num_draws == 0) return 0;
+	shadow_draw_kernel<<<std::min((args.num_draws + SHADOW_VIEW_WARPS - 1) / SHADOW_VIEW_WARPS, 65535u), SHADOW_VIEW_WARPS * 32, 0, stream>>>(args);
+	if (int e = int(cudaGetLastError())) return e;
+	return launch_shadow_chunks(args.chunks, args.storage, stream);
 }
 
 int launch_shadow_view(const ShadowViewArgs& args, cudaStream_t stream)
@@ -1301,7 +1403,8 @@ int launch_shadow_view(const ShadowViewArgs& args, cudaStream_t stream)
 	}
 	const uint32_t blocks = std::min<uint32_t>((args.num_candidates + SHADOW_VIEW_WARPS - 1) / SHADOW_VIEW_WARPS, uint32_t(resident));
 	shadow_view_kernel<<<blocks, SHADOW_VIEW_WARPS * 32, smem, stream>>>(args);
-	return int(cudaGetLastError());
+	if (int e2 = int(cudaGetLastError())) return e2;
+	return launch_shadow_chunks(args.chunks, args.storage, stream);
 }
 
 namespace

@@ -313,6 +313,26 @@ __host__ __device__ inline void draw_row_range(const SwDrawCmd& d, const SwVerte
 
 // ---- shadow maps ----
 
+// Up to 32 rows of a large part of a depth draw (the edges and line_inv_z of its first row): what one warp of
+// shadow_chunk_kernel draws.
+struct ShadowChunk
+{
+	uint64_t map_offset;
+	uint32_t seq;
+	int32_t size;
+	int32_t y0;
+	uint32_t rows;
+	int32_t x_left0, x_right0, dx_dy_left, dx_dy_right;
+	float line, dx, dy;
+};
+#define SW_SHADOW_CHUNKS 32768u // 2 MB; parts that find the list full are drawn by the warp that prepared them
+struct ShadowChunks
+{
+	ShadowChunk* items;
+	uint32_t* count; // [0] chunks listed, [1] finished CTAs of shadow_chunk_kernel; both 0 between calls
+	uint32_t capacity;
+	uint32_t num_sms;
+};
 
 struct ShadowArgs
 {
@@ -321,6 +341,7 @@ struct ShadowArgs
 	uint32_t seq_base;               // draw i writes sequence seq_base + i + 1 (< 2^32)
 	const SwVertex16* vertices;
 	unsigned long long* storage;     // the persistent storage: (sequence << 32 | f32 bits) per texel
+	ShadowChunks chunks;
 };
 // Draw every depth draw into the storage (last draw wins per texel).
 int launch_shadow_maps(const ShadowArgs& args, cudaStream_t stream);
@@ -337,6 +358,7 @@ struct ShadowViewArgs
 	const float* map_vertices;
 	unsigned long long* storage;
 	uint32_t seq_base;
+	ShadowChunks chunks;
 };
 int launch_shadow_view(const ShadowViewArgs& args, cudaStream_t stream);
 // make_shadow_map_circle on the size x size projector map at `map` with sequence `seq`.

@@ -198,7 +198,7 @@ struct SwCtx
 
 	// Shadow maps (sw_build_shadow_maps / sw_set_light_shadows): the persistent f32 storage (grows, keeps
 	// its contents), the packing scratch, and the frame's per-light descriptors on the device.
-	DevBuf shadow_storage, shadow_descs;
+	DevBuf shadow_storage, shadow_descs, shadow_chunks;
 	uint32_t shadow_seq = 0; // the next depth draw's sequence base (the storage's high words)
 	uint64_t shadow_texels = 0;
 	uint32_t num_shadow_descs = 0;
@@ -647,7 +647,7 @@ int sw_destroy(SwCtx* ctx)
 		&ctx->dir_lightmaps, &ctx->lights, &ctx->surfaces, &ctx->work_prefix, &ctx->arena, &ctx->draws, &ctx->vertices,
 		&ctx->draw_rows, &ctx->rdraws, &ctx->rows, &ctx->boxes, &ctx->tri_steps, &ctx->tri_vertices, &ctx->lite, &ctx->ldr[0], &ctx->ldr[1], &ctx->framebuffer, &ctx->bloom0, &ctx->bloom1, &ctx->line_sums,
 		&ctx->line_sums_f, &ctx->average, &ctx->error_counter, &ctx->up_src, &ctx->up_dst, &ctx->map_polygons,
-		&ctx->map_vertices, &ctx->vslab, &ctx->shadow_storage, &ctx->shadow_descs, &ctx->effect_buf, &ctx->sim_state, &ctx->sim_buf, &ctx->vbin_lists,
+		&ctx->map_vertices, &ctx->vslab, &ctx->shadow_storage, &ctx->shadow_descs, &ctx->shadow_chunks, &ctx->effect_buf, &ctx->sim_state, &ctx->sim_buf, &ctx->vbin_lists,
 		&ctx->vbin_counts};
 	for (DevBuf* b : bufs) release(*b);
 	for (const SwCtx::HostRange& h : ctx->registered) cudaHostUnregister(h.ptr);
@@ -2686,6 +2686,30 @@ int grow_shadow_storage(SwCtx* ctx, uint64_t total_texels)
 	return SW_OK;
 }
 
+// The list of large parts' chunks, empty (its counters zeroed before its first use; every later call leaves
+// them zero).
+int shadow_chunk_list(SwCtx* ctx, ShadowChunks* list)
+{
+	const size_t items = size_t(SW_SHADOW_CHUNKS) * sizeof(ShadowChunk);
+	const bool fresh = !ctx->shadow_chunks.ptr;
+	int r = ensure(ctx, ctx->shadow_chunks, items + 2 * sizeof(uint32_t));
+	if (r) return r;
+	list->items = static_cast<ShadowChunk*>(ctx->shadow_chunks.ptr);
+	list->count = reinterpret_cast<uint32_t*>(static_cast<unsigned char*>(ctx->shadow_chunks.ptr) + items);
+	list->capacity = SW_SHADOW_CHUNKS;
+	list->num_sms = uint32_t(ctx->num_sms);
+	if (fresh)
+	{
+		const cudaError_t e = cudaMemsetAsync(list->count, 0, 2 * sizeof(uint32_t), ctx->stream);
+		if (e != cudaSuccess)
+		{
+			release(ctx->shadow_chunks);
+			return cuda_fail(ctx, e, "cudaMemsetAsync");
+		}
+	}
+	return SW_OK;
+}
+
 // Sequences of the next `count` depth draws: base + 1 .. base + count, above every sequence in the
 // storage; when they would pass 2^32 - 1 the storage drops its sequences (keeping its depths) first.
 int shadow_sequence(SwCtx* ctx, uint64_t count, uint32_t* base)
@@ -2731,6 +2755,7 @@ int sw_build_shadow_maps(SwCtx* ctx, const SwDepthDraw* draws, uint32_t num_draw
 	if ((r = staging_commit(ctx, ctx->stage_shadow, ctx->up_src.ptr, bytes))) return r;
 	ShadowArgs a;
 	std::memset(&a, 0, sizeof(a));
+	if ((r = shadow_chunk_list(ctx, &a.chunks))) return r;
 	if ((r = shadow_sequence(ctx, num_draws, &a.seq_base))) return r;
 	a.draws = static_cast<const SwDepthDraw*>(ctx->up_src.ptr);
 	a.num_draws = num_draws;
@@ -2786,6 +2811,7 @@ int sw_build_shadow_maps_view(SwCtx* ctx, const SwShadowSide* sides, uint32_t nu
 	unsigned char* db = static_cast<unsigned char*>(ctx->up_src.ptr);
 	ShadowViewArgs a;
 	std::memset(&a, 0, sizeof(a));
+	if ((r = shadow_chunk_list(ctx, &a.chunks))) return r;
 	if ((r = shadow_sequence(ctx, candidates, &a.seq_base))) return r;
 	a.sides = reinterpret_cast<const SwShadowSide*>(db);
 	a.leafs = reinterpret_cast<const SwShadowLeaf*>(db + lo);
