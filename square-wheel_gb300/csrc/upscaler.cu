@@ -1010,16 +1010,14 @@ struct WgradArgs
 {
 	Planes x; // layer input (C8X chunks)
 	Planes g; // pre-activation gradient (NG / 8 chunks)
-	float* partial;    // per CTA: [3 dx][128 rows][NG] then the bias partials [NG]
+	float* partial;    // per CTA: [3 dx][wgrad_rows(C8X)][NG] then the bias partials [NG]
 	uint32_t tiles_x, row_blocks;
 	int* error;
 };
 
-template <int C8X, int NG>
-__host__ __device__ constexpr uint32_t wgrad_partial_floats()
-{
-	return 3 * 128 * NG + NG;
-}
+// The accumulator rows that are taps: (dy, chunk, ci % 8) for dy < 3; the rows above belong to no tap.
+__host__ __device__ constexpr uint32_t wgrad_rows(int c8x) { return 3 * c8x * 8; }
+__host__ __device__ constexpr uint32_t wgrad_partial_floats(int c8x, int ng) { return 3 * wgrad_rows(c8x) * ng + ng; }
 
 template <int C8X, int NG>
 __global__ void __launch_bounds__(128) wgrad_kernel(WgradArgs a)
@@ -1123,10 +1121,11 @@ __global__ void __launch_bounds__(128) wgrad_kernel(WgradArgs a)
 		return;
 	}
 	fence_after_sync();
-	float* out = a.partial + size_t(blockIdx.x) * wgrad_partial_floats<C8X, NG>();
-	const int m = warp * 32 + lane;
+	constexpr uint32_t MR = wgrad_rows(C8X);
+	float* out = a.partial + size_t(blockIdx.x) * wgrad_partial_floats(C8X, NG);
+	const uint32_t m = warp * 32 + lane;
 	const uint32_t lane_base = uint32_t(warp * 32) << 16;
-	for (int d = 0; d < 3; ++d)
+	for (int d = 0; d < 3 && warp * 32 < MR; ++d)
 	{
 #pragma unroll
 		for (int c8 = 0; c8 < G8; ++c8)
@@ -1134,7 +1133,8 @@ __global__ void __launch_bounds__(128) wgrad_kernel(WgradArgs a)
 			float t8[8];
 			tmem_ld8(tmem + lane_base + d * NG + c8 * 8, t8);
 			tmem_ld_wait();
-			float4* o = reinterpret_cast<float4*>(out + (size_t(d) * 128 + m) * NG + c8 * 8);
+			if (m >= MR) continue;
+			float4* o = reinterpret_cast<float4*>(out + (size_t(d) * MR + m) * NG + c8 * 8);
 			o[0] = make_float4(t8[0], t8[1], t8[2], t8[3]);
 			o[1] = make_float4(t8[4], t8[5], t8[6], t8[7]);
 		}
@@ -1144,7 +1144,7 @@ __global__ void __launch_bounds__(128) wgrad_kernel(WgradArgs a)
 		constexpr int PARTS = 128 / NG;
 		float s = 0.0f;
 		for (int q = 0; q < PARTS; ++q) s += s_bias[q * NG + tid];
-		out[3 * 128 * NG + tid] = s;
+		out[3 * MR * NG + tid] = s;
 	}
 	fence_before_sync();
 	__syncthreads();
@@ -1159,34 +1159,6 @@ template <int C8X, int NG>
 __host__ __device__ constexpr uint32_t wgrad_smem_bytes()
 {
 	return (ROWS + 16 / C8X - 1) * C8X * XS_BYTES + ROWS * (NG / 8) * XS_BYTES + 32 + 512;
-}
-
-// Sum the per-CTA partials (fixed order) into canonical gradients of one layer, times `scale`.
-__global__ void wgrad_reduce_kernel(const float* partial, uint32_t num_ctas, uint32_t partial_floats, int layer, int c8x, int ng,
-	float scale, float* grads)
-{
-	const LayerShape L = c_layers[layer];
-	const int nw = L.cout * 9 * L.cin;
-	const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-	if (idx >= nw + L.cout) return;
-	size_t off;
-	if (idx < nw)
-	{
-		int r = idx;
-		const int ci = r % L.cin;
-		r /= L.cin;
-		const int kx = r % 3;
-		r /= 3;
-		const int ky = r % 3;
-		const int co = r / 3;
-		const int m = (ky * c8x + ci / 8) * 8 + ci % 8;
-		off = (size_t(kx) * 128 + m) * ng + co;
-	}
-	else
-		off = size_t(3) * 128 * ng + (idx - nw);
-	float s = 0.0f;
-	for (uint32_t c = 0; c < num_ctas; ++c) s += partial[size_t(c) * partial_floats + off];
-	grads[L.param_offset + idx] = s * scale;
 }
 
 // Input conversion: Color32 window of each crop -> chunk 0 of the row planes (b, g, r, 0...) / 255.
@@ -1221,14 +1193,11 @@ struct AdamArgs
 	float* bias[NUM_LAYERS];
 };
 
-__global__ void adam_pack_kernel(AdamArgs a)
+__device__ __forceinline__ void adam_pack(const AdamArgs& a, int idx, float g)
 {
-	const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-	if (idx >= int(SW_UPSCALER_NUM_PARAMS)) return;
 	float p = a.params[idx];
 	if (a.update)
 	{
-		const float g = a.grads[idx];
 		const float m = a.beta1 * a.m[idx] + (1.0f - a.beta1) * g;
 		const float v = a.beta2 * a.v[idx] + (1.0f - a.beta2) * g * g;
 		a.m[idx] = m;
@@ -1267,6 +1236,77 @@ __global__ void adam_pack_kernel(AdamArgs a)
 		const int ks = co / 16, hh = (co / 8) % 2, e = co % 8;
 		a.wbwd[l][(((2 - kx) * (L.n_out / 16) + ks) * 2 + hh) * (3 * no) * 8 + ((2 - ky) * no + ci) * 8 + e] = h;
 	}
+}
+
+// Repacking without an update (new parameters).
+__global__ void adam_pack_kernel(AdamArgs a)
+{
+	const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+	if (idx < int(SW_UPSCALER_NUM_PARAMS)) adam_pack(a, idx, 0.0f);
+}
+
+// The weight gradients' per-CTA partials of every layer summed (times `scale`) into canonical gradients, and with
+// a.update Adam and the repacking right after, one launch for the four layers. A block takes 32 neighbouring
+// accumulator columns, so a warp reads whole 128-byte lines of a partial; its eight warps take every eighth
+// partial and their sums are added in order, so the result does not depend on the run. Bound by reading the
+// partials from L2 (28 MB at 16 crops). The four sums with one thread per parameter, 256 dependent reads of 4
+// bytes from lines of their own, took 121 us of a 334 us step.
+struct ReduceArgs
+{
+	const float* partial[NUM_LAYERS];
+	uint32_t num_ctas;
+	float scale;
+	float* grads;
+	AdamArgs adam;
+};
+constexpr int REDUCE_WARPS = 8;
+__host__ __device__ constexpr int reduce_items(int l) // accumulator columns of layer l: weights, then biases
+{
+	return 9 * LAYERS[l].cin * LAYERS[l].n_out + LAYERS[l].n_out;
+}
+__host__ __device__ constexpr int reduce_blocks(int l) { return (reduce_items(l) + 31) / 32; }
+__host__ __device__ constexpr int reduce_first(int l) { return l == 0 ? 0 : reduce_first(l - 1) + reduce_blocks(l - 1); }
+
+__global__ void __launch_bounds__(REDUCE_WARPS * 32) wgrad_reduce_kernel(const __grid_constant__ ReduceArgs a)
+{
+	__shared__ float s_sum[REDUCE_WARPS][32];
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	constexpr int F1 = reduce_first(1), F2 = reduce_first(2), F3 = reduce_first(3);
+	const int b = int(blockIdx.x), l = b < F1 ? 0 : b < F2 ? 1 : b < F3 ? 2 : 3;
+	const LayerShape L = c_layers[l];
+	const int item = (b - (l == 0 ? 0 : l == 1 ? F1 : l == 2 ? F2 : F3)) * 32 + lane, nw = 9 * L.cin * L.n_out;
+	const bool valid = item < nw + L.n_out;
+	const uint32_t mr = wgrad_rows(L.c8_in), stride = wgrad_partial_floats(L.c8_in, L.n_out);
+	const int co = item % L.n_out;
+	int idx = -1; // canonical parameter, -1 for the padded output channels
+	uint32_t off = 0;
+	if (item < nw)
+	{
+		const int r = item / L.n_out, ci = r % L.cin, t = r / L.cin, ky = t / 3, kx = t % 3;
+		off = (uint32_t(kx) * mr + uint32_t((ky * L.c8_in + ci / 8) * 8 + ci % 8)) * L.n_out + co;
+		if (co < L.cout) idx = L.param_offset + (co * 9 + t) * L.cin + ci;
+	}
+	else if (valid)
+	{
+		off = 3 * mr * L.n_out + co;
+		if (co < L.cout) idx = L.param_offset + L.cout * 9 * L.cin + co;
+	}
+	float s = 0.0f;
+	if (valid)
+	{
+		const float* p = a.partial[l] + off;
+#pragma unroll 8
+		for (uint32_t c = warp; c < a.num_ctas; c += REDUCE_WARPS) s += __ldg(p + size_t(c) * stride);
+	}
+	s_sum[warp][lane] = s;
+	__syncthreads();
+	if (warp || idx < 0) return;
+	float t = 0.0f;
+#pragma unroll
+	for (int w = 0; w < REDUCE_WARPS; ++w) t += s_sum[w][lane];
+	t *= a.scale;
+	a.grads[idx] = t;
+	if (a.adam.update) adam_pack(a.adam, idx, t);
 }
 
 __global__ void psnr_kernel(const uint32_t* a, uint32_t ap, const uint32_t* b, uint32_t bp, uint32_t w, uint32_t h,
@@ -1329,7 +1369,7 @@ struct SwUpscaler
 	DevMem wfwd[NUM_LAYERS], wbwd[NUM_LAYERS], bias[NUM_LAYERS];
 	DevMem error;
 	// training workspace (SW_UPSCALER_MAX_CROPS crops)
-	DevMem t_x0, t_a[3], t_g4, t_g[3], partial, loss_partial, crops;
+	DevMem t_x0, t_a[3], t_g4, t_g[3], partial[NUM_LAYERS], loss_partial, crops;
 	uint32_t crops_capacity = 0;
 	DevMem h_stage; // pinned: crops + loss partials
 	// inference workspace
@@ -1475,13 +1515,16 @@ int launch_conv(SwUpscaler* u, ConvArgs a, cudaStream_t s)
 	return SW_OK;
 }
 
+constexpr uint32_t WGRAD_CTAS_PER_CROP =
+	(SW_UPSCALER_CROP_W + TILE_X - 1) / TILE_X * ((SW_UPSCALER_CROP_H + ROWS - 1) / ROWS);
+
 template <int C8X, int NG>
-int launch_wgrad(SwUpscaler* u, const Planes& x, const Planes& g, int layer, float scale, cudaStream_t s)
+int launch_wgrad(SwUpscaler* u, const Planes& x, const Planes& g, int layer, cudaStream_t s)
 {
 	WgradArgs a;
 	a.x = x;
 	a.g = g;
-	a.partial = static_cast<float*>(u->partial.ptr);
+	a.partial = static_cast<float*>(u->partial[layer].ptr);
 	a.tiles_x = (x.width + TILE_X - 1) / TILE_X;
 	a.row_blocks = (x.height + ROWS - 1) / ROWS;
 	a.error = static_cast<int*>(u->error.ptr);
@@ -1493,20 +1536,15 @@ int launch_wgrad(SwUpscaler* u, const Planes& x, const Planes& g, int layer, flo
 		UP_CUDA(u, cudaFuncSetAttribute(wgrad_kernel<C8X, NG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
 		configured[key] = true;
 	}
-	const uint32_t blocks = x.images * a.tiles_x * a.row_blocks;
-	if (size_t(blocks) * wgrad_partial_floats<C8X, NG>() * 4 > u->partial.bytes)
+	const uint32_t blocks = x.images * a.tiles_x * a.row_blocks; // images * WGRAD_CTAS_PER_CROP for training crops
+	if (size_t(blocks) * wgrad_partial_floats(C8X, NG) * 4 > u->partial[layer].bytes)
 		return fail(u, SW_ERR_LIMIT, "weight-gradient partial buffer too small");
 	wgrad_kernel<C8X, NG><<<blocks, 128, smem, s>>>(a);
-	UP_CUDA(u, cudaGetLastError());
-	const LayerShape& L = LAYERS[layer];
-	const int n = L.cout * 9 * L.cin + L.cout;
-	wgrad_reduce_kernel<<<(n + 255) / 256, 256, 0, s>>>(static_cast<const float*>(u->partial.ptr), blocks,
-		wgrad_partial_floats<C8X, NG>(), layer, C8X, NG, scale, static_cast<float*>(u->grads.ptr));
 	UP_CUDA(u, cudaGetLastError());
 	return SW_OK;
 }
 
-int pack_weights(SwUpscaler* u, int update, float lr, cudaStream_t s)
+AdamArgs adam_args(SwUpscaler* u, int update, float lr)
 {
 	AdamArgs a;
 	a.params = static_cast<float*>(u->params.ptr);
@@ -1527,7 +1565,26 @@ int pack_weights(SwUpscaler* u, int update, float lr, cudaStream_t s)
 		a.wbwd[l] = l > 0 ? static_cast<uint16_t*>(u->wbwd[l].ptr) : nullptr;
 		a.bias[l] = static_cast<float*>(u->bias[l].ptr);
 	}
-	adam_pack_kernel<<<(SW_UPSCALER_NUM_PARAMS + 255) / 256, 256, 0, s>>>(a);
+	return a;
+}
+
+int pack_weights(SwUpscaler* u, cudaStream_t s)
+{
+	adam_pack_kernel<<<(SW_UPSCALER_NUM_PARAMS + 255) / 256, 256, 0, s>>>(adam_args(u, 0, 0.0f));
+	UP_CUDA(u, cudaGetLastError());
+	return SW_OK;
+}
+
+// The gradients from the step's partials, and with `update` the Adam step.
+int reduce_gradients(SwUpscaler* u, uint32_t num_crops, uint32_t count, int update, float lr, cudaStream_t s)
+{
+	ReduceArgs a;
+	for (int l = 0; l < NUM_LAYERS; ++l) a.partial[l] = static_cast<const float*>(u->partial[l].ptr);
+	a.num_ctas = num_crops * WGRAD_CTAS_PER_CROP;
+	a.scale = 1.0f / float(count);
+	a.grads = static_cast<float*>(u->grads.ptr);
+	a.adam = adam_args(u, update, lr);
+	wgrad_reduce_kernel<<<reduce_first(NUM_LAYERS), REDUCE_WARPS * 32, 0, s>>>(a);
 	UP_CUDA(u, cudaGetLastError());
 	if (update) ++u->steps;
 	return SW_OK;
@@ -1590,7 +1647,8 @@ int prepare_training(SwUpscaler* u, uint32_t n)
 		}
 		if ((r = dev_alloc(u, u->t_g4, planes_bytes(cap, W, H, 2)))) return r;
 		const size_t ctas = size_t(cap) * (H / ROWS) * ((W + TILE_X - 1) / TILE_X);
-		if ((r = dev_alloc(u, u->partial, ctas * wgrad_partial_floats<4, 32>() * 4, false))) return r;
+		for (int l = 0; l < NUM_LAYERS; ++l)
+			if ((r = dev_alloc(u, u->partial[l], ctas * wgrad_partial_floats(LAYERS[l].c8_in, LAYERS[l].n_out) * 4, false))) return r;
 		if ((r = dev_alloc(u, u->loss_partial, std::max<size_t>(ctas, 4096) * 4, false))) return r;
 		if ((r = dev_alloc(u, u->crops, cap * sizeof(CropGpu), false))) return r;
 		if (!u->h_stage.ptr)
@@ -1659,22 +1717,21 @@ int forward_backward(SwUpscaler* u, const SwUpscalerCrop* crops, uint32_t n, uin
 
 	const uint32_t count = n * (W - 2 * M) * (H - 2 * M) * 4 * 3;
 	*loss_count = count;
-	const float scale = 1.0f / float(count);
 	// layer 3 (32 -> 12): weight gradient, input gradient into G[2] masked by A[2]
-	if ((r = launch_wgrad<4, 16>(u, A[2], g4, 3, scale, s))) return r;
+	if ((r = launch_wgrad<4, 16>(u, A[2], g4, 3, s))) return r;
 	ConvArgs b{};
 	b.in = g4, b.out = G[2], b.mask = A[2], b.wpack = static_cast<uint16_t*>(u->wbwd[3].ptr);
 	if ((r = launch_conv<2, 32, EPI_MASK>(u, b, s))) return r;
 	// layer 2
-	if ((r = launch_wgrad<4, 32>(u, A[1], G[2], 2, scale, s))) return r;
+	if ((r = launch_wgrad<4, 32>(u, A[1], G[2], 2, s))) return r;
 	b.in = G[2], b.out = G[1], b.mask = A[1], b.wpack = static_cast<uint16_t*>(u->wbwd[2].ptr);
 	if ((r = launch_conv<4, 32, EPI_MASK>(u, b, s))) return r;
 	// layer 1
-	if ((r = launch_wgrad<4, 32>(u, A[0], G[1], 1, scale, s))) return r;
+	if ((r = launch_wgrad<4, 32>(u, A[0], G[1], 1, s))) return r;
 	b.in = G[1], b.out = G[0], b.mask = A[0], b.wpack = static_cast<uint16_t*>(u->wbwd[1].ptr);
 	if ((r = launch_conv<4, 32, EPI_MASK>(u, b, s))) return r;
 	// layer 0 (3 -> 32): weight gradient only
-	if ((r = launch_wgrad<2, 32>(u, x0, G[0], 0, scale, s))) return r;
+	if ((r = launch_wgrad<2, 32>(u, x0, G[0], 0, s))) return r;
 	return SW_OK;
 }
 
@@ -1755,7 +1812,7 @@ int sw_upscaler_destroy(SwUpscaler* u)
 	if (!u) return SW_ERR_INVALID_ARGUMENT;
 	cudaSetDevice(u->device);
 	if (u->stream) cudaStreamSynchronize(u->stream);
-	DevMem* all[] = {&u->params, &u->adam_m, &u->adam_v, &u->grads, &u->error, &u->t_x0, &u->t_g4, &u->partial,
+	DevMem* all[] = {&u->params, &u->adam_m, &u->adam_v, &u->grads, &u->error, &u->t_x0, &u->t_g4,
 		&u->loss_partial, &u->crops, &u->i_x0, &u->i_p, &u->i_q, &u->i_crop, &u->psnr_sum};
 	for (DevMem* m : all) dev_free(*m);
 	for (int i = 0; i < 3; ++i)
@@ -1765,6 +1822,7 @@ int sw_upscaler_destroy(SwUpscaler* u)
 	}
 	for (int l = 0; l < NUM_LAYERS; ++l)
 	{
+		dev_free(u->partial[l]);
 		dev_free(u->wfwd[l]);
 		dev_free(u->wbwd[l]);
 		dev_free(u->bias[l]);
@@ -1798,7 +1856,7 @@ int sw_upscaler_set_params(SwUpscaler* u, const float* params, uint32_t count)
 	UP_CUDA(u, cudaMemsetAsync(u->adam_m.ptr, 0, count * 4, u->stream));
 	UP_CUDA(u, cudaMemsetAsync(u->adam_v.ptr, 0, count * 4, u->stream));
 	u->steps = 0;
-	int r = pack_weights(u, 0, 0.0f, u->stream);
+	int r = pack_weights(u, u->stream);
 	if (r) return r;
 	UP_CUDA(u, cudaStreamSynchronize(u->stream));
 	return SW_OK;
@@ -1811,6 +1869,7 @@ int sw_upscaler_gradients(SwUpscaler* u, const SwUpscalerCrop* crops, uint32_t n
 	uint32_t count = 0;
 	int r = forward_backward(u, crops, num_crops, &count);
 	if (r) return r;
+	if ((r = reduce_gradients(u, num_crops, count, 0, 0.0f, u->stream))) return r;
 	UP_CUDA(u, cudaMemcpyAsync(grads, u->grads.ptr, SW_UPSCALER_NUM_PARAMS * 4, cudaMemcpyDeviceToHost, u->stream));
 	float mse = 0.0f;
 	if ((r = read_loss(u, count, &mse))) return r;
@@ -1825,7 +1884,7 @@ int sw_upscaler_train_step(SwUpscaler* u, const SwUpscalerCrop* crops, uint32_t 
 	uint32_t count = 0;
 	int r = forward_backward(u, crops, num_crops, &count);
 	if (r) return r;
-	if ((r = pack_weights(u, 1, lr, u->stream))) return r;
+	if ((r = reduce_gradients(u, num_crops, count, 1, lr, u->stream))) return r;
 	if (mse) return read_loss(u, count, mse);
 	return SW_OK;
 }
