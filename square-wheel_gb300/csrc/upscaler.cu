@@ -363,6 +363,10 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) conv_kernel(const __grid_cons
 	__syncthreads();
 	fence_after_sync();
 	bool failed = false;
+	// everything above touched only the SM: it overlaps the end of the kernel before. The next kernel may be
+	// scheduled from here on (this one's TMEM is allocated); it waits for this grid before it reads or writes.
+	pdl_trigger();
+	pdl_wait();
 
 	if (warp == 0)
 	{
@@ -1058,6 +1062,8 @@ __global__ void __launch_bounds__(128) wgrad_kernel(WgradArgs a)
 	__syncthreads();
 	fence_after_sync();
 	const uint32_t tmem = *s_tmem;
+	pdl_trigger();
+	pdl_wait(); // the planes are written
 
 	if (tid == 0)
 	{
@@ -1166,6 +1172,8 @@ __global__ void convert_input_kernel(const CropGpu* crops, Planes p)
 {
 	const uint32_t img = blockIdx.y;
 	const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
+	pdl_trigger();
+	pdl_wait();
 	if (idx >= p.width * p.height) return;
 	const int x = int(idx % p.width), y = int(idx / p.width);
 	const CropGpu c = crops[img];
@@ -1292,6 +1300,8 @@ __global__ void __launch_bounds__(REDUCE_WARPS * 32) wgrad_reduce_kernel(const _
 		if (co < L.cout) idx = L.param_offset + L.cout * 9 * L.cin + co;
 	}
 	float s = 0.0f;
+	pdl_trigger();
+	pdl_wait(); // every layer's partials are written
 	if (valid)
 	{
 		const float* p = a.partial[l] + off;
@@ -1510,8 +1520,7 @@ int launch_conv(SwUpscaler* u, ConvArgs a, cudaStream_t s)
 		if (blocks * 4 > u->loss_partial.bytes) return fail(u, SW_ERR_LIMIT, "loss partial buffer too small");
 		u->loss_ctas = blocks;
 	}
-	conv_kernel<C8, N, EPI><<<blocks, CONV_THREADS, smem, s>>>(a);
-	UP_CUDA(u, cudaGetLastError());
+	UP_CUDA(u, launch_dependent(conv_kernel<C8, N, EPI>, dim3(blocks), dim3(CONV_THREADS), smem, s, a));
 	return SW_OK;
 }
 
@@ -1539,8 +1548,7 @@ int launch_wgrad(SwUpscaler* u, const Planes& x, const Planes& g, int layer, cud
 	const uint32_t blocks = x.images * a.tiles_x * a.row_blocks; // images * WGRAD_CTAS_PER_CROP for training crops
 	if (size_t(blocks) * wgrad_partial_floats(C8X, NG) * 4 > u->partial[layer].bytes)
 		return fail(u, SW_ERR_LIMIT, "weight-gradient partial buffer too small");
-	wgrad_kernel<C8X, NG><<<blocks, 128, smem, s>>>(a);
-	UP_CUDA(u, cudaGetLastError());
+	UP_CUDA(u, launch_dependent(wgrad_kernel<C8X, NG>, dim3(blocks), dim3(128), smem, s, a));
 	return SW_OK;
 }
 
@@ -1584,8 +1592,7 @@ int reduce_gradients(SwUpscaler* u, uint32_t num_crops, uint32_t count, int upda
 	a.scale = 1.0f / float(count);
 	a.grads = static_cast<float*>(u->grads.ptr);
 	a.adam = adam_args(u, update, lr);
-	wgrad_reduce_kernel<<<reduce_first(NUM_LAYERS), REDUCE_WARPS * 32, 0, s>>>(a);
-	UP_CUDA(u, cudaGetLastError());
+	UP_CUDA(u, launch_dependent(wgrad_reduce_kernel, dim3(reduce_first(NUM_LAYERS)), dim3(REDUCE_WARPS * 32), 0, s, a));
 	if (update) ++u->steps;
 	return SW_OK;
 }
