@@ -73,20 +73,27 @@ __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.
 
 // ---- MMA ----
 
-// D[tmem] (+)= A * B^T, M x N x 16, one thread issues.
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate)
+// D[tmem] (+)= A * B^T, M x N x 16: called by a whole converged warp with the same operands in every lane, issued
+// by the one lane whose `issue` is non-zero. The instruction takes its operands from uniform registers: in code
+// that the whole warp runs the compiler keeps descriptors there, while in a branch that one thread takes it moves
+// them over for every MMA, which measured 142 cycles per MMA whatever its shape, against 57 for 128 x 96 x 16 (43
+// for N = 32, 97 for N = 192: 128 bytes of operands per cycle, or the math) with the predicate.
+__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate,
+	uint32_t issue)
 {
 	asm volatile(
-		"{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-		"tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-		"l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+		"{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+		"@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+		"l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(issue)
 		: "memory");
 }
 
-// Arrive on the mbarrier once every MMA this thread issued before has completed.
-__device__ __forceinline__ void mma_commit(uint64_t* mbar)
+// Arrive on the mbarrier once every MMA the issuing lane issued before has completed (the whole warp calls it).
+__device__ __forceinline__ void mma_commit(uint64_t* mbar, uint32_t issue)
 {
-	asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(mbar))
+	asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+				 "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" ::"r"(smem_addr(mbar)),
+		"r"(issue)
 				 : "memory");
 }
 
@@ -116,6 +123,11 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* mbar, uint32_t parit
 	for (uint32_t i = 0; i < max_polls; ++i)
 		if (mbar_try_wait(mbar, parity)) return true;
 	return false;
+}
+// The same by a whole warp, one answer for all lanes (true when every lane saw the phase complete).
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* mbar, uint32_t parity, uint32_t max_polls)
+{
+	return __all_sync(0xFFFFFFFFu, mbar_wait_bounded(mbar, parity, max_polls));
 }
 
 // ---- bulk copies (TMA, untiled) ----

@@ -279,7 +279,7 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, const float (&v
 // 3 x (C8 / 2) MMAs of 128 x 3N x 16 and released; an output row is complete after input row y + 1.
 //   warp 0 (one lane): bulk-copies the packed weights once, then loads input rows (all chunks, 136
 //     pixels; one tiled TMA each) into a ring of NSTAGE shared-memory rows;
-//   warp 1 (one lane; the warp owns the TMEM allocation): per input row waits for it (and, when it
+//   warp 1 (lane 0 issues; the warp owns the TMEM allocation): per input row waits for it (and, when it
 //     starts a new output row, for that row's accumulator to be free), issues the MMAs and commits the
 //     row to rowbar[k % NBAR]: that releases the input row's slot and completes output row y_in - 1;
 //   warps 2..9: per output row: TMEM -> registers (warp w reads lanes 32*(w%4).., i.e. pixels), zero
@@ -328,7 +328,8 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) conv_kernel(const __grid_cons
 	uint32_t* s_tmem = reinterpret_cast<uint32_t*>(donebar + 1);
 	float* s_red = reinterpret_cast<float*>(s_tmem + 4); // [CONV_EPI_WARPS]
 
-	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+	const int tid = threadIdx.x, lane = tid & 31;
+	const int warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0); // known to be the same in the whole warp
 	const uint32_t H = a.in.height;
 	const uint32_t tiles_x = (a.in.width + TILE_X - 1) / TILE_X;
 	const RowRange rows = cta_rows(a.in.images * tiles_x * H);
@@ -350,7 +351,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) conv_kernel(const __grid_cons
 	fence_before_sync();
 	__syncthreads();
 	fence_after_sync();
-	const uint32_t tmem = *s_tmem;
+	const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, *s_tmem, 0);
 	if (warp >= 2)
 	{
 		// every accumulator starts at zero (the MMAs always accumulate)
@@ -406,8 +407,8 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) conv_kernel(const __grid_cons
 	}
 	else if (warp == 1)
 	{
-		if (lane == 0)
 		{
+			const uint32_t issue = lane == 0 ? 1u : 0u; // the whole warp runs the role, lane 0 issues
 			// Descriptors are precomputed: the start-address field is the low 14 bits (address >> 4), so a
 			// descriptor of base + off is the base descriptor + (off >> 4) (shared addresses stay < 256 KB).
 			const uint64_t a_base = make_sdesc(smem_addr(s_ring), CXS_BYTES, 128);
@@ -415,7 +416,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) conv_kernel(const __grid_cons
 			constexpr uint32_t IDESC1 = make_idesc_bf16(128, N, 0, 0);
 			constexpr uint32_t IDESC2 = make_idesc_bf16(128, 2 * N, 0, 0);
 			constexpr uint32_t IDESC3 = make_idesc_bf16(128, 3 * N, 0, 0);
-			failed = !mbar_wait_bounded(wbar, 0, POLL_LIMIT);
+			failed = !mbar_wait_warp(wbar, 0, POLL_LIMIT);
 			uint32_t k = 0, o_base = 0;
 			for (uint32_t r = rows.begin; r < rows.end && !failed;)
 			{
@@ -423,13 +424,13 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) conv_kernel(const __grid_cons
 				r += y_hi - y_lo;
 				for (int yi = int(y_lo) - 1; yi <= int(y_hi); ++yi, ++k)
 				{
-					failed = !mbar_wait_bounded(&full[k % NSTAGE], (k / NSTAGE) & 1, POLL_LIMIT);
+					failed = !mbar_wait_warp(&full[k % NSTAGE], (k / NSTAGE) & 1, POLL_LIMIT);
 					// contributions j = 0, 1, 2 go to output rows yi + 1 - j; keep those in [y_lo, y_hi)
 					const int j_lo = max(0, yi + 2 - int(y_hi)), j_hi = min(2, yi + 1 - int(y_lo));
 					const uint32_t o_first = o_base + uint32_t(yi + 1 - j_lo - int(y_lo)); // counter of row yi + 1 - j_lo
 					const uint32_t b0 = (R - o_first % R) % R;
 					if (!failed && j_lo == 0 && o_first >= R) // a new row's accumulator must have been drained
-						failed = !mbar_wait_bounded(&acce[b0], ((o_first / R) - 1) & 1, POLL_LIMIT);
+						failed = !mbar_wait_warp(&acce[b0], ((o_first / R) - 1) & 1, POLL_LIMIT);
 					if (failed) break;
 					fence_after_sync();
 					const uint64_t a_row = a_base + (((k % NSTAGE) * SLOT_BYTES) >> 4);
@@ -442,7 +443,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) conv_kernel(const __grid_cons
 #pragma unroll
 							for (int ks = 0; ks < KSTEPS; ++ks)
 								mma_bf16(d, a_row + ((2 * ks * CXS_BYTES + dx * 16) >> 4),
-									b_base + (((dx * KSTEPS + ks) * (2 * NB * 16)) >> 4), IDESC3, 1u);
+									b_base + (((dx * KSTEPS + ks) * (2 * NB * 16)) >> 4), IDESC3, 1u, issue);
 					}
 					else
 					{
@@ -461,18 +462,18 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) conv_kernel(const __grid_cons
 							{
 								const uint64_t ad = a_row + ((2 * ks * CXS_BYTES + dx * 16) >> 4);
 								const uint64_t bk = b_base + (((dx * KSTEPS + ks) * (2 * NB * 16)) >> 4);
-								mma_bf16(d0, ad, bk + bo0, id0, 1u);
-								if (two) mma_bf16(d1, ad, bk + bo1, id1, 1u);
+								mma_bf16(d0, ad, bk + bo0, id0, 1u, issue);
+								if (two) mma_bf16(d1, ad, bk + bo1, id1, 1u, issue);
 							}
 					}
 					// one commit: the input row's slot is free and output row yi - 1 (if j_hi == 2) complete
-					mma_commit(&rowbar[k % NBAR]);
+					mma_commit(&rowbar[k % NBAR], issue);
 				}
 				if (failed) break;
 				o_base += y_hi - y_lo;
 			}
-			mma_commit(donebar);
-			if (!mbar_wait_bounded(donebar, 0, POLL_LIMIT)) failed = true;
+			mma_commit(donebar, issue);
+			if (!mbar_wait_warp(donebar, 0, POLL_LIMIT)) failed = true;
 		}
 	}
 	else
@@ -677,19 +678,19 @@ __device__ __forceinline__ void f0_load_row(const FusedArgs& a, int y, bool vali
 // MMA group of layer L for its input index i (row A - 1 + i): the dy-folded K steps into the TMEM ring.
 // Returns false if a bounded wait expired.
 template <int L>
-__device__ __forceinline__ bool fused_mma(unsigned char* smem, uint32_t tmem, int y_lo, int y_hi, int i)
+__device__ __forceinline__ bool fused_mma(unsigned char* smem, uint32_t tmem, int y_lo, int y_hi, int i, uint32_t issue)
 {
 	using F = FL<L>;
 	constexpr int N = F::N;
 	const LayerRows lr = layer_rows(L, y_lo, y_hi);
 	uint64_t* full = f_full(smem, L);
 	uint64_t* accfree = f_accfree(smem, L);
-	if (!mbar_wait_bounded(&full[i % FNS], (i / FNS) & 1, POLL_LIMIT)) return false;
+	if (!mbar_wait_warp(&full[i % FNS], (i / FNS) & 1, POLL_LIMIT)) return false;
 	const int yi = lr.A - 1 + i;
 	const int j_lo = max(0, yi + 2 - lr.B), j_hi = min(2, yi + 1 - lr.A);
 	const uint32_t o_first = uint32_t(yi + 1 - j_lo - lr.A);
 	const uint32_t b0 = (FR - o_first % FR) % FR;
-	if (j_lo == 0 && o_first >= FR && !mbar_wait_bounded(&accfree[b0], ((o_first / FR) - 1) & 1, POLL_LIMIT)) return false;
+	if (j_lo == 0 && o_first >= FR && !mbar_wait_warp(&accfree[b0], ((o_first / FR) - 1) & 1, POLL_LIMIT)) return false;
 	fence_after_sync();
 	const uint64_t a_row = make_sdesc(smem_addr(smem + ring_base(L) + (i % FNS) * F::SLOT), CXS_BYTES, 128);
 	const uint32_t wofs = L == 0 ? FusedSmem::W0 : L == 1 ? FusedSmem::W1 : L == 2 ? FusedSmem::W2 : FusedSmem::W3;
@@ -705,7 +706,7 @@ __device__ __forceinline__ bool fused_mma(unsigned char* smem, uint32_t tmem, in
 #pragma unroll
 			for (int ks = 0; ks < F::KSTEPS; ++ks)
 				mma_bf16(d, a_row + ((2 * ks * CXS_BYTES + dx * 16) >> 4), b_base + (((dx * F::KSTEPS + ks) * (2 * F::NB * 16)) >> 4),
-					ID3, 1u);
+					ID3, 1u, issue);
 	}
 	else
 	{
@@ -722,8 +723,8 @@ __device__ __forceinline__ bool fused_mma(unsigned char* smem, uint32_t tmem, in
 			{
 				const uint64_t ad = a_row + ((2 * ks * CXS_BYTES + dx * 16) >> 4);
 				const uint64_t bk = b_base + (((dx * F::KSTEPS + ks) * (2 * F::NB * 16)) >> 4);
-				mma_bf16(tcol + b0 * N, ad, bk + bo0, id0, 1u);
-				if (two) mma_bf16(tcol, ad, bk + bo1, id1, 1u);
+				mma_bf16(tcol + b0 * N, ad, bk + bo0, id0, 1u, issue);
+				if (two) mma_bf16(tcol, ad, bk + bo1, id1, 1u, issue);
 			}
 	}
 	return true;
@@ -845,7 +846,8 @@ __global__ void __launch_bounds__(F_THREADS, 1) fused_upscale_kernel(const __gri
 	uint64_t* done = wbar + 1; // [2]: one per MMA issuer
 	uint32_t* s_tmem = reinterpret_cast<uint32_t*>(smem + FusedSmem::MISC);
 
-	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+	const int tid = threadIdx.x, lane = tid & 31;
+	const int warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0); // known to be the same in the whole warp
 	const int strip = int(blockIdx.x % a.strips), seg = int(blockIdx.x / a.strips);
 	const int H = int(a.lo_h);
 	const int y_lo = int((int64_t(seg) * H) / int(a.segments)), y_hi = int((int64_t(seg + 1) * H) / int(a.segments));
@@ -876,7 +878,7 @@ __global__ void __launch_bounds__(F_THREADS, 1) fused_upscale_kernel(const __gri
 	fence_before_sync();
 	__syncthreads();
 	fence_after_sync();
-	const uint32_t tmem = *s_tmem;
+	const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, *s_tmem, 0);
 	if (warp >= 2 && warp <= 9)
 	{
 		// every accumulator starts at zero (the MMAs always accumulate)
@@ -938,32 +940,31 @@ __global__ void __launch_bounds__(F_THREADS, 1) fused_upscale_kernel(const __gri
 	}
 	else if (warp == 1 || warp == 10)
 	{
-		if (lane == 0)
+		const uint32_t issue = lane == 0 ? 1u : 0u; // the whole warp runs the role, lane 0 issues
+		if (warp == 1 && lane == 0)
 		{
-			if (warp == 1)
-			{
-				mbar_expect_tx(wbar, FL<0>::WBYTES + FL<1>::WBYTES + FL<2>::WBYTES + FL<3>::WBYTES);
-				bulk_g2s(smem + FusedSmem::W0, a.w[0], FL<0>::WBYTES, wbar);
-				bulk_g2s(smem + FusedSmem::W1, a.w[1], FL<1>::WBYTES, wbar);
-				bulk_g2s(smem + FusedSmem::W2, a.w[2], FL<2>::WBYTES, wbar);
-				bulk_g2s(smem + FusedSmem::W3, a.w[3], FL<3>::WBYTES, wbar);
-			}
-			failed = !mbar_wait_bounded(wbar, 0, POLL_LIMIT);
-			const int la = warp == 1 ? 0 : 1; // this issuer's layers: la and la + 2
-			const int n_a = layer_rows(la, y_lo, y_hi).inputs(), n_b = layer_rows(la + 2, y_lo, y_hi).inputs();
-			for (int s = 0; s < steps && !failed; ++s)
-			{
-				const int i0 = s - FLAG * la, i1 = s - FLAG * (la + 2);
-				if (i0 >= 0 && i0 < n_a)
-					failed = !(la == 0 ? fused_mma<0>(smem, tmem, y_lo, y_hi, i0) : fused_mma<1>(smem, tmem, y_lo, y_hi, i0));
-				if (!failed && i1 >= 0 && i1 < n_b)
-					failed = !(la == 0 ? fused_mma<2>(smem, tmem, y_lo, y_hi, i1) : fused_mma<3>(smem, tmem, y_lo, y_hi, i1));
-				if (!failed) mma_commit(&f_rowbar(smem, la)[s % NBAR]); // the step's rows are consumed
-			}
-			uint64_t* d = &done[warp == 1 ? 0 : 1];
-			mma_commit(d);
-			if (!mbar_wait_bounded(d, 0, POLL_LIMIT)) failed = true;
+			mbar_expect_tx(wbar, FL<0>::WBYTES + FL<1>::WBYTES + FL<2>::WBYTES + FL<3>::WBYTES);
+			bulk_g2s(smem + FusedSmem::W0, a.w[0], FL<0>::WBYTES, wbar);
+			bulk_g2s(smem + FusedSmem::W1, a.w[1], FL<1>::WBYTES, wbar);
+			bulk_g2s(smem + FusedSmem::W2, a.w[2], FL<2>::WBYTES, wbar);
+			bulk_g2s(smem + FusedSmem::W3, a.w[3], FL<3>::WBYTES, wbar);
 		}
+		__syncwarp();
+		failed = !mbar_wait_warp(wbar, 0, POLL_LIMIT);
+		const int la = warp == 1 ? 0 : 1; // this issuer's layers: la and la + 2
+		const int n_a = layer_rows(la, y_lo, y_hi).inputs(), n_b = layer_rows(la + 2, y_lo, y_hi).inputs();
+		for (int s = 0; s < steps && !failed; ++s)
+		{
+			const int i0 = s - FLAG * la, i1 = s - FLAG * (la + 2);
+			if (i0 >= 0 && i0 < n_a)
+				failed = !(la == 0 ? fused_mma<0>(smem, tmem, y_lo, y_hi, i0, issue) : fused_mma<1>(smem, tmem, y_lo, y_hi, i0, issue));
+			if (!failed && i1 >= 0 && i1 < n_b)
+				failed = !(la == 0 ? fused_mma<2>(smem, tmem, y_lo, y_hi, i1, issue) : fused_mma<3>(smem, tmem, y_lo, y_hi, i1, issue));
+			if (!failed) mma_commit(&f_rowbar(smem, la)[s % NBAR], issue); // the step's rows are consumed
+		}
+		uint64_t* d = &done[warp == 1 ? 0 : 1];
+		mma_commit(d, issue);
+		if (!mbar_wait_warp(d, 0, POLL_LIMIT)) failed = true;
 	}
 	else
 	{
@@ -1039,7 +1040,8 @@ __global__ void __launch_bounds__(128) wgrad_kernel(WgradArgs a)
 	uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + 2);
 	float* s_bias = reinterpret_cast<float*>(bars + 4); // [128]
 
-	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+	const int tid = threadIdx.x, lane = tid & 31;
+	const int warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0); // known to be the same in the whole warp
 	uint32_t bid = blockIdx.x;
 	const uint32_t tx = bid % a.tiles_x;
 	bid /= a.tiles_x;
@@ -1061,7 +1063,7 @@ __global__ void __launch_bounds__(128) wgrad_kernel(WgradArgs a)
 	fence_before_sync();
 	__syncthreads();
 	fence_after_sync();
-	const uint32_t tmem = *s_tmem;
+	const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, *s_tmem, 0);
 	pdl_trigger();
 	pdl_wait(); // the planes are written
 
@@ -1084,25 +1086,22 @@ __global__ void __launch_bounds__(128) wgrad_kernel(WgradArgs a)
 		if (warp == 0) tmem_dealloc(tmem, TMEM_COLS);
 		return;
 	}
-	if (tid == 0)
+	if (warp == 0)
 	{
+		const uint32_t issue = lane == 0 ? 1u : 0u;
 		fence_after_sync();
-		const uint32_t idesc = make_idesc_bf16(128, NG, 1, 1);
-		const uint32_t xb = smem_addr(s_x), gb = smem_addr(s_g);
-		bool first[3] = {true, true, true};
+		constexpr uint32_t idesc = make_idesc_bf16(128, NG, 1, 1);
+		// A = X^T: rows (dy, chunk, ci % 8), 8-row groups XS_BYTES apart; K = 16 pixels, LBO = 8 pixels.
+		const uint64_t xb = make_sdesc(smem_addr(s_x), 128, XS_BYTES);
+		// B = G^T: columns co, 8-column groups XS_BYTES apart; the same 16 pixels.
+		const uint64_t gb = make_sdesc(smem_addr(s_g), 128, XS_BYTES);
 		for (int rr = 0; rr < ROWS; ++rr)
 			for (int kc = 0; kc < TILE_X / 16; ++kc)
+#pragma unroll
 				for (int d = 0; d < 3; ++d)
-				{
-					// A = X^T: rows (dy, chunk, ci % 8), 8-row groups XS_BYTES apart; K = 16 pixels, LBO = 8 pixels.
-					const uint32_t aaddr = xb + (rr * C8X) * XS_BYTES + (1 + (d - 1) + 16 * kc) * 16;
-					// B = G^T: columns co, 8-column groups XS_BYTES apart; the same 16 pixels.
-					const uint32_t baddr = gb + (rr * G8) * XS_BYTES + (1 + 16 * kc) * 16;
-					mma_bf16(tmem + d * NG, make_sdesc(aaddr, 128, XS_BYTES), make_sdesc(baddr, 128, XS_BYTES), idesc,
-						first[d] ? 0u : 1u);
-					first[d] = false;
-				}
-		mma_commit(&bars[1]);
+					mma_bf16(tmem + d * NG, xb + (((rr * C8X) * XS_BYTES + (d + 16 * kc) * 16) >> 4),
+						gb + (((rr * G8) * XS_BYTES + (1 + 16 * kc) * 16) >> 4), idesc, rr || kc ? 1u : 0u, issue);
+		mma_commit(&bars[1], issue);
 	}
 	// Bias gradient partials from the staged gradient rows (pixels 0..127 of the tile).
 	{
