@@ -562,19 +562,24 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) conv_kernel(const __grid_cons
 // C8_l chunks x 136 pixels (the layout conv_kernel stages from HBM), written by
 //   warp 0 (all lanes) for layer 0: Color32 source -> (b, g, r) / 255 in bf16 (the input conversion),
 //   the epilogue warps of layer l - 1 for layers 1..3: TMEM -> bias + ReLU -> bf16.
-// MMAs are the dy-folded implicit GEMM of conv_kernel (128 pixels x 3 C_out x 16 per MMA, accumulated
-// in place in a TMEM ring of 4 output rows per layer), issued by two threads: warp 1 for layers 0 and
-// 2, warp 10 for layers 1 and 3 (in step s, layer l's input row s - FLAG l). Epilogue warps 2..5 drain
-// layers 0 and 2, warps 6..9 layers 1 and 3 (the last one writes the Color32 output: pixel shuffle +
-// bilinear residual); in step s they handle layer l's output row s - 2 - FLAG l. A layer's output row is
-// complete two rows after its first input row, so FLAG - 2 steps of slack separate the epilogue that
-// writes a row from the MMAs that read it: enough to cover the tensor pipe's queue and the epilogue
-// itself, so that the roles run as a pipeline rather than a chain. The slot an epilogue writes was read
-// about FNS + 2 - FLAG steps earlier.
-constexpr int FNS = 5;          // input-row slots per layer
-constexpr int FR = 4;           // TMEM output-row accumulators per layer
-constexpr int FLAG = 5;         // rows of lag between layers
-constexpr int F_THREADS = 352;  // 11 warps
+// MMAs are the dy-folded implicit GEMM of conv_kernel, 128 pixels x 3 C_out x 16 each, accumulated in place in
+// a TMEM ring of 3 output rows per layer. Input row i adds to output rows i, i - 1 and i - 2 of its layer, which
+// are the whole ring, so one MMA per K step always covers it; which of the three vertical taps meets which slot
+// rotates from row to row, and the packed weights therefore lie in shared memory as ky = 0, 1, 2, 0, 1, with the
+// B descriptor starting at the row's rotation (a ring of 4 slots that split half of the rows' MMAs in two
+// pieces cost half as many MMAs again). Two warps issue them: warp 1 for layers 0 and 2, warp 2 for layers 1 and
+// 3 (in step s, layer l's input row s - FLAG l). Each layer has an epilogue group of four warps, 4 + 4 l ..:
+// layers 0..2 write the next layer's input row, the last one the Color32 output (pixel shuffle + bilinear
+// residual). Output row o is complete after input row o + 2, so FLAG - 2 steps separate the epilogue that
+// writes a row from the MMAs that read it, and the slot it writes was read 2 + FNS - FLAG steps earlier: every
+// wait is for work of an earlier step, so the roles cannot wait in a circle.
+// Bound by shared-memory operand reads (128 bytes a cycle: 57 cycles per MMA of 7 KB, 1,137 per step of 21
+// MMAs) and the epilogues' writes beside them. 960x540: 71 us with two epilogue groups, split MMAs and issue from
+// divergent code, 52 us with uniform issue.
+constexpr int FNS = 4;          // input-row slots per layer
+constexpr int FR = 3;           // TMEM output-row accumulators per layer
+constexpr int FLAG = 4;         // rows of lag between layers
+constexpr int F_THREADS = 640;  // 20 warps: source, two issuers, one idle, 16 epilogue
 constexpr int F_VALID = 120;    // output columns per strip
 constexpr uint32_t F_TMEM_COLS = 512;
 
@@ -597,10 +602,11 @@ struct FL
 	static constexpr int C8 = L == 0 ? 2 : 4;
 	static constexpr int N = L == 3 ? 16 : 32;
 	static constexpr int KSTEPS = C8 / 2;
-	static constexpr int NB = 3 * N;
+	static constexpr int GROUPS = 3 * KSTEPS * 2; // (kx, 16-channel step, half) groups of 8-channel weight rows
+	static constexpr int NB = 5 * N;              // rows of a group: ky = 0, 1, 2, 0, 1
 	static constexpr uint32_t SLOT = (C8 * CXS_BYTES + 127) / 128 * 128;
-	static constexpr uint32_t WBYTES = 3 * KSTEPS * 2 * NB * 16;
-	static constexpr uint32_t TCOL = L * 4 * 32; // TMEM column base (layers 0..2: 128 columns, 3: 64)
+	static constexpr uint32_t WBYTES = GROUPS * NB * 16;
+	static constexpr uint32_t TCOL = L * FR * 32; // TMEM column base (layers 0..2: 96 columns, 3: 48)
 };
 
 struct FusedSmem
@@ -636,13 +642,10 @@ __device__ __forceinline__ uint64_t* f_rowbar(unsigned char* smem, int l)
 {
 	return reinterpret_cast<uint64_t*>(smem + FusedSmem::BARS) + 4 * FNS + l * NBAR;
 }
-// Each MMA issuer commits once per step (issuer l & 1 serves layers l and l + 2; layer l's input row i
-// is issued in step i + FLAG l), so "input row i of layer l consumed" is the completion of that step.
+// Wait until the MMAs of layer l's input row i are done (its slot is free, output row i - 2 complete).
 __device__ __forceinline__ bool f_wait_input_done(unsigned char* smem, int l, int i)
 {
-	const int s = i + FLAG * l;
-	const bool ok = mbar_wait_bounded(&f_rowbar(smem, l & 1)[s % NBAR], (s / NBAR) & 1, POLL_LIMIT);
-	return __all_sync(0xFFFFFFFFu, ok);
+	return mbar_wait_warp(&f_rowbar(smem, l)[i % NBAR], (i / NBAR) & 1, POLL_LIMIT);
 }
 __device__ __forceinline__ uint64_t* f_accfree(unsigned char* smem, int l)
 {
@@ -675,58 +678,52 @@ __device__ __forceinline__ void f0_load_row(const FusedArgs& a, int y, bool vali
 	}
 }
 
-// MMA group of layer L for its input index i (row A - 1 + i): the dy-folded K steps into the TMEM ring.
-// Returns false if a bounded wait expired.
+// MMA group of layer L for its input index i (row A - 1 + i): the dy-folded K steps into the TMEM ring, then the
+// commit. Called by a whole warp. Returns false if a bounded wait expired.
 template <int L>
 __device__ __forceinline__ bool fused_mma(unsigned char* smem, uint32_t tmem, int y_lo, int y_hi, int i, uint32_t issue)
 {
 	using F = FL<L>;
 	constexpr int N = F::N;
 	const LayerRows lr = layer_rows(L, y_lo, y_hi);
-	uint64_t* full = f_full(smem, L);
-	uint64_t* accfree = f_accfree(smem, L);
-	if (!mbar_wait_warp(&full[i % FNS], (i / FNS) & 1, POLL_LIMIT)) return false;
-	const int yi = lr.A - 1 + i;
-	const int j_lo = max(0, yi + 2 - lr.B), j_hi = min(2, yi + 1 - lr.A);
-	const uint32_t o_first = uint32_t(yi + 1 - j_lo - lr.A);
-	const uint32_t b0 = (FR - o_first % FR) % FR;
-	if (j_lo == 0 && o_first >= FR && !mbar_wait_warp(&accfree[b0], ((o_first / FR) - 1) & 1, POLL_LIMIT)) return false;
+	if (!mbar_wait_warp(&f_full(smem, L)[i % FNS], (i / FNS) & 1, POLL_LIMIT)) return false;
+	// taps j = 0, 1, 2 go to output indexes i - j; keep those in [0, outputs)
+	const int j_lo = max(0, i + 1 - lr.outputs()), j_hi = min(2, i);
+	const uint32_t b0 = (FR - uint32_t(i) % FR) % FR; // slot of output i; i - 1 and i - 2 follow it around the ring
+	if (j_lo == 0 && i >= FR && !mbar_wait_warp(&f_accfree(smem, L)[b0], ((i / FR) - 1) & 1, POLL_LIMIT)) return false;
 	fence_after_sync();
 	const uint64_t a_row = make_sdesc(smem_addr(smem + ring_base(L) + (i % FNS) * F::SLOT), CXS_BYTES, 128);
 	const uint32_t wofs = L == 0 ? FusedSmem::W0 : L == 1 ? FusedSmem::W1 : L == 2 ? FusedSmem::W2 : FusedSmem::W3;
 	const uint64_t b_base = make_sdesc(smem_addr(smem + wofs), F::NB * 16, 128);
-	constexpr uint32_t ID1 = make_idesc_bf16(128, N, 0, 0), ID2 = make_idesc_bf16(128, 2 * N, 0, 0),
-					   ID3 = make_idesc_bf16(128, 3 * N, 0, 0);
+	constexpr uint32_t ID1 = make_idesc_bf16(128, N, 0, 0), ID3 = make_idesc_bf16(128, 3 * N, 0, 0);
 	const uint32_t tcol = tmem + F::TCOL;
-	if (j_lo == 0 && j_hi == 2 && b0 + 3 <= uint32_t(FR))
+	if (j_lo == 0 && j_hi == 2)
 	{
-		const uint32_t d = tcol + b0 * N;
+		// slot k takes tap (k - b0) mod 3: the weight rows from block (3 - b0) % 3 on
+		const uint64_t b_row = b_base + ((((FR - b0) % FR) * N * 16) >> 4);
 #pragma unroll
 		for (int dx = 0; dx < 3; ++dx)
 #pragma unroll
 			for (int ks = 0; ks < F::KSTEPS; ++ks)
-				mma_bf16(d, a_row + ((2 * ks * CXS_BYTES + dx * 16) >> 4), b_base + (((dx * F::KSTEPS + ks) * (2 * F::NB * 16)) >> 4),
+				mma_bf16(tcol, a_row + ((2 * ks * CXS_BYTES + dx * 16) >> 4), b_row + (((dx * F::KSTEPS + ks) * (2 * F::NB * 16)) >> 4),
 					ID3, 1u, issue);
 	}
 	else
 	{
-		const int nj = j_hi - j_lo + 1;
-		const int len0 = min(nj, int(FR - b0));
-		const uint32_t bo0 = uint32_t(j_lo * N * 16) >> 4, bo1 = uint32_t((j_lo + len0) * N * 16) >> 4;
-		const uint32_t id0 = len0 == 1 ? ID1 : len0 == 2 ? ID2 : ID3;
-		const uint32_t id1 = nj - len0 == 1 ? ID1 : ID2;
-		const bool two = len0 < nj;
+		// first and last rows of the segment: the taps that have an output row, one slot each
+		for (int j = j_lo; j <= j_hi; ++j)
+		{
+			const uint32_t d = tcol + ((b0 + uint32_t(j)) % FR) * N;
+			const uint64_t b_row = b_base + ((uint32_t(j) * N * 16) >> 4);
 #pragma unroll
-		for (int dx = 0; dx < 3; ++dx)
+			for (int dx = 0; dx < 3; ++dx)
 #pragma unroll
-			for (int ks = 0; ks < F::KSTEPS; ++ks)
-			{
-				const uint64_t ad = a_row + ((2 * ks * CXS_BYTES + dx * 16) >> 4);
-				const uint64_t bk = b_base + (((dx * F::KSTEPS + ks) * (2 * F::NB * 16)) >> 4);
-				mma_bf16(tcol + b0 * N, ad, bk + bo0, id0, 1u, issue);
-				if (two) mma_bf16(tcol, ad, bk + bo1, id1, 1u, issue);
-			}
+				for (int ks = 0; ks < F::KSTEPS; ++ks)
+					mma_bf16(d, a_row + ((2 * ks * CXS_BYTES + dx * 16) >> 4), b_row + (((dx * F::KSTEPS + ks) * (2 * F::NB * 16)) >> 4),
+						ID1, 1u, issue);
+		}
 	}
+	mma_commit(&f_rowbar(smem, L)[i % NBAR], issue);
 	return true;
 }
 
@@ -768,17 +765,9 @@ __device__ __forceinline__ bool fused_epilogue(const FusedArgs& a, unsigned char
 	const uint32_t b = (FR - uint32_t(o) % FR) % FR;
 	const uint32_t taddr = tmem + (uint32_t(quad * 32) << 16) + F::TCOL + b * N;
 	float v[N];
-#pragma unroll
-	for (int c8 = 0; c8 < N / 8; ++c8)
-	{
-		float t8[8];
-		tmem_ld8(taddr + c8 * 8, t8);
-#pragma unroll
-		for (int e = 0; e < 8; ++e) v[c8 * 8 + e] = t8[e];
-	}
+	tmem_ld<N>(taddr, v);
 	tmem_ld_wait();
-#pragma unroll
-	for (int c8 = 0; c8 < N / 8; ++c8) tmem_zero8(taddr + c8 * 8);
+	tmem_zero<N>(taddr);
 	tmem_st_wait();
 	fence_before_sync();
 	__syncwarp();
@@ -839,6 +828,32 @@ __device__ __forceinline__ bool fused_epilogue(const FusedArgs& a, unsigned char
 	return true;
 }
 
+// Layer L's epilogue group: every output row of the segment.
+template <int L>
+__device__ __forceinline__ bool fused_epilogues(const FusedArgs& a, unsigned char* smem, uint32_t tmem, int y_lo, int y_hi, int c0, int quad,
+	int lane)
+{
+	float bias[FL<L>::N];
+#pragma unroll
+	for (int c = 0; c < FL<L>::N; ++c) bias[c] = a.bias[L][c];
+	const int n = layer_rows(L, y_lo, y_hi).outputs();
+	for (int o = 0; o < n; ++o)
+		if (!fused_epilogue<L>(a, smem, tmem, y_lo, y_hi, o, c0, quad, lane, bias)) return false;
+	return true;
+}
+
+// The packed weights of layer L (conv_kernel's forward layout, ky = 0, 1, 2 in a group) into shared memory as
+// ky = 0, 1, 2, 0, 1; one lane per group.
+template <int L>
+__device__ __forceinline__ void f_load_weights(unsigned char* dst, const uint16_t* w, uint64_t* wbar, int lane)
+{
+	using F = FL<L>;
+	if (lane >= F::GROUPS) return;
+	const unsigned char* src = reinterpret_cast<const unsigned char*>(w) + lane * (3 * F::N * 16);
+	bulk_g2s(dst + lane * (F::NB * 16), src, 3 * F::N * 16, wbar);
+	bulk_g2s(dst + lane * (F::NB * 16) + 3 * F::N * 16, src, 2 * F::N * 16, wbar);
+}
+
 __global__ void __launch_bounds__(F_THREADS, 1) fused_upscale_kernel(const __grid_constant__ FusedArgs a)
 {
 	extern __shared__ __align__(1024) unsigned char smem[];
@@ -879,12 +894,11 @@ __global__ void __launch_bounds__(F_THREADS, 1) fused_upscale_kernel(const __gri
 	__syncthreads();
 	fence_after_sync();
 	const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, *s_tmem, 0);
-	if (warp >= 2 && warp <= 9)
+	if (warp >= 4)
 	{
-		// every accumulator starts at zero (the MMAs always accumulate)
-		const uint32_t lb = uint32_t((warp & 3) * 32) << 16;
-		const uint32_t c_lo = warp <= 5 ? 0u : 256u, c_hi = warp <= 5 ? 256u : 448u; // halves of the 448 used columns
-		for (uint32_t c = c_lo; c < c_hi; c += 8) tmem_zero8(tmem + lb + c);
+		// every accumulator starts at zero (the MMAs always accumulate): 96 columns per group
+		const uint32_t t = tmem + (uint32_t((warp & 3) * 32) << 16) + uint32_t((warp - 4) / 4) * (FR * 32);
+		for (uint32_t c = 0; c < FR * 32; c += 32) tmem_zero<32>(t + c);
 		tmem_st_wait();
 	}
 	fence_before_sync();
@@ -938,20 +952,20 @@ __global__ void __launch_bounds__(F_THREADS, 1) fused_upscale_kernel(const __gri
 				for (int k = 0; k < F0_PX; ++k) pre[r][k] = pre[r + 1][k];
 		}
 	}
-	else if (warp == 1 || warp == 10)
+	else if (warp == 1 || warp == 2)
 	{
 		const uint32_t issue = lane == 0 ? 1u : 0u; // the whole warp runs the role, lane 0 issues
-		if (warp == 1 && lane == 0)
+		if (warp == 1)
 		{
-			mbar_expect_tx(wbar, FL<0>::WBYTES + FL<1>::WBYTES + FL<2>::WBYTES + FL<3>::WBYTES);
-			bulk_g2s(smem + FusedSmem::W0, a.w[0], FL<0>::WBYTES, wbar);
-			bulk_g2s(smem + FusedSmem::W1, a.w[1], FL<1>::WBYTES, wbar);
-			bulk_g2s(smem + FusedSmem::W2, a.w[2], FL<2>::WBYTES, wbar);
-			bulk_g2s(smem + FusedSmem::W3, a.w[3], FL<3>::WBYTES, wbar);
+			if (lane == 0) mbar_expect_tx(wbar, FL<0>::WBYTES + FL<1>::WBYTES + FL<2>::WBYTES + FL<3>::WBYTES);
+			__syncwarp();
+			f_load_weights<0>(smem + FusedSmem::W0, a.w[0], wbar, lane);
+			f_load_weights<1>(smem + FusedSmem::W1, a.w[1], wbar, lane);
+			f_load_weights<2>(smem + FusedSmem::W2, a.w[2], wbar, lane);
+			f_load_weights<3>(smem + FusedSmem::W3, a.w[3], wbar, lane);
 		}
-		__syncwarp();
 		failed = !mbar_wait_warp(wbar, 0, POLL_LIMIT);
-		const int la = warp == 1 ? 0 : 1; // this issuer's layers: la and la + 2
+		const int la = warp - 1; // this issuer's layers: la and la + 2
 		const int n_a = layer_rows(la, y_lo, y_hi).inputs(), n_b = layer_rows(la + 2, y_lo, y_hi).inputs();
 		for (int s = 0; s < steps && !failed; ++s)
 		{
@@ -960,44 +974,23 @@ __global__ void __launch_bounds__(F_THREADS, 1) fused_upscale_kernel(const __gri
 				failed = !(la == 0 ? fused_mma<0>(smem, tmem, y_lo, y_hi, i0, issue) : fused_mma<1>(smem, tmem, y_lo, y_hi, i0, issue));
 			if (!failed && i1 >= 0 && i1 < n_b)
 				failed = !(la == 0 ? fused_mma<2>(smem, tmem, y_lo, y_hi, i1, issue) : fused_mma<3>(smem, tmem, y_lo, y_hi, i1, issue));
-			if (!failed) mma_commit(&f_rowbar(smem, la)[s % NBAR], issue); // the step's rows are consumed
 		}
-		uint64_t* d = &done[warp == 1 ? 0 : 1];
+		uint64_t* d = &done[la];
 		mma_commit(d, issue);
 		if (!mbar_wait_warp(d, 0, POLL_LIMIT)) failed = true;
 	}
-	else
+	else if (warp >= 4)
 	{
 		const int quad = warp & 3;
-		const bool group_a = warp <= 5; // layers 0 and 2; otherwise 1 and 3
-		const int la = group_a ? 0 : 1, lb = la + 2;
-		float bias_a[32], bias_b2[32], bias_b3[16];
-#pragma unroll
-		for (int c = 0; c < 32; ++c)
-		{
-			bias_a[c] = a.bias[la][c];
-			bias_b2[c] = a.bias[2][c];
-		}
-#pragma unroll
-		for (int c = 0; c < 16; ++c) bias_b3[c] = a.bias[3][c];
-		const int n_a = layer_rows(la, y_lo, y_hi).outputs(), n_b = layer_rows(lb, y_lo, y_hi).outputs();
-		for (int s = 0; s < steps && !failed; ++s)
-		{
-			// layer l's output o completes at its input o + 2, i.e. in step o + 2 + FLAG * l
-			const int oa = s - 2 - FLAG * la, ob = s - 2 - FLAG * lb;
-			if (oa >= 0 && oa < n_a)
-			{
-				const bool ok = group_a ? fused_epilogue<0>(a, smem, tmem, y_lo, y_hi, oa, c0, quad, lane, bias_a)
-										: fused_epilogue<1>(a, smem, tmem, y_lo, y_hi, oa, c0, quad, lane, bias_a);
-				if (!ok) failed = true;
-			}
-			if (!failed && ob >= 0 && ob < n_b)
-			{
-				const bool ok = group_a ? fused_epilogue<2>(a, smem, tmem, y_lo, y_hi, ob, c0, quad, lane, bias_b2)
-										: fused_epilogue<3>(a, smem, tmem, y_lo, y_hi, ob, c0, quad, lane, bias_b3);
-				if (!ok) failed = true;
-			}
-		}
+		const int layer = (warp - 4) >> 2;
+		if (layer == 0)
+			failed = !fused_epilogues<0>(a, smem, tmem, y_lo, y_hi, c0, quad, lane);
+		else if (layer == 1)
+			failed = !fused_epilogues<1>(a, smem, tmem, y_lo, y_hi, c0, quad, lane);
+		else if (layer == 2)
+			failed = !fused_epilogues<2>(a, smem, tmem, y_lo, y_hi, c0, quad, lane);
+		else
+			failed = !fused_epilogues<3>(a, smem, tmem, y_lo, y_hi, c0, quad, lane);
 	}
 	if (failed) atomicExch(a.error, 1);
 	fence_before_sync();
