@@ -121,6 +121,19 @@ __device__ __forceinline__ uint32_t to_byte(float v)
 	return uint32_t(fminf(fmaxf(s, 0.0f), 255.0f));
 }
 
+// Byte k of w as a float, and the clamped and rounded byte of a value as the low byte of the result, without the
+// conversion unit (a quarter of the other pipes' rate): 2^23 + b is exact for a byte, and adding 2^23 to a value
+// in [0, 255] rounds it to the nearest even integer. The bounds are integers, so clamping first changes nothing.
+template <int k>
+__device__ __forceinline__ float byte_float(uint32_t w)
+{
+	return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440 | k)) - 8388608.0f;
+}
+__device__ __forceinline__ uint32_t float_byte(float v)
+{
+	return __float_as_uint(fminf(fmaxf(v * 255.0f, 0.0f), 255.0f) + 8388608.0f);
+}
+
 constexpr int NSTAGE = 6;    // input rows staged in shared memory (ring)
 constexpr int CONV_RING = 8; // TMEM output-row accumulators of the convolution
 
@@ -727,118 +740,173 @@ __device__ __forceinline__ bool fused_mma(unsigned char* smem, uint32_t tmem, in
 	return true;
 }
 
-// Epilogue of layer L for its output index o (row A + o): accumulators -> registers, zero and release the
-// accumulator, then the next layer's input row (layers 0..2) or the Color32 output (layer 3). The four
-// warps of one group call this together (warp quad = lane quadrant = pixels quad*32..).
-template <int L>
-__device__ __forceinline__ bool fused_epilogue(const FusedArgs& a, unsigned char* smem, uint32_t tmem, int y_lo, int y_hi, int o, int c0,
-	int quad, int lane, const float (&bias)[FL<L>::N])
+// bf16 pair (low, high) of (a + bias) after ReLU: packed addition, rounding, then the maximum with 0, which is
+// what rounding the maximum gives.
+__device__ __forceinline__ uint32_t relu_pack(float a, float b, float2 bias)
 {
-	using F = FL<L>;
-	constexpr int N = F::N;
-	const LayerRows lr = layer_rows(L, y_lo, y_hi);
-	uint64_t* accfree = f_accfree(smem, L);
+	uint32_t lo, hi, r;
+	asm("{\n\t.reg .b64 v, c;\n\tmov.b64 v, {%2, %3};\n\tmov.b64 c, {%4, %5};\n\tadd.rn.f32x2 v, v, c;\n\tmov.b64 {%0, %1}, v;\n\t}"
+		: "=r"(lo), "=r"(hi)
+		: "f"(a), "f"(b), "f"(bias.x), "f"(bias.y));
+	asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(__uint_as_float(hi)), "f"(__uint_as_float(lo)));
+	asm("max.bf16x2 %0, %0, %1;" : "+r"(r) : "r"(0u));
+	return r;
+}
+
+// Epilogue of layer 0, 1 or 2 for its output rows in turn (output index o = row A + o), by the layer's four warps
+// (warp quad = lane quadrant = pixels quad*32..): accumulators -> registers, zero and release the accumulator,
+// then the next layer's input row. One instance for the three layers: their code stays in the instruction cache.
+__device__ __forceinline__ bool fused_epilogue_mid(const FusedArgs& a, unsigned char* smem, uint32_t tmem, int layer, int y_lo, int y_hi, int c0,
+	int quad, int lane)
+{
+	constexpr int N = 32;
+	const LayerRows lr = layer_rows(layer, y_lo, y_hi);
+	uint64_t* accfree = f_accfree(smem, layer);
+	uint64_t* next_full = f_full(smem, layer + 1);
 	const int i = quad * 32 + lane; // pixel of the strip
 	const int x = c0 + i;
-	const int y = lr.A + o;
-	// layer 3: the source pixels of the bilinear residual, loaded before the wait (rows y - 1, y, y + 1
-	// and columns x - 1, x, x + 1, clamped to the frame)
-	const bool out_px = L == 3 && i >= 4 && i < 4 + F_VALID && x < int(a.lo_w) && y < int(a.lo_h);
-	uint32_t p[3][3];
-	if constexpr (L == 3)
+	const bool x_in = x >= 0 && x < int(a.lo_w);
+	const uint32_t tcol = tmem + (uint32_t(quad * 32) << 16) + uint32_t(layer) * (FR * 32);
+	unsigned char* ring = smem + ring_base(layer + 1) + (1 + i) * 16;
+	float2 bias[N / 2];
+#pragma unroll
+	for (int c = 0; c < N / 2; ++c) bias[c] = make_float2(a.bias[layer][2 * c], a.bias[layer][2 * c + 1]);
+	const int n = lr.outputs();
+	for (int o = 0; o < n; ++o)
 	{
-		if (out_px)
+		if (!f_wait_input_done(smem, layer, o + 2)) return false; // the input row that completes output o
+		fence_after_sync();
+		const uint32_t b = (FR - uint32_t(o) % FR) % FR;
+		float v[N];
+		tmem_ld<N>(tcol + b * N, v);
+		tmem_ld_wait();
+		tmem_zero<N>(tcol + b * N);
+		const int y = lr.A + o;
+		const bool inside = x_in && y >= 0 && y < int(a.lo_h);
+		uint32_t w[N / 2];
+#pragma unroll
+		for (int c = 0; c < N / 2; ++c) w[c] = relu_pack(v[2 * c], v[2 * c + 1], bias[c]);
+		if (!__all_sync(0xFFFFFFFFu, inside)) // the next layer's zero padding
 		{
 #pragma unroll
-			for (int r = 0; r < 3; ++r)
-			{
-				const uint32_t* row = a.lo + size_t(min(max(y - 1 + r, 0), int(a.lo_h) - 1)) * a.lo_pitch;
-				p[r][0] = __ldg(row + max(x - 1, 0));
-				p[r][1] = __ldg(row + x);
-				p[r][2] = __ldg(row + min(x + 1, int(a.lo_w) - 1));
-			}
+			for (int c = 0; c < N / 2; ++c) w[c] = inside ? w[c] : 0u;
 		}
-	}
-	const int kc = o + 2; // the layer's input index that completes output o
-	if (!f_wait_input_done(smem, L, kc)) return false;
-	fence_after_sync();
-	const uint32_t b = (FR - uint32_t(o) % FR) % FR;
-	const uint32_t taddr = tmem + (uint32_t(quad * 32) << 16) + F::TCOL + b * N;
-	float v[N];
-	tmem_ld<N>(taddr, v);
-	tmem_ld_wait();
-	tmem_zero<N>(taddr);
-	tmem_st_wait();
-	fence_before_sync();
-	__syncwarp();
-	if (lane == 0) mbar_arrive(&accfree[b]);
-	if constexpr (L < 3)
-	{
-		uint64_t* next_full = f_full(smem, L + 1);
+		tmem_st_wait();
+		fence_before_sync();
+		__syncwarp();
+		if (lane == 0) mbar_arrive(&accfree[b]);
 		// next layer's input index o: wait until its slot's previous row was consumed
-		if (o >= FNS && !f_wait_input_done(smem, L + 1, o - FNS)) return false;
-		const bool inside = x >= 0 && x < int(a.lo_w) && y >= 0 && y < int(a.lo_h);
-		unsigned char* dst = smem + ring_base(L + 1) + (o % FNS) * FL<L + 1>::SLOT + (1 + i) * 16;
+		if (o >= FNS && !f_wait_input_done(smem, layer + 1, o - FNS)) return false;
+		unsigned char* dst = ring + (o % FNS) * FL<1>::SLOT; // the same slot size for layers 1..3
 #pragma unroll
 		for (int c8 = 0; c8 < N / 8; ++c8)
-		{
-			uint32_t w4[4];
-#pragma unroll
-			for (int q = 0; q < 4; ++q)
-				w4[q] = inside ? pack2(fmaxf(v[c8 * 8 + 2 * q] + bias[c8 * 8 + 2 * q], 0.0f),
-									 fmaxf(v[c8 * 8 + 2 * q + 1] + bias[c8 * 8 + 2 * q + 1], 0.0f))
-							   : 0u;
-			*reinterpret_cast<uint4*>(dst + c8 * CXS_BYTES) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
-		}
+			*reinterpret_cast<uint4*>(dst + c8 * CXS_BYTES) = make_uint4(w[c8 * 4], w[c8 * 4 + 1], w[c8 * 4 + 2], w[c8 * 4 + 3]);
 		fence_proxy_async();
 		__syncwarp();
 		if (lane == 0) mbar_arrive(&next_full[o % FNS]);
 	}
-	else
+	return true;
+}
+static_assert(FL<1>::SLOT == FL<2>::SLOT && FL<2>::SLOT == FL<3>::SLOT, "input rows of layers 1..3");
+
+// Source pixels x - 1, x, x + 1 (clamped) of source row y (clamped), and their horizontal 2x upsample: h[sx][c] is
+// colour c of output column 2x + sx.
+__device__ __forceinline__ void f3_load(const FusedArgs& a, int x, int y, uint32_t (&p)[3])
+{
+	const uint32_t* row = a.lo + size_t(min(max(y, 0), int(a.lo_h) - 1)) * a.lo_pitch;
+	p[0] = __ldg(row + max(x - 1, 0));
+	p[1] = __ldg(row + x);
+	p[2] = __ldg(row + min(x + 1, int(a.lo_w) - 1));
+}
+__device__ __forceinline__ void f3_upsample(const uint32_t (&p)[3], float (&h)[2][3])
+{
+	const float c[3][3] = {{byte_float<0>(p[0]), byte_float<1>(p[0]), byte_float<2>(p[0])},
+		{byte_float<0>(p[1]), byte_float<1>(p[1]), byte_float<2>(p[1])}, {byte_float<0>(p[2]), byte_float<1>(p[2]), byte_float<2>(p[2])}};
+#pragma unroll
+	for (int ch = 0; ch < 3; ++ch)
 	{
-		// output stage: columns c0 + 4 .. c0 + 123 of the strip, inside the frame
+		h[0][ch] = 0.75f * c[1][ch] + 0.25f * c[0][ch];
+		h[1][ch] = 0.75f * c[1][ch] + 0.25f * c[2][ch];
+	}
+}
+
+// Epilogue of the last layer: the Color32 output rows (pixel shuffle + bilinear residual) of the strip's columns
+// c0 + 4 .. c0 + 123 inside the frame. The source rows around the output row are kept upsampled, and the
+// next one is loaded a row ahead.
+__device__ __forceinline__ bool fused_epilogue_last(const FusedArgs& a, unsigned char* smem, uint32_t tmem, int y_lo, int y_hi, int c0, int quad,
+	int lane)
+{
+	constexpr int N = 16;
+	const LayerRows lr = layer_rows(3, y_lo, y_hi);
+	uint64_t* accfree = f_accfree(smem, 3);
+	const int i = quad * 32 + lane;
+	const int x = c0 + i;
+	const bool out_px = i >= 4 && i < 4 + F_VALID && x < int(a.lo_w);
+	const int xl = min(max(x, 0), int(a.lo_w) - 1); // lanes without an output pixel load some pixel of the row
+	const uint32_t tcol = tmem + (uint32_t(quad * 32) << 16) + FL<3>::TCOL;
+	float bias[12];
+#pragma unroll
+	for (int c = 0; c < 12; ++c) bias[c] = a.bias[3][c];
+	const int n = lr.outputs();
+	float h[3][2][3]; // source rows y - 1, y, y + 1
+	uint32_t p[3], alpha, alpha_next;
+	f3_load(a, xl, lr.A - 1, p);
+	f3_upsample(p, h[0]);
+	f3_load(a, xl, lr.A, p);
+	f3_upsample(p, h[1]);
+	alpha = p[1];
+	f3_load(a, xl, lr.A + 1, p);
+	f3_upsample(p, h[2]);
+	alpha_next = p[1];
+	for (int o = 0; o < n; ++o)
+	{
+		const int y = lr.A + o;
+		f3_load(a, xl, y + 2, p);
+		if (!f_wait_input_done(smem, 3, o + 2)) return false;
+		fence_after_sync();
+		const uint32_t b = (FR - uint32_t(o) % FR) % FR;
+		float v[N];
+		tmem_ld<N>(tcol + b * N, v);
+		tmem_ld_wait();
+		tmem_zero<N>(tcol + b * N);
+		tmem_st_wait();
+		fence_before_sync();
+		__syncwarp();
+		if (lane == 0) mbar_arrive(&accfree[b]);
 		if (out_px)
 		{
 #pragma unroll
 			for (int sy = 0; sy < 2; ++sy)
 			{
-				const uint32_t p11 = p[1][1], p10 = p[1][0], p12 = p[1][2];
-				const uint32_t p21 = p[sy ? 2 : 0][1], p20 = p[sy ? 2 : 0][0], p22 = p[sy ? 2 : 0][2];
 				uint32_t px[2];
 #pragma unroll
 				for (int sx = 0; sx < 2; ++sx)
 				{
-					const int s = sy * 2 + sx;
-					const uint32_t a01 = sx ? p12 : p10, a11 = sx ? p22 : p20;
-					uint32_t bytes = p11 & 0xFF000000u;
+					uint32_t q[3];
 #pragma unroll
 					for (int ch = 0; ch < 3; ++ch)
 					{
-						const float top = 0.75f * float((p11 >> (8 * ch)) & 255u) + 0.25f * float((a01 >> (8 * ch)) & 255u);
-						const float bot = 0.75f * float((p21 >> (8 * ch)) & 255u) + 0.25f * float((a11 >> (8 * ch)) & 255u);
-						const float pred = (0.75f * top + 0.25f * bot) * (1.0f / 255.0f) + (v[ch * 4 + s] + bias[ch * 4 + s]);
-						bytes |= to_byte(pred) << (8 * ch);
+						const float top = h[1][sx][ch], bot = h[sy ? 2 : 0][sx][ch];
+						q[ch] = float_byte((0.75f * top + 0.25f * bot) * (1.0f / 255.0f) + (v[ch * 4 + sy * 2 + sx] + bias[ch * 4 + sy * 2 + sx]));
 					}
-					px[sx] = bytes;
+					// bytes b, g, r of the values and the source pixel's alpha
+					px[sx] = __byte_perm(__byte_perm(q[0], q[1], 0x0040), __byte_perm(q[2], alpha, 0x0070), 0x5410);
 				}
 				*reinterpret_cast<uint2*>(a.hi + size_t(2 * y + sy) * a.hi_pitch + 2 * x) = make_uint2(px[0], px[1]);
 			}
 		}
-	}
-	return true;
-}
-
-// Layer L's epilogue group: every output row of the segment.
-template <int L>
-__device__ __forceinline__ bool fused_epilogues(const FusedArgs& a, unsigned char* smem, uint32_t tmem, int y_lo, int y_hi, int c0, int quad,
-	int lane)
-{
-	float bias[FL<L>::N];
 #pragma unroll
-	for (int c = 0; c < FL<L>::N; ++c) bias[c] = a.bias[L][c];
-	const int n = layer_rows(L, y_lo, y_hi).outputs();
-	for (int o = 0; o < n; ++o)
-		if (!fused_epilogue<L>(a, smem, tmem, y_lo, y_hi, o, c0, quad, lane, bias)) return false;
+		for (int sx = 0; sx < 2; ++sx)
+#pragma unroll
+			for (int ch = 0; ch < 3; ++ch)
+			{
+				h[0][sx][ch] = h[1][sx][ch];
+				h[1][sx][ch] = h[2][sx][ch];
+			}
+		f3_upsample(p, h[2]);
+		alpha = alpha_next;
+		alpha_next = p[1];
+	}
 	return true;
 }
 
@@ -937,8 +1005,8 @@ __global__ void __launch_bounds__(F_THREADS, 1) fused_upscale_kernel(const __gri
 				{
 					const uint32_t px = pre[0][k];
 					uint4 w4;
-					w4.x = pack2(float(px & 255u) * (1.0f / 255.0f), float((px >> 8) & 255u) * (1.0f / 255.0f));
-					w4.y = pack2(float((px >> 16) & 255u) * (1.0f / 255.0f), 0.0f);
+					w4.x = pack2(byte_float<0>(px) * (1.0f / 255.0f), byte_float<1>(px) * (1.0f / 255.0f));
+					w4.y = pack2(byte_float<2>(px) * (1.0f / 255.0f), 0.0f);
 					w4.z = 0u;
 					w4.w = 0u;
 					*reinterpret_cast<uint4*>(dst + j * 16) = w4;
@@ -983,14 +1051,8 @@ __global__ void __launch_bounds__(F_THREADS, 1) fused_upscale_kernel(const __gri
 	{
 		const int quad = warp & 3;
 		const int layer = (warp - 4) >> 2;
-		if (layer == 0)
-			failed = !fused_epilogues<0>(a, smem, tmem, y_lo, y_hi, c0, quad, lane);
-		else if (layer == 1)
-			failed = !fused_epilogues<1>(a, smem, tmem, y_lo, y_hi, c0, quad, lane);
-		else if (layer == 2)
-			failed = !fused_epilogues<2>(a, smem, tmem, y_lo, y_hi, c0, quad, lane);
-		else
-			failed = !fused_epilogues<3>(a, smem, tmem, y_lo, y_hi, c0, quad, lane);
+		failed = !(layer < 3 ? fused_epilogue_mid(a, smem, tmem, layer, y_lo, y_hi, c0, quad, lane)
+							 : fused_epilogue_last(a, smem, tmem, y_lo, y_hi, c0, quad, lane));
 	}
 	if (failed) atomicExch(a.error, 1);
 	fence_before_sync();
