@@ -580,19 +580,17 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) conv_kernel(const __grid_cons
 // are the whole ring, so one MMA per K step always covers it; which of the three vertical taps meets which slot
 // rotates from row to row, and the packed weights therefore lie in shared memory as ky = 0, 1, 2, 0, 1, with the
 // B descriptor starting at the row's rotation (a ring of 4 slots that split half of the rows' MMAs in two
-// pieces cost half as many MMAs again). Two warps issue them: warp 1 for layers 0 and 2, warp 2 for layers 1 and
-// 3 (in step s, layer l's input row s - FLAG l). Each layer has an epilogue group of four warps, 4 + 4 l ..:
-// layers 0..2 write the next layer's input row, the last one the Color32 output (pixel shuffle + bilinear
-// residual). Output row o is complete after input row o + 2, so FLAG - 2 steps separate the epilogue that
-// writes a row from the MMAs that read it, and the slot it writes was read 2 + FNS - FLAG steps earlier: every
-// wait is for work of an earlier step, so the roles cannot wait in a circle.
-// Bound by shared-memory operand reads (128 bytes a cycle: 57 cycles per MMA of 7 KB, 1,137 per step of 21
-// MMAs) and the epilogues' writes beside them. 960x540: 71 us with two epilogue groups, split MMAs and issue from
-// divergent code, 52 us with uniform issue.
+// pieces cost half as many MMAs again). Each layer has a warp that issues its MMAs, so that the tensor pipe has
+// another layer's queued while one waits on its barriers (two issuers with two layers each left it idle a third of
+// the time), and an epilogue group of four warps, 4 + 4 l ..: layers 0..2 write the next layer's input row, the
+// last one the Color32 output (pixel shuffle + bilinear residual). Output row o is complete after input row
+// o + 2. Every wait of layer l's row i is for layer l - 1's row i + 2 or earlier, or for layer l + 1's row
+// i - FNS - 3 or earlier, so the roles cannot wait in a circle.
+// Bound by shared-memory operand reads (128 bytes a cycle: 57 cycles per MMA of 7 KB, 1,129 for the 21 MMAs of
+// one row of every layer) and the epilogues' writes beside them.
 constexpr int FNS = 4;          // input-row slots per layer
 constexpr int FR = 3;           // TMEM output-row accumulators per layer
-constexpr int FLAG = 4;         // rows of lag between layers
-constexpr int F_THREADS = 640;  // 20 warps: source, two issuers, one idle, 16 epilogue
+constexpr int F_THREADS = 672;  // 21 warps: source, issuers of layers 0..2, 16 epilogue, issuer of layer 3
 constexpr int F_VALID = 120;    // output columns per strip
 constexpr uint32_t F_TMEM_COLS = 512;
 
@@ -633,8 +631,8 @@ struct FusedSmem
 	static constexpr uint32_t W2 = W1 + FL<1>::WBYTES;
 	static constexpr uint32_t W3 = W2 + FL<2>::WBYTES;
 	static constexpr uint32_t BARS = W3 + FL<3>::WBYTES;
-	// barriers: full[4][FNS], rowbar[4][NBAR], accfree[4][FR], wbar, done[2]
-	static constexpr uint32_t NUM_BARS = 4 * FNS + 4 * NBAR + 4 * FR + 3;
+	// barriers: full[4][FNS], rowbar[4][NBAR], accfree[4][FR], wbar, done[4]
+	static constexpr uint32_t NUM_BARS = 4 * FNS + 4 * NBAR + 4 * FR + 5;
 	static constexpr uint32_t MISC = BARS + NUM_BARS * 8;
 	static constexpr uint32_t TOTAL = MISC + 64;
 };
@@ -691,52 +689,60 @@ __device__ __forceinline__ void f0_load_row(const FusedArgs& a, int y, bool vali
 	}
 }
 
-// MMA group of layer L for its input index i (row A - 1 + i): the dy-folded K steps into the TMEM ring, then the
-// commit. Called by a whole warp. Returns false if a bounded wait expired.
-template <int L>
-__device__ __forceinline__ bool fused_mma(unsigned char* smem, uint32_t tmem, int y_lo, int y_hi, int i, uint32_t issue)
+// Layer `layer`'s MMAs for its input rows in turn (input index i = row A - 1 + i): the dy-folded K steps into the
+// TMEM ring, then the row's commit. Called by a whole warp; one instance for layers 1 and 2. Returns false if a
+// bounded wait expired.
+template <int KSTEPS, int N>
+__device__ __forceinline__ bool fused_mmas(unsigned char* smem, uint32_t tmem, int layer, uint32_t slot_bytes, uint32_t weights, int y_lo, int y_hi,
+	uint32_t issue)
 {
-	using F = FL<L>;
-	constexpr int N = F::N;
-	const LayerRows lr = layer_rows(L, y_lo, y_hi);
-	if (!mbar_wait_warp(&f_full(smem, L)[i % FNS], (i / FNS) & 1, POLL_LIMIT)) return false;
-	// taps j = 0, 1, 2 go to output indexes i - j; keep those in [0, outputs)
-	const int j_lo = max(0, i + 1 - lr.outputs()), j_hi = min(2, i);
-	const uint32_t b0 = (FR - uint32_t(i) % FR) % FR; // slot of output i; i - 1 and i - 2 follow it around the ring
-	if (j_lo == 0 && i >= FR && !mbar_wait_warp(&f_accfree(smem, L)[b0], ((i / FR) - 1) & 1, POLL_LIMIT)) return false;
-	fence_after_sync();
-	const uint64_t a_row = make_sdesc(smem_addr(smem + ring_base(L) + (i % FNS) * F::SLOT), CXS_BYTES, 128);
-	const uint32_t wofs = L == 0 ? FusedSmem::W0 : L == 1 ? FusedSmem::W1 : L == 2 ? FusedSmem::W2 : FusedSmem::W3;
-	const uint64_t b_base = make_sdesc(smem_addr(smem + wofs), F::NB * 16, 128);
+	constexpr int NB = 5 * N;
 	constexpr uint32_t ID1 = make_idesc_bf16(128, N, 0, 0), ID3 = make_idesc_bf16(128, 3 * N, 0, 0);
-	const uint32_t tcol = tmem + F::TCOL;
-	if (j_lo == 0 && j_hi == 2)
+	const LayerRows lr = layer_rows(layer, y_lo, y_hi);
+	const int n = lr.inputs(), outputs = lr.outputs();
+	const uint64_t a_base = make_sdesc(smem_addr(smem + ring_base(layer)), CXS_BYTES, 128);
+	const uint64_t b_base = make_sdesc(smem_addr(smem + weights), NB * 16, 128);
+	const uint32_t tcol = tmem + uint32_t(layer) * (FR * 32);
+	uint64_t* full = f_full(smem, layer);
+	uint64_t* accfree = f_accfree(smem, layer);
+	uint64_t* rowbar = f_rowbar(smem, layer);
+	for (int i = 0; i < n; ++i)
 	{
-		// slot k takes tap (k - b0) mod 3: the weight rows from block (3 - b0) % 3 on
-		const uint64_t b_row = b_base + ((((FR - b0) % FR) * N * 16) >> 4);
-#pragma unroll
-		for (int dx = 0; dx < 3; ++dx)
-#pragma unroll
-			for (int ks = 0; ks < F::KSTEPS; ++ks)
-				mma_bf16(tcol, a_row + ((2 * ks * CXS_BYTES + dx * 16) >> 4), b_row + (((dx * F::KSTEPS + ks) * (2 * F::NB * 16)) >> 4),
-					ID3, 1u, issue);
-	}
-	else
-	{
-		// first and last rows of the segment: the taps that have an output row, one slot each
-		for (int j = j_lo; j <= j_hi; ++j)
+		if (!mbar_wait_warp(&full[i % FNS], (i / FNS) & 1, POLL_LIMIT)) return false;
+		// taps j = 0, 1, 2 go to output indexes i - j; keep those in [0, outputs)
+		const int j_lo = max(0, i + 1 - outputs), j_hi = min(2, i);
+		const uint32_t b0 = (FR - uint32_t(i) % FR) % FR; // slot of output i; i - 1 and i - 2 follow it around the ring
+		if (j_lo == 0 && i >= FR && !mbar_wait_warp(&accfree[b0], ((i / FR) - 1) & 1, POLL_LIMIT)) return false;
+		fence_after_sync();
+		const uint64_t a_row = a_base + (((i % FNS) * slot_bytes) >> 4);
+		if (j_lo == 0 && j_hi == 2)
 		{
-			const uint32_t d = tcol + ((b0 + uint32_t(j)) % FR) * N;
-			const uint64_t b_row = b_base + ((uint32_t(j) * N * 16) >> 4);
+			// slot k takes tap (k - b0) mod 3: the weight rows from block (3 - b0) % 3 on
+			const uint64_t b_row = b_base + ((((FR - b0) % FR) * N * 16) >> 4);
 #pragma unroll
 			for (int dx = 0; dx < 3; ++dx)
 #pragma unroll
-				for (int ks = 0; ks < F::KSTEPS; ++ks)
-					mma_bf16(d, a_row + ((2 * ks * CXS_BYTES + dx * 16) >> 4), b_row + (((dx * F::KSTEPS + ks) * (2 * F::NB * 16)) >> 4),
-						ID1, 1u, issue);
+				for (int ks = 0; ks < KSTEPS; ++ks)
+					mma_bf16(tcol, a_row + ((2 * ks * CXS_BYTES + dx * 16) >> 4), b_row + (((dx * KSTEPS + ks) * (2 * NB * 16)) >> 4), ID3,
+						1u, issue);
 		}
+		else
+		{
+			// first and last rows of the segment: the taps that have an output row, one slot each
+			for (int j = j_lo; j <= j_hi; ++j)
+			{
+				const uint32_t d = tcol + ((b0 + uint32_t(j)) % FR) * N;
+				const uint64_t b_row = b_base + ((uint32_t(j) * N * 16) >> 4);
+#pragma unroll
+				for (int dx = 0; dx < 3; ++dx)
+#pragma unroll
+					for (int ks = 0; ks < KSTEPS; ++ks)
+						mma_bf16(d, a_row + ((2 * ks * CXS_BYTES + dx * 16) >> 4), b_row + (((dx * KSTEPS + ks) * (2 * NB * 16)) >> 4), ID1,
+							1u, issue);
+			}
+		}
+		mma_commit(&rowbar[i % NBAR], issue);
 	}
-	mma_commit(&f_rowbar(smem, L)[i % NBAR], issue);
 	return true;
 }
 
@@ -926,7 +932,7 @@ __global__ void __launch_bounds__(F_THREADS, 1) fused_upscale_kernel(const __gri
 {
 	extern __shared__ __align__(1024) unsigned char smem[];
 	uint64_t* wbar = reinterpret_cast<uint64_t*>(smem + FusedSmem::BARS) + 4 * FNS + 4 * NBAR + 4 * FR;
-	uint64_t* done = wbar + 1; // [2]: one per MMA issuer
+	uint64_t* done = wbar + 1; // [4]: one per MMA issuer
 	uint32_t* s_tmem = reinterpret_cast<uint32_t*>(smem + FusedSmem::MISC);
 
 	const int tid = threadIdx.x, lane = tid & 31;
@@ -948,8 +954,7 @@ __global__ void __launch_bounds__(F_THREADS, 1) fused_upscale_kernel(const __gri
 			for (int k = 0; k < FR; ++k) mbar_init(&f_accfree(smem, l)[k], 4);
 		}
 		mbar_init(wbar, 1);
-		mbar_init(&done[0], 1);
-		mbar_init(&done[1], 1);
+		for (int l = 0; l < 4; ++l) mbar_init(&done[l], 1);
 		fence_mbar_init();
 	}
 	if (warp == 1)
@@ -962,7 +967,7 @@ __global__ void __launch_bounds__(F_THREADS, 1) fused_upscale_kernel(const __gri
 	__syncthreads();
 	fence_after_sync();
 	const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, *s_tmem, 0);
-	if (warp >= 4)
+	if (warp >= 4 && warp < 20)
 	{
 		// every accumulator starts at zero (the MMAs always accumulate): 96 columns per group
 		const uint32_t t = tmem + (uint32_t((warp & 3) * 32) << 16) + uint32_t((warp - 4) / 4) * (FR * 32);
@@ -974,7 +979,6 @@ __global__ void __launch_bounds__(F_THREADS, 1) fused_upscale_kernel(const __gri
 	fence_after_sync();
 
 	const LayerRows lr0 = layer_rows(0, y_lo, y_hi);
-	const int steps = lr0.inputs() + 3 * FLAG;
 	bool failed = false;
 
 	if (warp == 0)
@@ -1020,8 +1024,9 @@ __global__ void __launch_bounds__(F_THREADS, 1) fused_upscale_kernel(const __gri
 				for (int k = 0; k < F0_PX; ++k) pre[r][k] = pre[r + 1][k];
 		}
 	}
-	else if (warp == 1 || warp == 2)
+	else if (warp <= 3 || warp == 20)
 	{
+		const int layer = warp == 20 ? 3 : warp - 1;
 		const uint32_t issue = lane == 0 ? 1u : 0u; // the whole warp runs the role, lane 0 issues
 		if (warp == 1)
 		{
@@ -1033,21 +1038,19 @@ __global__ void __launch_bounds__(F_THREADS, 1) fused_upscale_kernel(const __gri
 			f_load_weights<3>(smem + FusedSmem::W3, a.w[3], wbar, lane);
 		}
 		failed = !mbar_wait_warp(wbar, 0, POLL_LIMIT);
-		const int la = warp - 1; // this issuer's layers: la and la + 2
-		const int n_a = layer_rows(la, y_lo, y_hi).inputs(), n_b = layer_rows(la + 2, y_lo, y_hi).inputs();
-		for (int s = 0; s < steps && !failed; ++s)
+		if (!failed)
 		{
-			const int i0 = s - FLAG * la, i1 = s - FLAG * (la + 2);
-			if (i0 >= 0 && i0 < n_a)
-				failed = !(la == 0 ? fused_mma<0>(smem, tmem, y_lo, y_hi, i0, issue) : fused_mma<1>(smem, tmem, y_lo, y_hi, i0, issue));
-			if (!failed && i1 >= 0 && i1 < n_b)
-				failed = !(la == 0 ? fused_mma<2>(smem, tmem, y_lo, y_hi, i1, issue) : fused_mma<3>(smem, tmem, y_lo, y_hi, i1, issue));
+			if (layer == 0)
+				failed = !fused_mmas<1, 32>(smem, tmem, 0, FL<0>::SLOT, FusedSmem::W0, y_lo, y_hi, issue);
+			else if (layer == 3)
+				failed = !fused_mmas<2, 16>(smem, tmem, 3, FL<3>::SLOT, FusedSmem::W3, y_lo, y_hi, issue);
+			else
+				failed = !fused_mmas<2, 32>(smem, tmem, layer, FL<1>::SLOT, layer == 1 ? FusedSmem::W1 : FusedSmem::W2, y_lo, y_hi, issue);
 		}
-		uint64_t* d = &done[la];
-		mma_commit(d, issue);
-		if (!mbar_wait_warp(d, 0, POLL_LIMIT)) failed = true;
+		mma_commit(&done[layer], issue);
+		if (!mbar_wait_warp(&done[layer], 0, POLL_LIMIT)) failed = true;
 	}
-	else if (warp >= 4)
+	else
 	{
 		const int quad = warp & 3;
 		const int layer = (warp - 4) >> 2;
