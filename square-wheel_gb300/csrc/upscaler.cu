@@ -631,8 +631,8 @@ struct FusedSmem
 	static constexpr uint32_t W2 = W1 + FL<1>::WBYTES;
 	static constexpr uint32_t W3 = W2 + FL<2>::WBYTES;
 	static constexpr uint32_t BARS = W3 + FL<3>::WBYTES;
-	// barriers: full[4][FNS], rowbar[4][NBAR], accfree[4][FR], wbar, done[4]
-	static constexpr uint32_t NUM_BARS = 4 * FNS + 4 * NBAR + 4 * FR + 5;
+	// barriers: full[4][FNS], rowbar[4][NBAR], accfree[4][FR], wbar[4], done[4]
+	static constexpr uint32_t NUM_BARS = 4 * FNS + 4 * NBAR + 4 * FR + 8;
 	static constexpr uint32_t MISC = BARS + NUM_BARS * 8;
 	static constexpr uint32_t TOTAL = MISC + 64;
 };
@@ -917,11 +917,13 @@ __device__ __forceinline__ bool fused_epilogue_last(const FusedArgs& a, unsigned
 }
 
 // The packed weights of layer L (conv_kernel's forward layout, ky = 0, 1, 2 in a group) into shared memory as
-// ky = 0, 1, 2, 0, 1; one lane per group.
+// ky = 0, 1, 2, 0, 1; by the layer's issuing warp, one lane per group.
 template <int L>
 __device__ __forceinline__ void f_load_weights(unsigned char* dst, const uint16_t* w, uint64_t* wbar, int lane)
 {
 	using F = FL<L>;
+	if (lane == 0) mbar_expect_tx(wbar, F::WBYTES);
+	__syncwarp();
 	if (lane >= F::GROUPS) return;
 	const unsigned char* src = reinterpret_cast<const unsigned char*>(w) + lane * (3 * F::N * 16);
 	bulk_g2s(dst + lane * (F::NB * 16), src, 3 * F::N * 16, wbar);
@@ -932,7 +934,7 @@ __global__ void __launch_bounds__(F_THREADS, 1) fused_upscale_kernel(const __gri
 {
 	extern __shared__ __align__(1024) unsigned char smem[];
 	uint64_t* wbar = reinterpret_cast<uint64_t*>(smem + FusedSmem::BARS) + 4 * FNS + 4 * NBAR + 4 * FR;
-	uint64_t* done = wbar + 1; // [4]: one per MMA issuer
+	uint64_t* done = wbar + 4; // [4] each: one per MMA issuer
 	uint32_t* s_tmem = reinterpret_cast<uint32_t*>(smem + FusedSmem::MISC);
 
 	const int tid = threadIdx.x, lane = tid & 31;
@@ -942,9 +944,20 @@ __global__ void __launch_bounds__(F_THREADS, 1) fused_upscale_kernel(const __gri
 	const int y_lo = int((int64_t(seg) * H) / int(a.segments)), y_hi = int((int64_t(seg + 1) * H) / int(a.segments));
 	const int c0 = strip * F_VALID - 4;
 
-	// zero every ring slot (halo pixels are never written; layer 0's second chunk stays zero)
-	for (uint32_t off = tid * 16; off < FusedSmem::W0; off += F_THREADS * 16)
+	// zero what no role writes: layer 0's second chunk, and in layers 1..3 the pixels outside the strip's 128
+	constexpr int EDGE = CXS - 128, L0_ZERO = FNS * CXS, ZEROS = L0_ZERO + 3 * FNS * FL<1>::C8 * EDGE;
+	for (int z = tid; z < ZEROS; z += F_THREADS)
+	{
+		uint32_t off;
+		if (z < L0_ZERO)
+			off = FusedSmem::RING0 + (z / CXS) * FL<0>::SLOT + CXS_BYTES + (z % CXS) * 16;
+		else
+		{
+			const int k = z - L0_ZERO, e = k % EDGE, chunk = k / EDGE % FL<1>::C8, slot = k / (EDGE * FL<1>::C8) % FNS, l = 1 + k / (EDGE * FL<1>::C8 * FNS);
+			off = ring_base(l) + slot * FL<1>::SLOT + chunk * CXS_BYTES + (e ? 128 + e : 0) * 16; // pixel 0, pixels 129..135
+		}
 		*reinterpret_cast<uint4*>(smem + off) = make_uint4(0u, 0u, 0u, 0u);
+	}
 	if (tid == 0)
 	{
 		for (int l = 0; l < 4; ++l)
@@ -953,8 +966,11 @@ __global__ void __launch_bounds__(F_THREADS, 1) fused_upscale_kernel(const __gri
 			for (int k = 0; k < NBAR; ++k) mbar_init(&f_rowbar(smem, l)[k], 1);
 			for (int k = 0; k < FR; ++k) mbar_init(&f_accfree(smem, l)[k], 4);
 		}
-		mbar_init(wbar, 1);
-		for (int l = 0; l < 4; ++l) mbar_init(&done[l], 1);
+		for (int l = 0; l < 4; ++l)
+		{
+			mbar_init(&wbar[l], 1);
+			mbar_init(&done[l], 1);
+		}
 		fence_mbar_init();
 	}
 	if (warp == 1)
@@ -980,6 +996,9 @@ __global__ void __launch_bounds__(F_THREADS, 1) fused_upscale_kernel(const __gri
 
 	const LayerRows lr0 = layer_rows(0, y_lo, y_hi);
 	bool failed = false;
+	// everything above touched only the SM: it overlaps the end of the kernel before
+	pdl_trigger();
+	pdl_wait();
 
 	if (warp == 0)
 	{
@@ -1028,16 +1047,13 @@ __global__ void __launch_bounds__(F_THREADS, 1) fused_upscale_kernel(const __gri
 	{
 		const int layer = warp == 20 ? 3 : warp - 1;
 		const uint32_t issue = lane == 0 ? 1u : 0u; // the whole warp runs the role, lane 0 issues
-		if (warp == 1)
-		{
-			if (lane == 0) mbar_expect_tx(wbar, FL<0>::WBYTES + FL<1>::WBYTES + FL<2>::WBYTES + FL<3>::WBYTES);
-			__syncwarp();
-			f_load_weights<0>(smem + FusedSmem::W0, a.w[0], wbar, lane);
-			f_load_weights<1>(smem + FusedSmem::W1, a.w[1], wbar, lane);
-			f_load_weights<2>(smem + FusedSmem::W2, a.w[2], wbar, lane);
-			f_load_weights<3>(smem + FusedSmem::W3, a.w[3], wbar, lane);
-		}
-		failed = !mbar_wait_warp(wbar, 0, POLL_LIMIT);
+		if (layer == 0)
+			f_load_weights<0>(smem + FusedSmem::W0, a.w[0], &wbar[0], lane);
+		else if (layer == 3)
+			f_load_weights<3>(smem + FusedSmem::W3, a.w[3], &wbar[3], lane);
+		else
+			f_load_weights<1>(smem + (layer == 1 ? FusedSmem::W1 : FusedSmem::W2), a.w[layer], &wbar[layer], lane);
+		failed = !mbar_wait_warp(&wbar[layer], 0, POLL_LIMIT);
 		if (!failed)
 		{
 			if (layer == 0)
@@ -1993,8 +2009,7 @@ int sw_upscaler_infer(SwUpscaler* u, const uint32_t* lo, uint32_t lo_width, uint
 		f.strips = (lo_width + F_VALID - 1) / F_VALID;
 		f.segments = std::max(1u, std::min(lo_height, uint32_t(u->num_sms) / f.strips));
 		f.error = static_cast<int*>(u->error.ptr);
-		fused_upscale_kernel<<<f.strips * f.segments, F_THREADS, FusedSmem::TOTAL, s>>>(f);
-		UP_CUDA(u, cudaGetLastError());
+		UP_CUDA(u, launch_dependent(fused_upscale_kernel, dim3(f.strips * f.segments), dim3(F_THREADS), FusedSmem::TOTAL, s, f));
 		return SW_OK;
 	}
 	if (lo_width != u->i_w || lo_height != u->i_h)
