@@ -520,7 +520,7 @@ int launch_bloom(const PostArgs& a, cudaStream_t stream, bool downscale)
 } // namespace
 
 int launch_postprocess(const PostArgs& a, int num_sms, cudaStream_t stream, cudaStream_t aux, cudaEvent_t fork,
-	cudaEvent_t join, cudaEvent_t average_done)
+	cudaEvent_t join, cudaEvent_t average_done, unsigned average_flags)
 {
 	(void)num_sms;
 	const dim3 block(256);
@@ -540,8 +540,9 @@ int launch_postprocess(const PostArgs& a, int num_sms, cudaStream_t stream, cuda
 			cudaStreamWaitEvent(aux, fork, 0);
 		}
 		pp_average_bloom_kernel<<<1, 256, 0, overlap ? aux : stream>>>(a);
-		// the average is final here: inside a captured graph this is an event record node
-		if (average_done) cudaEventRecordWithFlags(average_done, overlap ? aux : stream, cudaEventRecordExternal);
+		// the average is final here
+		if (average_done)
+			if (int e = int(cudaEventRecordWithFlags(average_done, overlap ? aux : stream, average_flags))) return e;
 		if (overlap) cudaEventRecord(join, aux);
 		// blur + tonemap with the bloom sample
 		if (int e = launch_bloom(a, stream, false)) return e;
@@ -551,7 +552,8 @@ int launch_postprocess(const PostArgs& a, int num_sms, cudaStream_t stream, cuda
 	{
 		pp_line_sums_kernel<<<(a.height + 127) / 128, 128, 0, stream>>>(a);
 		pp_average_plain_kernel<<<1, 256, 0, stream>>>(a);
-		if (average_done) cudaEventRecordWithFlags(average_done, stream, cudaEventRecordExternal);
+		if (average_done)
+			if (int e = int(cudaEventRecordWithFlags(average_done, stream, average_flags))) return e;
 		pp_tonemap_plain_kernel<<<dim3((a.width + 255) / 256, a.height), block, 0, stream>>>(a);
 	}
 	return int(cudaGetLastError());

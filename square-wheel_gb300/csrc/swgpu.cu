@@ -129,7 +129,7 @@ struct SwCtx
 	bool fb_valid = false;
 
 	// postprocessor
-	DevBuf bloom0, bloom1, line_sums, line_sums_f, average, error_counter;
+	DevBuf bloom0, bloom1, line_sums, line_sums_f, error_counter;
 	float exposure = 1.0f;
 	bool exposure_pending = false;
 	SwPostConfig pending_config{};
@@ -630,7 +630,6 @@ int sw_create(const SwCreateInfo* info, SwCtx** out_ctx)
 	ctx->num_dir_lightmap_elements = info->num_directional_lightmap_elements;
 	if ((r = ensure(ctx, ctx->error_counter, 16))) return bail(r);
 	if (cudaMemset(ctx->error_counter.ptr, 0, 16) != cudaSuccess) return bail(SW_ERR_CUDA);
-	if ((r = ensure(ctx, ctx->average, 16))) return bail(r);
 	if (info->max_surface_texels && (r = ensure(ctx, ctx->arena, info->max_surface_texels * 8))) return bail(r);
 	*out_ctx = ctx;
 	return SW_OK;
@@ -646,7 +645,7 @@ int sw_destroy(SwCtx* ctx)
 		&ctx->skybox64, &ctx->frame_in,
 		&ctx->dir_lightmaps, &ctx->lights, &ctx->surfaces, &ctx->work_prefix, &ctx->arena, &ctx->draws, &ctx->vertices,
 		&ctx->draw_rows, &ctx->rdraws, &ctx->rows, &ctx->boxes, &ctx->tri_steps, &ctx->tri_vertices, &ctx->lite, &ctx->ldr[0], &ctx->ldr[1], &ctx->framebuffer, &ctx->bloom0, &ctx->bloom1, &ctx->line_sums,
-		&ctx->line_sums_f, &ctx->average, &ctx->error_counter, &ctx->up_src, &ctx->up_dst, &ctx->map_polygons,
+		&ctx->line_sums_f, &ctx->error_counter, &ctx->up_src, &ctx->up_dst, &ctx->map_polygons,
 		&ctx->map_vertices, &ctx->vslab, &ctx->shadow_storage, &ctx->shadow_descs, &ctx->shadow_chunks, &ctx->effect_buf, &ctx->sim_state, &ctx->sim_buf, &ctx->vbin_lists,
 		&ctx->vbin_counts};
 	for (DevBuf* b : bufs) release(*b);
@@ -1223,7 +1222,9 @@ int prepare_post(SwCtx* ctx, const SwPostConfig* config, const float color_modul
 
 	std::memset(&a, 0, sizeof(a));
 	a.hdr = static_cast<const uint64_t*>(ctx->framebuffer.ptr);
-	a.average = static_cast<float*>(ctx->average.ptr);
+	// The frame's average colour goes straight to host memory and average_ready fires as soon as it is there, so
+	// that the next frame's exposure is known, and its host work done, while this frame is still tonemapped.
+	a.average = ctx->d_average_mapped;
 	if (!post_args_from_config(a, post_config_clamped(*config), ctx->exposure, color_modulate, w, h))
 		return fail(ctx, SW_ERR_INVALID_ARGUMENT, "frame too small for bloom");
 	if (a.use_bloom)
@@ -1266,12 +1267,10 @@ int sw_postprocess(SwCtx* ctx, const SwPostConfig* config, float frame_duration_
 	a.dst = static_cast<uint32_t*>(out);
 	a.dst_pitch = out_pitch;
 	stage_begin(ctx, STAGE_POST);
-	r = check_kernel(ctx, launch_postprocess(a, ctx->num_sms, ctx->stream, ctx->aux, ctx->ev_fork, ctx->ev_join),
+	r = check_kernel(ctx, launch_postprocess(a, ctx->num_sms, ctx->stream, ctx->aux, ctx->ev_fork, ctx->ev_join, ctx->average_ready),
 		"postprocess");
 	stage_end(ctx, STAGE_POST);
 	if (r) return r;
-	SW_CUDA(ctx, cudaMemcpyAsync(ctx->h_average, ctx->average.ptr, 16, cudaMemcpyDeviceToHost, ctx->stream));
-	SW_CUDA(ctx, cudaEventRecord(ctx->average_ready, ctx->stream));
 	stage_end(ctx, STAGE_FRAME);
 	ctx->exposure_pending = true;
 	ctx->pending_config = post_config_clamped(*config);
@@ -1763,8 +1762,11 @@ int fuse_bloom_downscale(SwCtx* ctx, RasterArgs& ra, PostArgs& pa, cudaStream_t 
 	return SW_OK;
 }
 
+// Recording average_ready inside a frame graph is an event record node.
+unsigned average_flags(const SwCtx* ctx) { return ctx->capturing ? cudaEventRecordExternal : cudaEventRecordDefault; }
+
 int enqueue_frame(SwCtx* ctx, const SwFrameInput& f, const unsigned char* h, const size_t* off, uint64_t rows,
-	const PostArgs* post, cudaEvent_t average_done = nullptr)
+	const PostArgs* post)
 {
 	cudaStream_t s = ctx->stream, aux = ctx->aux;
 	// every per-frame array in one copy: the device buffer has the staging block's layout
@@ -1837,11 +1839,10 @@ int enqueue_frame(SwCtx* ctx, const SwFrameInput& f, const unsigned char* h, con
 	if (post)
 	{
 		stage_begin(ctx, STAGE_POST);
-		r = check_kernel(ctx, launch_postprocess(pp, ctx->num_sms, s, aux, ctx->ev_fork, ctx->ev_join, average_done),
+		r = check_kernel(ctx, launch_postprocess(pp, ctx->num_sms, s, aux, ctx->ev_fork, ctx->ev_join, ctx->average_ready, average_flags(ctx)),
 			"postprocess");
 		stage_end(ctx, STAGE_POST);
 		if (r) return r;
-		if (!average_done) SW_CUDA(ctx, cudaMemcpyAsync(ctx->h_average, ctx->average.ptr, 16, cudaMemcpyDeviceToHost, s));
 	}
 	else if (f.dst && f.dst_is_device)
 	{
@@ -2003,7 +2004,6 @@ int finish_graph_frame(SwCtx* ctx, Staging& st, const SwFrameParams& p, bool pos
 	}
 	if (postprocess)
 	{
-		SW_CUDA(ctx, cudaEventRecord(ctx->average_ready, ctx->stream));
 		ctx->exposure_pending = true;
 		ctx->pending_config = post_config_clamped(post);
 		ctx->pending_dt = dt;
@@ -2121,17 +2121,14 @@ int sw_draw_frame(SwCtx* ctx, const SwFrameInput* in)
 		return r;
 	if (pslot >= 0)
 	{
-		// a frame in flight: the average kernel writes the average straight to host memory, where the next
-		// frame's exposure update reads it once the graph's average event has fired; the slot's output
-		// buffer is free once its previous copy-out has finished
-		pa.average = ctx->d_average_mapped;
+		// a frame in flight: the slot's output buffer is free once its previous copy-out has finished
 		if (ctx->d2h_pending[pslot]) SW_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->ev_d2h[pslot], 0));
 	}
 
 	// 3. capture the device work and update (or instantiate) the frame graph; with the graph off, the
 	// same work is launched directly (with per-stage timing events when timing is on)
 	auto enqueue = [&]() {
-		return enqueue_frame(ctx, f, h, off, rows, f.postprocess ? &pa : nullptr, pslot >= 0 ? ctx->average_ready : nullptr);
+		return enqueue_frame(ctx, f, h, off, rows, f.postprocess ? &pa : nullptr);
 	};
 	if (ctx->graph_enabled)
 	{
@@ -2551,7 +2548,6 @@ int sw_draw_frame_view(SwCtx* ctx, const SwViewFrameInput* in)
 	{
 		key.post = pa;
 		key.post.inv_scale_dev = reinterpret_cast<const float*>(d + vb.inv_scale);
-		key.post.average = ctx->d_average_mapped; // the frame's average colour goes straight to host memory
 	}
 	key.staging = st.host;
 	key.block_bytes = vb.bytes;
@@ -2591,7 +2587,7 @@ int sw_draw_frame_view(SwCtx* ctx, const SwViewFrameInput* in)
 			if (f.postprocess)
 			{
 				if ((rr = check_kernel(ctx, launch_postprocess(pp2, ctx->num_sms, s, aux, ctx->ev_fork, ctx->ev_join,
-												key.in_flight ? ctx->average_ready : nullptr),
+												ctx->average_ready, average_flags(ctx)),
 						 "postprocess")))
 					return rr;
 			}
