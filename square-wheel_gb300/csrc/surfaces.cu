@@ -7,13 +7,14 @@
 //
 // Work decomposition: the frame's surfaces form one flat texel index space (prefix sums of surface
 // areas, in descriptor order). A grid of (#SMs x resident blocks) threads strides over it, so surfaces
-// from 4x4 to 512x512 texels share one launch without tail effects. Each warp owns 32 consecutive
-// texels: lane 0 finds the first texel's surface by binary search over the prefix array, every lane
-// then steps forward to its own surface (at most a few steps, only across tiny surfaces). Each thread
-// rebuilds the reference's row-interpolated lightmap line entries it needs (the two vertical mixes of
-// the line buffer and the horizontal mix, in the reference's operation order), evaluates lighting and
-// stores its texel. Neighbouring threads read neighbouring TextureElements and share lightmap elements,
-// so texture reads and surface writes are coalesced and lightmap reads are L1 broadcasts.
+// from 4x4 to 512x512 texels share one launch without tail effects. A warp takes `runs` runs of 32 consecutive
+// texels: it finds the first texel's surface by a 32-way search of the prefix array, and every lane then steps
+// forward to its own surface (at most a few steps, only across tiny surfaces). Neighbouring lanes read
+// neighbouring TextureElements, so texture reads and surface writes are coalesced.
+// A directional lightmap goes through the reference's row buffer (surfaces.rs:477-502): where the 32 texels lie in one or two
+// surface rows (all but surfaces narrower than 17), the warp builds the line entries they touch together, one
+// component per lane from neighbouring floats, in shared memory, and each texel only mixes its two entries;
+// elsewhere, and for the three floats of a simple lightmap's element, every thread builds its two entries alone. Operations and their order are the reference's either way.
 #include "sw_kernels.cuh"
 
 #include <cmath>
@@ -61,16 +62,26 @@ struct Lm
 	float dev;
 	float col[3];
 };
+// Floats of a lightmap element: ambient, direction, deviation, colour; or the colour alone.
+template <bool DIRECTIONAL>
+constexpr uint32_t LM_FLOATS = DIRECTIONAL ? 10 : 3;
+static_assert(sizeof(SwDirectionalLightmapElement) == LM_FLOATS<true> * sizeof(float), "lightmap element");
 
 template <bool DIRECTIONAL>
-__device__ __forceinline__ Lm lm_load(const SurfaceKernelArgs& a, uint64_t index)
+__device__ __forceinline__ const float* lm_floats(const SurfaceKernelArgs& a)
+{
+	return DIRECTIONAL ? reinterpret_cast<const float*>(a.directional_lightmaps) : a.lightmaps;
+}
+
+template <bool DIRECTIONAL>
+__device__ __forceinline__ Lm lm_load(const float* p)
 {
 	Lm e;
 	if (DIRECTIONAL)
 	{
-		// 40-byte element, 8-byte aligned: five 64-bit read-only loads.
-		const float2* p = reinterpret_cast<const float2*>(a.directional_lightmaps + index);
-		const float2 q0 = __ldg(p + 0), q1 = __ldg(p + 1), q2 = __ldg(p + 2), q3 = __ldg(p + 3), q4 = __ldg(p + 4);
+		// 40-byte elements, 8-byte aligned in global and shared memory
+		const float2* q = reinterpret_cast<const float2*>(p);
+		const float2 q0 = q[0], q1 = q[1], q2 = q[2], q3 = q[3], q4 = q[4];
 		e.amb[0] = q0.x;
 		e.amb[1] = q0.y;
 		e.amb[2] = q1.x;
@@ -82,10 +93,9 @@ __device__ __forceinline__ Lm lm_load(const SurfaceKernelArgs& a, uint64_t index
 	}
 	else
 	{
-		const float* p = a.lightmaps + index * 3;
-		e.amb[0] = __ldg(p + 0);
-		e.amb[1] = __ldg(p + 1);
-		e.amb[2] = __ldg(p + 2);
+		e.amb[0] = p[0];
+		e.amb[1] = p[1];
+		e.amb[2] = p[2];
 	}
 	return e;
 }
@@ -187,81 +197,102 @@ __device__ __forceinline__ float light_shadow_factor(const SurfaceKernelArgs& a,
 							  : cube_side_fetch(maps + 4 * side_texels, m.size, -to_light.x, -to_light.y, az);
 }
 
-// The line buffer of the reference's row loop (surfaces.rs:477-502) for one thread's run of texels: the
-// entries line_lightmap[lu] and [lu + 1] of texel row v (the vertical mixes of lightmap rows lv and
-// lv + 1 at ratio kv), kept while the run stays in that row and column and shifted by one when it
-// steps into the next lightmap column, as the reference's row buffer holds them.
-template <bool DIRECTIONAL>
-struct LineCache
+// The fields of a SurfaceGpu that a texel's shading reads, loaded as 16-byte words. (The lightmap's are read where
+// they are needed: together they do not fit the registers.)
+struct Surf
 {
-	uint32_t si = 0xFFFFFFFFu, v = 0, lu = 0;
-	Lm line0, line1;
+	V3 start_pos, u, v, normal, u_norm, v_norm;
+	uint64_t tex_offset;
+	uint32_t tex_w, tex_h, flags;
+	int32_t tc0, tc1;
+	uint32_t num_lights;
+	const SurfaceGpu* g;
 };
-
-template <bool DIRECTIONAL>
-__device__ __forceinline__ void line_entries(const SurfaceKernelArgs& a, const SurfaceGpu& s, uint32_t si, uint32_t v,
-	uint32_t lv, uint32_t lu, float kv, LineCache<DIRECTIONAL>& c)
+__device__ __forceinline__ Surf load_surf(const SurfaceGpu* g)
 {
-	if (c.si == si && c.v == v && c.lu == lu) return;
-	const uint64_t row0 = uint64_t(s.lm_offset) + uint64_t(lv) * s.lm_width;
-	const uint64_t row1 = row0 + s.lm_width;
-	if (c.si == si && c.v == v && c.lu + 1 == lu)
-		c.line0 = c.line1;
-	else
-		c.line0 = lm_mix<DIRECTIONAL>(lm_load<DIRECTIONAL>(a, row1 + lu), lm_load<DIRECTIONAL>(a, row0 + lu), kv);
-	c.line1 = lm_mix<DIRECTIONAL>(lm_load<DIRECTIONAL>(a, row1 + lu + 1), lm_load<DIRECTIONAL>(a, row0 + lu + 1), kv);
-	c.si = si;
-	c.v = v;
-	c.lu = lu;
+	static_assert(offsetof(SurfaceGpu, tex_offset) == 80 && offsetof(SurfaceGpu, tex_h) == 96 && offsetof(SurfaceGpu, lm_offset) == 112 &&
+			offsetof(SurfaceGpu, inv_scale) == 72,
+		"SurfaceGpu layout");
+	const float4* f = reinterpret_cast<const float4*>(g);
+	const float4 a = f[0], b = f[1], c = f[2], d = f[3], e = f[4];
+	const uint4* w = reinterpret_cast<const uint4*>(g);
+	const uint4 t = w[5], q = w[6];
+	Surf s;
+	s.start_pos = mkv3(a.x, a.y, a.z);
+	s.u = mkv3(a.w, b.x, b.y);
+	s.v = mkv3(b.z, b.w, c.x);
+	s.normal = mkv3(c.y, c.z, c.w);
+	s.u_norm = mkv3(d.x, d.y, d.z);
+	s.v_norm = mkv3(d.w, e.x, e.y);
+	s.tex_offset = uint64_t(t.x) | (uint64_t(t.y) << 32);
+	s.tex_w = t.w;
+	s.tex_h = q.x;
+	s.flags = q.y;
+	s.tc0 = int32_t(q.z);
+	s.tc1 = int32_t(q.w);
+	s.num_lights = g->num_lights;
+	s.g = g;
+	return s;
+}
+
+// Line entries of one surface row, by the warp (`s` the same in every lane): the vertical mixes of lightmap rows lv
+// and lv + 1 at ratio kv for the columns [lu0, lu1 + 1] that texels [u0, u1] of row v read, as consecutive floats
+// at `line`. Returns their number.
+__device__ __forceinline__ uint32_t build_line(const SurfaceKernelArgs& a, const SurfaceGpu& s, uint32_t v, uint32_t u0, uint32_t u1, float* line,
+	uint32_t lane)
+{
+	constexpr uint32_t F = LM_FLOATS<true>;
+	const uint32_t base_v = v + s.lm_shift1;
+	const uint32_t lu0 = (u0 + s.lm_shift0) >> s.lm_log2, lu1 = (u1 + s.lm_shift0) >> s.lm_log2;
+	const float kv = mad2(float(base_v & ((1u << s.lm_log2) - 1u)), s.inv_scale, s.k_shift);
+	const float omr = fsub(1.0f, kv);
+	const float* row0 = lm_floats<true>(a) + (uint64_t(s.lm_offset) + uint64_t(base_v >> s.lm_log2) * s.lm_width + lu0) * F;
+	const float* row1 = row0 + uint64_t(s.lm_width) * F;
+	const uint32_t n = (lu1 - lu0 + 2) * F;
+	for (uint32_t i = lane; i < n; i += 32) line[i] = mad2(__ldg(row1 + i), kv, fmul(__ldg(row0 + i), omr));
+	return n;
 }
 
 // The texel's lightmap element (surfaces.rs:504-513): the horizontal mix of its two line entries.
-template <bool DIRECTIONAL>
-__device__ __forceinline__ Lm lightmap_sample(const SurfaceKernelArgs& a, const SurfaceGpu& s, uint32_t si, uint32_t u,
-	uint32_t v, LineCache<DIRECTIONAL>& c)
+__device__ __forceinline__ Lm mix_line(const SurfaceGpu& s, const float* line, uint32_t u, uint32_t u0)
 {
-	const uint32_t log2 = s.lm_log2;
-	const uint32_t mask = (1u << log2) - 1u;
-	const uint32_t base_v = v + s.lm_shift1;
-	const float kv = mad2(float(base_v & mask), s.inv_scale, s.k_shift);
+	constexpr uint32_t F = LM_FLOATS<true>;
 	const uint32_t base_u = u + s.lm_shift0;
-	const float ku = mad2(float(base_u & mask), s.inv_scale, s.k_shift);
-	line_entries<DIRECTIONAL>(a, s, si, v, base_v >> log2, base_u >> log2, kv, c);
-	return lm_mix<DIRECTIONAL>(c.line1, c.line0, ku);
+	const float ku = mad2(float(base_u & ((1u << s.lm_log2) - 1u)), s.inv_scale, s.k_shift);
+	const float* e = line + ((base_u >> s.lm_log2) - ((u0 + s.lm_shift0) >> s.lm_log2)) * F;
+	return lm_mix<true>(lm_load<true>(e + F), lm_load<true>(e), ku);
 }
 
 // The same element for a single texel: both line entries built for it alone.
 template <bool DIRECTIONAL>
 __device__ __forceinline__ Lm lightmap_sample_once(const SurfaceKernelArgs& a, const SurfaceGpu& s, uint32_t u, uint32_t v)
 {
+	constexpr uint32_t F = LM_FLOATS<DIRECTIONAL>;
 	const uint32_t log2 = s.lm_log2;
 	const uint32_t mask = (1u << log2) - 1u;
 	const uint32_t base_v = v + s.lm_shift1;
 	const float kv = mad2(float(base_v & mask), s.inv_scale, s.k_shift);
 	const uint32_t base_u = u + s.lm_shift0;
-	const uint32_t lu = base_u >> log2;
 	const float ku = mad2(float(base_u & mask), s.inv_scale, s.k_shift);
-	const uint64_t row0 = uint64_t(s.lm_offset) + uint64_t(base_v >> log2) * s.lm_width;
-	const uint64_t row1 = row0 + s.lm_width;
-	const Lm line0 = lm_mix<DIRECTIONAL>(lm_load<DIRECTIONAL>(a, row1 + lu), lm_load<DIRECTIONAL>(a, row0 + lu), kv);
-	const Lm line1 = lm_mix<DIRECTIONAL>(lm_load<DIRECTIONAL>(a, row1 + lu + 1), lm_load<DIRECTIONAL>(a, row0 + lu + 1), kv);
+	const float* row0 = lm_floats<DIRECTIONAL>(a) + (uint64_t(s.lm_offset) + uint64_t(base_v >> log2) * s.lm_width + (base_u >> log2)) * F;
+	const float* row1 = row0 + uint64_t(s.lm_width) * F;
+	const Lm line0 = lm_mix<DIRECTIONAL>(lm_load<DIRECTIONAL>(row1), lm_load<DIRECTIONAL>(row0), kv);
+	const Lm line1 = lm_mix<DIRECTIONAL>(lm_load<DIRECTIONAL>(row1 + F), lm_load<DIRECTIONAL>(row0 + F), kv);
 	return lm_mix<DIRECTIONAL>(line1, line0, ku);
 }
 
 // Lighting of one texel (surfaces.rs:515-842) with its lightmap element `l` (when the surface has a
 // lightmap); returns the ColorVec before conversion.
 template <bool DIRECTIONAL>
-__device__ __forceinline__ CV shade_texel(const SurfaceKernelArgs& a, const SurfaceGpu& s, uint64_t texel, uint32_t u,
+__device__ __forceinline__ CV shade_texel(const SurfaceKernelArgs& a, const Surf& s, uint64_t texel, uint32_t u,
 	uint32_t v, V3 cam, const Lm& l)
 {
 	const uint32_t tex_flags = s.flags & 7u;
 	const bool use_normal_map = (tex_flags & SW_TEX_HAS_NORMAL_MAP) != 0;
 	const int spec = (tex_flags & SW_TEX_HAS_NON_ONE_ROUGHNESS) ? ((tex_flags & SW_TEX_IS_METAL) ? 2 : 1) : 0;
 
-	const V3 u_vec = mkv3(s.u[0], s.u[1], s.u[2]);
-	const V3 v_vec = mkv3(s.v[0], s.v[1], s.v[2]);
-	const V3 bnormal = mkv3(s.normal[0], s.normal[1], s.normal[2]);
-	const V3 pos = v3sma(u_vec, float(u), v3sma(v_vec, float(v), mkv3(s.start_pos[0], s.start_pos[1], s.start_pos[2])));
+	const V3 bnormal = s.normal;
+	const V3 pos = v3sma(s.u, float(u), v3sma(s.v, float(v), s.start_pos));
 
 	V3 tn = mkv3(0.0f, 0.0f, 1.0f);
 	float rough = 0.0f;
@@ -291,8 +322,7 @@ __device__ __forceinline__ CV shade_texel(const SurfaceKernelArgs& a, const Surf
 		}
 		else
 		{
-			const V3 u_norm = mkv3(s.u_norm[0], s.u_norm[1], s.u_norm[2]);
-			const V3 v_norm = mkv3(s.v_norm[0], s.v_norm[1], s.v_norm[2]);
+			const V3 u_norm = s.u_norm, v_norm = s.v_norm;
 			const V3 normal = use_normal_map ? tn : mkv3(0.0f, 0.0f, 1.0f);
 			const V3 to_cam = v3sub(cam, pos);
 			const V3 to_cam_ts = mkv3(v3dot(to_cam, u_norm), v3dot(to_cam, v_norm), v3dot(to_cam, bnormal));
@@ -335,8 +365,7 @@ __device__ __forceinline__ CV shade_texel(const SurfaceKernelArgs& a, const Surf
 		V3 normal = bnormal;
 		if (use_normal_map)
 		{
-			const V3 u_norm = mkv3(s.u_norm[0], s.u_norm[1], s.u_norm[2]);
-			const V3 v_norm = mkv3(s.v_norm[0], s.v_norm[1], s.v_norm[2]);
+			const V3 u_norm = s.u_norm, v_norm = s.v_norm;
 			normal = mkv3(mad2(tn.x, u_norm.x, mad2(tn.y, v_norm.x, fmul(tn.z, bnormal.x))),
 				mad2(tn.x, u_norm.y, mad2(tn.y, v_norm.y, fmul(tn.z, bnormal.y))),
 				mad2(tn.x, u_norm.z, mad2(tn.y, v_norm.z, fmul(tn.z, bnormal.z))));
@@ -356,10 +385,10 @@ __device__ __forceinline__ CV shade_texel(const SurfaceKernelArgs& a, const Surf
 		}
 		for (uint32_t li = 0; li < s.num_lights; ++li)
 		{
-			const SwLight& L = a.lights[s.lights[li]];
+			const SwLight& L = a.lights[s.g->lights[li]];
 			const V3 to_light = v3sub(mkv3(L.position[0], L.position[1], L.position[2]), pos);
 			const float tl_len2 = fmaxf(v3dot(to_light, to_light), MIN_POSITIVE_VALUE);
-			const float sdf = fmul(light_shadow_factor(a, s.lights[li], to_light), fmaxf(fsub(inv_fast(tl_len2), L.inv_square_radius), 0.0f));
+			const float sdf = fmul(light_shadow_factor(a, s.g->lights[li], to_light), fmaxf(fsub(inv_fast(tl_len2), L.inv_square_radius), 0.0f));
 			float di = 0.0f;
 			if (spec != 2) di = fmaxf(fmul(v3dot(normal, to_light), inv_sqrt_fast(tl_len2)), 0.0f);
 			float si = 0.0f;
@@ -403,109 +432,127 @@ __device__ __forceinline__ typename P::T emissive_mix(const SurfaceKernelArgs& a
 	return P::from_ci(m);
 }
 
-// K consecutive texels of the flat texel space per thread (a warp owns 32 * K): the thread's surface is
-// found once (lane 0's binary search for the warp, then forward steps), its later texels step along the
-// row and into following surfaces, and its line-buffer entries carry from texel to texel. K = 1 runs
-// four blocks per SM (64 registers, a few bytes spilled): the kernel issues ~600 instructions per
-// texel of exact, unfused f32 shading and integer indexing, and more resident warps hide their latency
-// better than fewer, longer threads (K = 4 and its shared line entries measured no faster).
-template <class P, bool DIRECTIONAL, int K>
-__global__ void __launch_bounds__(256, K == 1 ? 4 : 2) surf_build_kernel(SurfaceKernelArgs a)
+// Surface of texel t: the largest i with prefix[i] <= t, by the whole warp (32 probes a round).
+__device__ __forceinline__ uint32_t find_surface(const uint64_t* prefix, uint32_t n, uint64_t t, uint32_t lane)
+{
+	uint32_t lo = 0; // prefix[lo] <= t < prefix[lo + n]
+	while (n > 1)
+	{
+		const uint32_t step = (n + 31) >> 5;
+		const uint32_t i = lane * step;
+		const uint32_t below = __popc(__ballot_sync(0xFFFFFFFFu, i < n && __ldg(prefix + lo + i) <= t)); // >= 1: lane 0
+		const uint32_t k = (below - 1) * step;
+		lo += k;
+		n = min(step, n - k);
+	}
+	return lo;
+}
+
+// Bound by issue (78% of the slots): exact, unfused f32 shading and integer indexing, 500 instructions per 32 texels.
+// One launch over 4,096 surfaces of 4x4 to 512x512 texels (46.9 M texels, directional lightmaps, half of the
+// materials specular, colour64): 765 us, 61 Gtexel/s; 1,119 us and 628 instructions with two lightmap entries per
+// texel from global memory and a serial search per 32 texels. Four blocks per SM (64 registers, 44 bytes spilled):
+// three measured 8% slower, five 24% (spills).
+template <class P, bool DIRECTIONAL>
+__global__ void __launch_bounds__(256, 4) surf_build_kernel(SurfaceKernelArgs a, uint32_t runs)
 {
 	typedef typename P::T T;
+	// two rows' entries of 32 texels, at least one texel apart
+	__shared__ __align__(16) float s_line[8][DIRECTIONAL ? 34 * LM_FLOATS<true> : 1];
 	T* arena = static_cast<T*>(a.arena);
 	const uint64_t total = a.counts ? a.counts->total_texels : a.total_work;
 	const V3 cam = a.cam_pos_dev ? mkv3(a.cam_pos_dev[0], a.cam_pos_dev[1], a.cam_pos_dev[2])
 								 : mkv3(a.cam_pos[0], a.cam_pos[1], a.cam_pos[2]);
 	const uint32_t num_surfaces = a.counts ? a.counts->num_surfaces : a.num_surfaces;
-	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x * K;
+	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x * runs;
 	const uint32_t lane = threadIdx.x & 31u;
-	const uint64_t warp_first = (uint64_t(blockIdx.x) * blockDim.x + (threadIdx.x & ~31u)) * K;
-	for (uint64_t wbase = a.work_begin + warp_first; wbase < total; wbase += stride)
+	float* line = s_line[threadIdx.x >> 5];
+	for (uint64_t first = a.work_begin + (uint64_t(blockIdx.x) * blockDim.x + (threadIdx.x & ~31u)) * runs; first < total; first += stride)
 	{
-		const uint64_t t0 = wbase + uint64_t(lane) * K;
-		// Surface of the warp's first texel (binary search by lane 0), then forward steps per lane.
-		uint32_t s0 = 0;
-		if (lane == 0)
-		{
-			uint32_t lo = 0, hi = num_surfaces; // prefix[lo] <= wbase < prefix[hi]
-			while (hi - lo > 1)
-			{
-				const uint32_t mid = (lo + hi) >> 1;
-				if (__ldg(a.work_prefix + mid) <= wbase)
-					lo = mid;
-				else
-					hi = mid;
-			}
-			s0 = lo;
-		}
-		uint32_t si = __shfl_sync(0xFFFFFFFFu, s0, 0);
-		if (t0 >= total) continue;
-		uint64_t next = __ldg(a.work_prefix + si + 1);
-		while (next <= t0)
-		{
-			++si;
-			next = __ldg(a.work_prefix + si + 1);
-		}
-		uint32_t local = uint32_t(t0 - __ldg(a.work_prefix + si));
-		uint32_t width = a.surfaces[si].width;
-		uint32_t v, u;
-		div_row(local, width, a.surfaces[si].inv_width, v, u);
-		[[maybe_unused]] LineCache<DIRECTIONAL> cache;
+		uint32_t si = find_surface(a.work_prefix, num_surfaces, first, lane);
+		uint64_t begin = __ldg(a.work_prefix + si), next = __ldg(a.work_prefix + si + 1);
 #pragma unroll 1
-		for (int k = 0; k < K; ++k)
+		for (uint32_t run = 0; run < runs; ++run)
 		{
-			if (k > 0)
+			const uint64_t t = first + run * 32 + lane;
+			const bool active = t < total;
+			const uint32_t mask = __ballot_sync(0xFFFFFFFFu, active);
+			if (!mask) break;
+			if (active && next <= t)
 			{
-				const uint64_t t = t0 + uint64_t(k);
-				if (t >= total) break;
-				if (t >= next)
+				do
 				{
-					// the next surface with texels: its first texel
-					do
-					{
-						++si;
-						next = __ldg(a.work_prefix + si + 1);
-					} while (next <= t);
-					width = a.surfaces[si].width;
-					local = 0;
-					u = 0;
-					v = 0;
-				}
-				else
+					++si;
+					begin = next;
+					next = __ldg(a.work_prefix + si + 1);
+				} while (next <= t);
+			}
+			const SurfaceGpu* g = a.surfaces + si;
+			const uint32_t local = uint32_t(t - begin);
+			uint32_t u = 0, v = 0;
+			if (active) div_row(local, g->width, g->inv_width, v, u);
+			// the run's surface rows: row 0 is the first lane's, row 1 the first other one (a row's lanes are
+			// neighbours: its last texel is its first plus its lanes)
+			bool together = false;
+			uint32_t row1 = 0, u0 = 0, u1 = 0, line1 = 0;
+			if constexpr (DIRECTIONAL)
+			{
+				const uint32_t si0 = __shfl_sync(0xFFFFFFFFu, si, 0), v0 = __shfl_sync(0xFFFFFFFFu, v, 0);
+				const uint32_t row0 = __ballot_sync(0xFFFFFFFFu, active && si == si0 && v == v0);
+				const uint32_t rest = mask & ~row0;
+				const uint32_t lane1 = rest ? uint32_t(__ffs(int(rest))) - 1u : 0u;
+				const uint32_t si1 = __shfl_sync(0xFFFFFFFFu, si, lane1), v1 = __shfl_sync(0xFFFFFFFFu, v, lane1);
+				row1 = __ballot_sync(0xFFFFFFFFu, ((rest >> lane) & 1u) && si == si1 && v == v1);
+				together = rest == row1;
+				u0 = __shfl_sync(0xFFFFFFFFu, u, 0);
+				u1 = __shfl_sync(0xFFFFFFFFu, u, lane1);
+				if (together)
 				{
-					++local;
-					if (++u == width)
+					const SurfaceGpu& s0 = a.surfaces[si0];
+					__syncwarp(); // the last run's entries have been read
+					if (s0.flags & SW_SG_LIGHTMAP) line1 = build_line(a, s0, v0, u0, u0 + __popc(row0) - 1, line, lane);
+					if (row1)
 					{
-						u = 0;
-						++v;
+						const SurfaceGpu& s1 = a.surfaces[si1];
+						if (s1.flags & SW_SG_LIGHTMAP) build_line(a, s1, v1, u1, u1 + __popc(row1) - 1, line + line1, lane);
 					}
+					__syncwarp();
 				}
 			}
-			const SurfaceGpu& s = a.surfaces[si];
+			if (!active) continue;
+			const Surf s = load_surf(g);
+			const uint32_t flags = s.flags;
 			T out = T(0);
-			const bool diffuse_layer = (s.flags & SW_SG_DIFFUSE) != 0;
+			const bool diffuse_layer = (flags & SW_SG_DIFFUSE) != 0;
 			if (diffuse_layer)
 			{
-				const uint32_t sv = wrap_side(s.tc1 + int32_t(v), s.tex_h, s.tex_mask[1]);
-				const uint32_t su = wrap_side(s.tc0 + int32_t(u), s.tex_w, s.tex_mask[0]);
+				const uint2 masks = *reinterpret_cast<const uint2*>(g->tex_mask);
+				const uint32_t sv = wrap_side(s.tc1 + int32_t(v), s.tex_h, masks.y);
+				const uint32_t su = wrap_side(s.tc0 + int32_t(u), s.tex_w, masks.x);
 				const uint64_t texel =
 					__ldg(reinterpret_cast<const unsigned long long*>(a.texels) + s.tex_offset + uint64_t(sv) * s.tex_w + su);
 				Lm l;
-				if (s.flags & SW_SG_LIGHTMAP)
+				if (flags & SW_SG_LIGHTMAP)
 				{
-					if constexpr (K == 1)
-						l = lightmap_sample_once<DIRECTIONAL>(a, s, u, v);
+					const bool second = (row1 >> lane) & 1u;
+					if (DIRECTIONAL && together)
+						l = mix_line(*g, second ? line + line1 : line, u, second ? u1 : u0);
 					else
-						l = lightmap_sample<DIRECTIONAL>(a, s, si, u, v, cache);
+						l = lightmap_sample_once<DIRECTIONAL>(a, *g, u, v);
 				}
 				out = P::from_cv(shade_texel<DIRECTIONAL>(a, s, texel, u, v, cam, l));
 			}
-			if (s.flags & SW_SG_EMISSIVE) out = emissive_mix<P>(a, s, u, v, out, diffuse_layer);
-			arena[s.out_offset + local] = out;
+			if (flags & SW_SG_EMISSIVE) out = emissive_mix<P>(a, *g, u, v, out, diffuse_layer);
+			arena[g->out_offset + local] = out;
 		}
 	}
 	pdl_trigger(); // the tile pass may be scheduled (it waits for this grid before reading the arena)
+}
+
+template <class P, bool DIRECTIONAL>
+void launch_build(const SurfaceKernelArgs& args, unsigned blocks, uint32_t runs, cudaStream_t stream)
+{
+	surf_build_kernel<P, DIRECTIONAL><<<blocks, 256, 0, stream>>>(args, runs);
 }
 
 } // namespace
@@ -515,32 +562,21 @@ int launch_surface_build(const SurfaceKernelArgs& args, uint32_t pixel_format, i
 {
 	const uint64_t work = args.counts ? work_hint : args.total_work - args.work_begin;
 	if (work == 0 && !args.counts) return 0;
-	const int threads = 256;
-	// texels per thread: as tuned (by default 1: the shading arithmetic, not the lightmap mixes, bounds the
-	// kernel, and carrying line entries over 4 texels measured no faster)
-	const int k = texels_per_thread == 4 ? 4 : 1;
-	uint64_t blocks_needed = (work + uint64_t(threads) * k - 1) / (uint64_t(threads) * k);
+	// Runs of 32 texels per warp and search: one while the launch is not several times what the GPU holds at once
+	// (a frame's 0.6 M texels hide latency by parallelism), up to 8 for large batches; at least 4 when tuned so.
+	const uint64_t resident = uint64_t(num_sms) * 2048 * 2;
+	uint64_t runs = std::min<uint64_t>(std::max<uint64_t>(work / resident, 1), 8);
+	if (texels_per_thread == 4) runs = std::max<uint64_t>(runs, 4);
+	uint64_t blocks_needed = (work + 256 * runs - 1) / (256 * runs);
 	if (args.counts && blocks_needed < uint64_t(num_sms)) blocks_needed = uint64_t(num_sms);
-	// At most blocks_per_sm blocks per SM (several waves of resident blocks): small frames get one
-	// texel per thread (latency hidden by parallelism), large batches stride.
-	uint64_t blocks_max = uint64_t(num_sms) * uint64_t(blocks_per_sm);
-	unsigned blocks = unsigned(blocks_needed < blocks_max ? blocks_needed : blocks_max);
-	const bool c64 = pixel_format == SW_PIXEL_C64;
-	if (k == 4)
-	{
-		if (c64)
-			args.directional ? surf_build_kernel<PixC64, true, 4><<<blocks, threads, 0, stream>>>(args)
-							 : surf_build_kernel<PixC64, false, 4><<<blocks, threads, 0, stream>>>(args);
-		else
-			args.directional ? surf_build_kernel<PixC32, true, 4><<<blocks, threads, 0, stream>>>(args)
-							 : surf_build_kernel<PixC32, false, 4><<<blocks, threads, 0, stream>>>(args);
-	}
-	else if (c64)
-		args.directional ? surf_build_kernel<PixC64, true, 1><<<blocks, threads, 0, stream>>>(args)
-						 : surf_build_kernel<PixC64, false, 1><<<blocks, threads, 0, stream>>>(args);
+	// At most blocks_per_sm blocks per SM (several waves of resident blocks); large batches stride.
+	const uint64_t blocks_max = uint64_t(num_sms) * uint64_t(blocks_per_sm);
+	const unsigned blocks = unsigned(std::min(blocks_needed, blocks_max));
+	const uint32_t r = uint32_t(runs);
+	if (pixel_format == SW_PIXEL_C64)
+		args.directional ? launch_build<PixC64, true>(args, blocks, r, stream) : launch_build<PixC64, false>(args, blocks, r, stream);
 	else
-		args.directional ? surf_build_kernel<PixC32, true, 1><<<blocks, threads, 0, stream>>>(args)
-						 : surf_build_kernel<PixC32, false, 1><<<blocks, threads, 0, stream>>>(args);
+		args.directional ? launch_build<PixC32, true>(args, blocks, r, stream) : launch_build<PixC32, false>(args, blocks, r, stream);
 	return int(cudaGetLastError());
 }
 

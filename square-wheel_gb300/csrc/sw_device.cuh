@@ -41,8 +41,10 @@ cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
 	return cudaLaunchKernelEx(&cfg, kernel, static_cast<Args&&>(args)...);
 }
 
-__device__ __forceinline__ float inv_fast(float x) { return __fdiv_rn(1.0f, x); }
-__device__ __forceinline__ float inv_sqrt_fast(float x) { return __fdiv_rn(1.0f, __fsqrt_rn(x)); }
+// 1 / x and 1 / sqrt(x), each operation rounded once: the correctly rounded reciprocal is the correctly rounded
+// quotient of 1 and x, and takes fewer instructions than the general division.
+__device__ __forceinline__ float inv_fast(float x) { return __frcp_rn(x); }
+__device__ __forceinline__ float inv_sqrt_fast(float x) { return __frcp_rn(__fsqrt_rn(x)); }
 __device__ __forceinline__ float fmul(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float fsub(float a, float b) { return __fsub_rn(a, b); }
