@@ -11,15 +11,15 @@
 //     start and step of the mode's interpolants (the span setup of rasterizer.rs:329-422 / 513-556 /
 //     686-703), evaluated once per (draw, row) over the whole span with the frame as clip rectangle
 //     (the reference's num_threads == 1 ClipRect).
-//   raster_tiles: one 256-thread CTA per 64x16 tile, each thread a 1x4 pixel strip of one row (about
-//     one wave of CTAs at 1080p). The CTA streams over the draws in submission order, 256 at a time;
-//     each thread tests one draw's box against the tile and a ballot + prefix sum compacts the hits
-//     (with their draw records) into shared memory in order. For batches of 32 hits the CTA stages
-//     their 16 rows of this tile in shared memory with parallel loads; every thread then walks the
-//     hits in order for its strip: for span pixel i it takes start + i*step (the reference's repeated
-//     wrapping addition), the per-pixel z division and the texel address, issues its four texel loads
-//     at once and blends them in submission order into registers. Blending order is the reference's,
-//     the frame buffer is read and written once, and coverage and texel addresses are bit-exact.
+//   raster_tiles: one 256-thread CTA per 64x16 tile, each thread a 1x4 pixel strip of one row; every warp
+//     works on its own two rows and never waits for the others. It streams over its bin's draws in submission
+//     order, 32 at a time: each lane tests one draw's box against the warp's rows and a ballot compacts the
+//     hits in order; the lanes then fetch the hits' rows and draw records together (16 hits a round trip) into
+//     shared memory, and every thread walks the hits in order for its strip: for span pixel i it takes start +
+//     i*step (the reference's repeated wrapping addition), the per-pixel z division and the texel address,
+//     issues its four texel loads at once and blends them in submission order into registers. Blending order
+//     is the reference's, the frame buffer is read and written once, and coverage and texel addresses are
+//     bit-exact.
 #include "sw_kernels.cuh"
 #include "warp_prep.cuh"
 
@@ -624,14 +624,13 @@ __global__ void __launch_bounds__(256) raster_setup_kernel(RasterArgs a)
 			// Rows outside the host's row range have no record; clamp the box to it.
 			by0 = max(by0, dr.y0);
 			by1 = min(by1, dr.y0 + int32_t(dr.nrows));
-			a.boxes[di] = (np > 0 && bx0 < bx1 && by0 < by1) ? RasterBox{int16_t(bx0), int16_t(by0), int16_t(bx1), int16_t(by1)}
-																: RasterBox{0, 0, 0, 0};
+			a.boxes[di] = (np > 0 && bx0 < bx1 && by0 < by1) ? RasterBox{int16_t(bx0), int16_t(by0), int16_t(bx1), int16_t(by1), dr.row_base - uint32_t(dr.y0), 0u}
+																: RasterBox{0, 0, 0, 0, 0u, 0u};
 			RasterDraw rd;
 			rd.tex_offset = d.tex_offset;
 			rd.tex_w = d.tex_size[0];
 			rd.tex_h = d.tex_size[1];
-			rd.row_base = dr.row_base;
-			rd.y0 = dr.y0;
+			rd.reserved = 0;
 			rd.mode = d.mode;
 			rd.blend = uint16_t(d.blend);
 			rd.tex_source = uint16_t(d.tex_source);
@@ -695,8 +694,6 @@ __device__ __forceinline__ uint64_t pixel_address(const RasterRow& r, uint32_t m
 	if (mode == SW_RASTER_LINE_Z_CORRECTED) return uint32_t(t0 >> 16) + uint32_t(t1 >> 16) * tex_w;
 	return uint64_t(int64_t(wadd(t0 >> 16, wmul(t1 >> 16, int32_t(tex_w)))));
 }
-
-constexpr int BATCH = 32; // draws whose tile rows are staged in shared memory at a time
 
 // A thread's strip of one triangle row (fill_triangle_part's pixel loop, rasterizer.rs:1213-1279):
 // texture coordinates and light of span pixel i are start + i * step (the reference's per-pixel
@@ -763,7 +760,7 @@ __device__ __forceinline__ void triangle_strip(const RasterArgs& a, const Raster
 }
 
 // The bloom downscale of a tile's final colour64 pixels (downscale_hdr_buffer, postprocessor.rs:792-844):
-// the pixels go to shared memory (the row staging area, free once the draws are done), each bloom cell
+// the pixels go to shared memory (the warps' staging area, free once the draws are done), each bloom cell
 // whose S x S source pixels lie in the tile gets their box average (i32 lanes, (sum * (256 / S^2)) >> 8),
 // and the tile's part of each bloom line's lane sums is added to the line's global sums. The sums are
 // wrapping i32 additions, associative and commutative, so the atomics keep them exact in any order.
@@ -773,10 +770,9 @@ __device__ __forceinline__ void bloom_epilogue(const RasterArgs& a, const uint64
 {
 	constexpr int TPR = TILE_W / STRIP;
 	static_assert(TILE_W % 8 == 0 && TILE_H % 8 == 0, "bloom cells must not straddle tiles");
-	static_assert(size_t(TILE_W) * TILE_H * 8 <= sizeof(RasterRow) * BATCH * TILE_H, "tile pixels fit the row staging");
 	__shared__ int32_t s_ls[TILE_H / 2][4];
 	uint64_t* s_pix = static_cast<uint64_t*>(staging);
-	__syncthreads(); // the row staging area is free
+	__syncthreads(); // the staging area is free
 	{
 		const int ly = tid / TPR, lx = (tid % TPR) * STRIP;
 #pragma unroll
@@ -915,118 +911,152 @@ struct TileShape
 };
 constexpr TileShape TILE_SHAPES[SW_RASTER_TILE_VARIANTS] = {{64, 16, 4}, {32, 32, 4}, {128, 8, 4}, {64, 32, 8}, {32, 16, 2}};
 
+// STRIP pixels of a row from / to memory: 16 bytes at a time where `vec` says that the address allows it and the
+// whole strip lies in the row.
+template <class T, int STRIP>
+__device__ __forceinline__ void load_strip(T (&pix)[STRIP], const T* p, int n, bool vec)
+{
+	constexpr int W = 16 / int(sizeof(T));
+	if constexpr (STRIP % W == 0)
+		if (vec && n >= STRIP)
+		{
+#pragma unroll
+			for (int k = 0; k < STRIP; k += W) *reinterpret_cast<uint4*>(&pix[k]) = *reinterpret_cast<const uint4*>(p + k);
+			return;
+		}
+#pragma unroll
+	for (int k = 0; k < STRIP; ++k)
+		if (k < n) pix[k] = p[k];
+}
+template <class T, int STRIP>
+__device__ __forceinline__ void store_strip(const T (&pix)[STRIP], T* p, int n, bool vec)
+{
+	constexpr int W = 16 / int(sizeof(T));
+	if constexpr (STRIP % W == 0)
+		if (vec && n >= STRIP)
+		{
+#pragma unroll
+			for (int k = 0; k < STRIP; k += W) *reinterpret_cast<uint4*>(p + k) = *reinterpret_cast<const uint4*>(&pix[k]);
+			return;
+		}
+#pragma unroll
+	for (int k = 0; k < STRIP; ++k)
+		if (k < n) p[k] = pix[k];
+}
+template <class T>
+__device__ __forceinline__ bool rows_aligned(const T* p, uint32_t pitch)
+{
+	return ((reinterpret_cast<uintptr_t>(p) | (uintptr_t(pitch) * sizeof(T))) & 15) == 0;
+}
+
+// Bound by latency: list -> box -> row and draw records -> texels are four dependent round trips per tile, so what
+// counts is how many warps are in flight and that none waits for another (with the tile's draws compacted and staged
+// by the CTA between barriers, 26 KB of shared memory and four CTAs per SM, a pass over a sheet of 46.9 M colour64
+// pixels took 103 us more of 1,620, and a 1920x1080 frame 4 us more of 49). Six CTAs per SM (40 registers, a few bytes spilled) measured 1% faster than four.
 template <class P, int TILE_W, int TILE_H, int STRIP>
-__global__ void __launch_bounds__(256) raster_tiles_kernel(RasterArgs a)
+__global__ void __launch_bounds__(256, 6) raster_tiles_kernel(RasterArgs a)
 {
 	static_assert((TILE_W / STRIP) * TILE_H == 256, "256 threads per tile");
 	constexpr int TPR = TILE_W / STRIP; // threads per tile row
+	constexpr int RPW = 32 / TPR;       // rows per warp
+	constexpr int BATCH = 32 / RPW;     // hits whose rows the warp stages at a time, one row record per lane
+	static_assert(32 % TPR == 0, "whole rows per warp");
 	typedef typename P::T T;
-	__shared__ uint32_t s_warp_counts[8];
-	__shared__ RasterDraw s_rd[256];
-	__shared__ RasterBox s_box[256];
-	__shared__ __align__(16) RasterRow s_row[BATCH][TILE_H]; // also the bloom epilogue's pixel staging (8-byte lanes)
+	struct WarpShared
+	{
+		uint4 hit[32]; // draw, row offset, first row, end row
+		RasterRow row[BATCH][RPW];
+		RasterDraw rd[BATCH];
+	};
+	constexpr size_t SMEM = sizeof(WarpShared) * 8, BLOOM = P::FORMAT == SW_PIXEL_C64 ? size_t(TILE_W) * TILE_H * 8 : 0;
+	__shared__ __align__(16) unsigned char s_mem[SMEM > BLOOM ? SMEM : BLOOM]; // also the bloom epilogue's pixel staging
 
 	const int tiles_x = (a.width + TILE_W - 1) / TILE_W;
 	const int tx0 = int(blockIdx.x % tiles_x) * TILE_W;
 	const int ty0 = int(blockIdx.x / tiles_x) * TILE_H;
-	const int tid = threadIdx.x;
+	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+	WarpShared& sw = reinterpret_cast<WarpShared*>(s_mem)[warp];
 	const int ly = tid / TPR;
 	pdl_wait(); // the surface build (launched before this kernel) has completed
-	const uint32_t num_draws = a.counts ? a.counts->num_draws : a.num_draws;
 	const int xb = tx0 + (tid % TPR) * STRIP; // first pixel of this thread's strip
 	const int y = ty0 + ly;
 	const bool row_valid = y < a.height;
-	const int tx1 = min(tx0 + TILE_W, a.width), ty1 = min(ty0 + TILE_H, a.height);
+	const int in_row = row_valid ? a.width - xb : 0; // the strip's pixels inside the frame (at most STRIP of them)
+	const int tx1 = min(tx0 + TILE_W, a.width);
+	const int wy0 = ty0 + warp * RPW, wy1 = min(wy0 + RPW, a.height); // the warp's rows
 
-	T* fb = static_cast<T*>(a.framebuffer);
+	T* fb = static_cast<T*>(a.framebuffer) + int64_t(y) * a.width + xb;
+	const bool fb_vec = rows_aligned(static_cast<const T*>(a.framebuffer), uint32_t(a.width));
 	const T* arena = static_cast<const T*>(a.arena);
 	const T* skybox = static_cast<const T*>(a.skybox);
 	T pix[STRIP];
+	// ColorVec::from_color_f32x3(&[32.0, 16.0, 8.0]).into(), partial_renderer.rs:255
+	const T background = P::FORMAT == SW_PIXEL_C64 ? T(8ull | (16ull << 16) | (32ull << 32)) : T(0x00201008u);
 #pragma unroll
-	for (int k = 0; k < STRIP; ++k)
-	{
-		pix[k] = T(0);
-		const int x = xb + k;
-		if (row_valid && x < a.width)
-		{
-			if (a.clear_background) // ColorVec::from_color_f32x3(&[32.0, 16.0, 8.0]).into(), partial_renderer.rs:255
-				pix[k] = P::FORMAT == SW_PIXEL_C64 ? T(8ull | (16ull << 16) | (32ull << 32)) : T(0x00201008u);
-			else
-				pix[k] = fb[uint64_t(y) * a.width + x];
-		}
-	}
+	for (int k = 0; k < STRIP; ++k) pix[k] = a.clear_background && k < in_row ? background : T(0);
+	if (!a.clear_background) load_strip(pix, fb, in_row, fb_vec);
 	unsigned int local_errors = 0, local_writes = 0;
 
-	const int lane = tid & 31, warp = tid >> 5;
 	// the draws to scan: the tile's bin's list (draw order), or every draw
 	const uint32_t* list = nullptr;
-	uint32_t list_len = num_draws;
+	uint32_t list_len;
 	if (a.bin_lists)
 	{
 		const uint32_t bin = uint32_t(tx0 / RASTER_BIN_W) + uint32_t(ty0 / RASTER_BIN_H) * a.bins_x;
 		list = a.bin_lists + uint64_t(bin) * a.bin_cap;
 		list_len = a.bin_counts[bin];
 	}
-	for (uint32_t chunk = 0; chunk < list_len; chunk += 256)
-	{
-		// Ordered compaction of the chunk's draws whose box meets the tile; the hitting thread stages
-		// the draw's record and box.
-		const uint32_t k = chunk + tid;
-		bool hit = false;
-		RasterBox b{0, 0, 0, 0};
-		RasterDraw rd{};
+	else
+		list_len = a.counts ? a.counts->num_draws : a.num_draws;
+	if (wy0 >= wy1) list_len = 0;
+	// lane i's draw of the 32 scanned next, fetched while the 32 before are drawn
+	uint32_t next_di = 0;
+	RasterBox next_box{0, 0, 0, 0, 0u, 0u};
+	auto fetch = [&](uint32_t k) {
+		next_box = RasterBox{0, 0, 0, 0, 0u, 0u};
 		if (k < list_len)
 		{
-			const uint32_t di = list ? list[k] : k;
-			b = a.boxes[di];
-			hit = b.x0 < tx1 && b.x1 > tx0 && b.y0 < ty1 && b.y1 > ty0 && b.x0 < b.x1 && b.y0 < b.y1;
-			if (hit) rd = a.rdraws[di];
+			next_di = list ? list[k] : k;
+			next_box = a.boxes[next_di];
 		}
+	};
+	fetch(uint32_t(lane));
+	for (uint32_t chunk = 0; chunk < list_len; chunk += 32)
+	{
+		const uint32_t di = next_di;
+		const RasterBox b = next_box;
+		if (chunk + 32 < list_len) fetch(chunk + 32 + uint32_t(lane));
+		// (an empty box is 0, 0, 0, 0)
+		const bool hit = b.x0 < tx1 && b.x1 > tx0 && b.y0 < wy1 && b.y1 > wy0;
 		const unsigned mask = __ballot_sync(0xFFFFFFFFu, hit);
-		if (lane == 0) s_warp_counts[warp] = __popc(mask);
-		__syncthreads();
-		uint32_t base = 0, total = 0;
-#pragma unroll
-		for (int w = 0; w < 8; ++w)
-		{
-			const uint32_t c = s_warp_counts[w];
-			if (w < warp) base += c;
-			total += c;
-		}
+		if (!mask) continue;
 		if (hit)
+			sw.hit[__popc(mask & ((1u << lane) - 1u))] = make_uint4(di, b.row_off, uint32_t(int32_t(b.y0)), uint32_t(int32_t(b.y1)));
+		__syncwarp();
+		const int total = __popc(mask);
+		for (int b0 = 0; b0 < total; b0 += BATCH)
 		{
-			const uint32_t pos = base + __popc(mask & ((1u << lane) - 1u));
-			s_rd[pos] = rd;
-			s_box[pos] = b;
-		}
-		__syncthreads();
-
-		for (uint32_t b0 = 0; b0 < total; b0 += BATCH)
-		{
-			const uint32_t n = min(uint32_t(BATCH), total - b0);
-			// Stage the batch's rows of this tile (independent loads, one per thread).
-			for (uint32_t k = tid; k < n * TILE_H; k += 256)
+			const int n = min(BATCH, total - b0);
 			{
-				const uint32_t h = k / TILE_H, r = k % TILE_H;
-				const RasterBox bx = s_box[b0 + h];
-				const int32_t ry = ty0 + int32_t(r);
-				RasterRow row;
-				if (ry >= bx.y0 && ry < bx.y1)
+				const int h = lane / RPW, r = lane % RPW;
+				if (h < n)
 				{
-					const RasterDraw& d = s_rd[b0 + h];
-					row = a.rows[d.row_base + uint32_t(ry - d.y0)];
-				}
-				else
+					const uint4 e = sw.hit[b0 + h];
+					const int ry = wy0 + r;
+					RasterRow row;
 					row.xs = row.xe = 0;
-				s_row[h][r] = row;
+					if (ry >= int(e.z) && ry < int(e.w)) row = a.rows[e.y + uint32_t(ry)];
+					sw.row[h][r] = row;
+				}
+				if (lane < n) sw.rd[lane] = a.rdraws[sw.hit[b0 + lane].x];
 			}
-			__syncthreads();
+			__syncwarp();
 			if (row_valid)
-				for (uint32_t h = 0; h < n; ++h)
+				for (int h = 0; h < n; ++h)
 				{
-					const RasterRow row = s_row[h][ly];
+					const RasterRow row = sw.row[h][lane / TPR];
 					if (xb + STRIP <= row.xs || xb >= row.xe) continue;
-					const RasterDraw& d = s_rd[b0 + h];
+					const RasterDraw& d = sw.rd[h];
 					if (d.mode == SW_RASTER_TRIANGLE)
 					{
 						triangle_strip<P, STRIP>(a, d, row, xb, pix, local_errors, local_writes);
@@ -1060,15 +1090,10 @@ __global__ void __launch_bounds__(256) raster_tiles_kernel(RasterArgs a)
 							++local_writes;
 						}
 				}
-			__syncthreads();
+			__syncwarp(); // the staged records are overwritten by the next batch or chunk
 		}
 	}
-	if (row_valid)
-	{
-#pragma unroll
-		for (int k = 0; k < STRIP; ++k)
-			if (xb + k < a.width) fb[uint64_t(y) * a.width + xb + k] = pix[k];
-	}
+	store_strip(pix, fb, in_row, fb_vec);
 	if constexpr (P::FORMAT == SW_PIXEL_C64)
 	{
 		if constexpr (TILE_W / STRIP <= 16)
@@ -1076,10 +1101,10 @@ __global__ void __launch_bounds__(256) raster_tiles_kernel(RasterArgs a)
 			if (a.bloom_scale == 2)
 				bloom_epilogue_s2<TILE_W, STRIP>(a, reinterpret_cast<const uint64_t*>(pix), tx0, ty0, tid);
 			else if (a.bloom_scale)
-				bloom_epilogue<TILE_W, TILE_H, STRIP>(a, pix, tx0, ty0, tid, &s_row[0][0]);
+				bloom_epilogue<TILE_W, TILE_H, STRIP>(a, pix, tx0, ty0, tid, s_mem);
 		}
 		else if (a.bloom_scale)
-			bloom_epilogue<TILE_W, TILE_H, STRIP>(a, pix, tx0, ty0, tid, &s_row[0][0]);
+			bloom_epilogue<TILE_W, TILE_H, STRIP>(a, pix, tx0, ty0, tid, s_mem);
 	}
 	if (local_errors) atomicAdd(a.error_counter, local_errors);
 	// Pixel writes (span pixels processed) for the traffic accounting, one atomic per warp.

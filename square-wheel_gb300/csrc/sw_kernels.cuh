@@ -225,16 +225,17 @@ struct RasterDraw
 {
 	uint64_t tex_offset;
 	uint32_t tex_w, tex_h;
-	uint32_t row_base;
-	int32_t y0;
 	uint32_t mode;
 	uint16_t blend, tex_source; // SwBlend, SwTexSource
+	uint64_t reserved;
 };
 
-// Pixel bounds of a draw: [x0, x1) x [y0, y1); empty when x0 >= x1 or y0 >= y1.
-struct RasterBox
+// Pixel bounds of a draw, [x0, x1) x [y0, y1), all 0 when empty; row y's record is rows[row_off + y] (u32 arithmetic).
+struct __align__(16) RasterBox
 {
 	int16_t x0, y0, x1, y1;
+	uint32_t row_off;
+	uint32_t reserved;
 };
 
 struct RasterArgs
