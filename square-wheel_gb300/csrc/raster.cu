@@ -1094,6 +1094,8 @@ __global__ void __launch_bounds__(256, 6) raster_tiles_kernel(RasterArgs a)
 		}
 	}
 	store_strip(pix, fb, in_row, fb_vec);
+	if (a.out)
+		store_strip(pix, static_cast<T*>(a.out) + int64_t(y) * a.out_pitch + xb, in_row, rows_aligned(static_cast<const T*>(a.out), a.out_pitch));
 	if constexpr (P::FORMAT == SW_PIXEL_C64)
 	{
 		if constexpr (TILE_W / STRIP <= 16)

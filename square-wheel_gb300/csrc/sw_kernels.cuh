@@ -260,6 +260,8 @@ struct RasterArgs
 	uint64_t arena_texels;
 	const void* skybox; // skybox texels of the frame's pixel format (SW_TEXSRC_SKYBOX draws)
 	void* framebuffer;  // width * height pixels, tightly packed
+	void* out;          // the frame once more in the caller's device memory, out_pitch pixels per row (NULL: not)
+	uint32_t out_pitch;
 	unsigned int* error_counter;
 	// Bloom downscale fused into the tile pass (colour64 frames of a whole-frame graph): with
 	// bloom_scale S != 0 each tile box-averages its final pixels into the bloom buffer (bloom_w x

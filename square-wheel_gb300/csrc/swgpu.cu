@@ -266,6 +266,15 @@ RasterArgs raster_args(SwCtx* ctx)
 
 
 
+// A frame that ends with rasterisation and goes to device memory: the tile pass writes it there beside the frame
+// buffer (which the next frame and sw_postprocess read), instead of a copy that reads the frame buffer again.
+void frame_to_device(RasterArgs& a, void* dst, uint32_t pitch, int dst_is_device)
+{
+	if (!dst || !dst_is_device) return;
+	a.out = dst;
+	a.out_pitch = pitch;
+}
+
 void stage_begin(SwCtx* ctx, int s)
 {
 	if (ctx->timing && !ctx->capturing) cudaEventRecord(ctx->t_begin[s], ctx->stream);
@@ -1177,7 +1186,8 @@ int sw_render(SwCtx* ctx, void* dst, uint32_t pitch, int dst_is_device)
 		ctx->fb_format = fmt;
 		ctx->fb_valid = true;
 	}
-	const RasterArgs a = raster_args(ctx);
+	RasterArgs a = raster_args(ctx);
+	frame_to_device(a, dst, pitch, dst_is_device);
 	SW_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->ev_setup, 0));
 	stage_begin(ctx, STAGE_RASTER);
 	r = check_kernel(ctx, launch_raster_tiles(a, fmt, ctx->tuning.raster_tile, ctx->stream), "raster");
@@ -1186,7 +1196,7 @@ int sw_render(SwCtx* ctx, void* dst, uint32_t pitch, int dst_is_device)
 	SW_CUDA(ctx, cudaEventRecord(ctx->ev_tiles, ctx->stream));
 	ctx->tiles_recorded = true;
 	ctx->frame_open = false;
-	if (dst) return copy_out(ctx, dst, pitch, dst_is_device, ctx->framebuffer.ptr, w, w, h, bpp);
+	if (dst && !dst_is_device) return copy_out(ctx, dst, pitch, 0, ctx->framebuffer.ptr, w, w, h, bpp);
 	return SW_OK;
 }
 
@@ -1831,6 +1841,8 @@ int enqueue_frame(SwCtx* ctx, const SwFrameInput& f, const unsigned char* h, con
 		pp = *post;
 		if ((r = fuse_bloom_downscale(ctx, ra, pp, s))) return r;
 	}
+	else
+		frame_to_device(ra, f.dst, f.dst_pitch, f.dst_is_device);
 	stage_begin(ctx, STAGE_RASTER);
 	r = check_kernel(ctx, launch_raster_tiles(ra, f.params.pixel_format, ctx->tuning.raster_tile, s), "raster");
 	stage_end(ctx, STAGE_RASTER);
@@ -1843,11 +1855,6 @@ int enqueue_frame(SwCtx* ctx, const SwFrameInput& f, const unsigned char* h, con
 			"postprocess");
 		stage_end(ctx, STAGE_POST);
 		if (r) return r;
-	}
-	else if (f.dst && f.dst_is_device)
-	{
-		SW_CUDA(ctx, cudaMemcpy2DAsync(f.dst, size_t(f.dst_pitch) * bpp, ctx->framebuffer.ptr, size_t(f.params.width) * bpp,
-						 size_t(f.params.width) * bpp, f.params.height, cudaMemcpyDeviceToDevice, s));
 	}
 	return SW_OK;
 }
@@ -2581,7 +2588,12 @@ int sw_draw_frame_view(SwCtx* ctx, const SwViewFrameInput* in)
 			SW_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_setup, 0));
 			RasterArgs ra2 = key.raster;
 			PostArgs pp2 = key.post;
-			if (f.postprocess && (rr = fuse_bloom_downscale(ctx, ra2, pp2, s))) return rr;
+			if (f.postprocess)
+			{
+				if ((rr = fuse_bloom_downscale(ctx, ra2, pp2, s))) return rr;
+			}
+			else
+				frame_to_device(ra2, f.dst, f.dst_pitch, f.dst_is_device);
 			if ((rr = check_kernel(ctx, launch_raster_tiles(ra2, p.pixel_format, ctx->tuning.raster_tile, s), "raster")))
 				return rr;
 			if (f.postprocess)
@@ -2591,9 +2603,6 @@ int sw_draw_frame_view(SwCtx* ctx, const SwViewFrameInput* in)
 						 "postprocess")))
 					return rr;
 			}
-			else if (f.dst && f.dst_is_device)
-				SW_CUDA(ctx, cudaMemcpy2DAsync(f.dst, size_t(f.dst_pitch) * bpp, ctx->framebuffer.ptr, size_t(p.width) * bpp,
-								 size_t(p.width) * bpp, p.height, cudaMemcpyDeviceToDevice, s));
 			SW_CUDA(ctx, cudaMemcpyAsync(ctx->h_counts + slot, counts, sizeof(SwViewCounts), cudaMemcpyDeviceToHost, s));
 			return SW_OK;
 		};
