@@ -238,6 +238,9 @@ struct __align__(16) RasterBox
 	uint32_t reserved;
 };
 
+#define SW_WRITE_COUNTERS 512u
+#define SW_WRITE_COUNTER_STRIDE 4u
+
 struct RasterArgs
 {
 	const SwDrawCmd* draws;
@@ -263,6 +266,7 @@ struct RasterArgs
 	void* out;          // the frame once more in the caller's device memory, out_pitch pixels per row (NULL: not)
 	uint32_t out_pitch;
 	unsigned int* error_counter;
+	unsigned long long* write_counters; // SW_WRITE_COUNTERS of them, one per 32 bytes; their sum counts the pixel writes
 	// Bloom downscale fused into the tile pass (colour64 frames of a whole-frame graph): with
 	// bloom_scale S != 0 each tile box-averages its final pixels into the bloom buffer (bloom_w x
 	// bloom_h cells, downscale_hdr_buffer, postprocessor.rs:792-844) and adds its part of every bloom

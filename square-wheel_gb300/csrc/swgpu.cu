@@ -66,6 +66,9 @@ struct ViewGraphKey
 
 } // namespace
 
+// The tile pass's counters on the device, in 8-byte words: the bad fetches (u32), then the pixel writes'.
+constexpr uint32_t COUNTER_WORDS = (SW_WRITE_COUNTERS + 1) * SW_WRITE_COUNTER_STRIDE;
+
 struct SwCtx
 {
 	int device = 0;
@@ -256,6 +259,7 @@ RasterArgs raster_args(SwCtx* ctx)
 	a.skybox = ctx->frame.pixel_format == SW_PIXEL_C64 ? ctx->skybox64.ptr : ctx->skybox32.ptr;
 	a.framebuffer = ctx->framebuffer.ptr;
 	a.error_counter = static_cast<unsigned int*>(ctx->error_counter.ptr);
+	a.write_counters = static_cast<unsigned long long*>(ctx->error_counter.ptr) + SW_WRITE_COUNTER_STRIDE;
 	a.bin_lists = static_cast<uint32_t*>(ctx->bin_lists.ptr);
 	a.bin_counts = static_cast<uint32_t*>(ctx->bin_counts.ptr);
 	a.bin_cap = ctx->bin_cap;
@@ -637,8 +641,8 @@ int sw_create(const SwCreateInfo* info, SwCtx** out_ctx)
 	ctx->num_emissive_pixels = info->num_emissive_pixels;
 	ctx->num_lightmap_elements = info->num_lightmap_elements;
 	ctx->num_dir_lightmap_elements = info->num_directional_lightmap_elements;
-	if ((r = ensure(ctx, ctx->error_counter, 16))) return bail(r);
-	if (cudaMemset(ctx->error_counter.ptr, 0, 16) != cudaSuccess) return bail(SW_ERR_CUDA);
+	if ((r = ensure(ctx, ctx->error_counter, COUNTER_WORDS * 8))) return bail(r);
+	if (cudaMemset(ctx->error_counter.ptr, 0, COUNTER_WORDS * 8) != cudaSuccess) return bail(SW_ERR_CUDA);
 	if (info->max_surface_texels && (r = ensure(ctx, ctx->arena, info->max_surface_texels * 8))) return bail(r);
 	*out_ctx = ctx;
 	return SW_OK;
@@ -2995,12 +2999,13 @@ int sw_abi_layout(uint32_t* sizes, uint32_t count)
 int sw_get_stats(SwCtx* ctx, SwStats* out)
 {
 	if (!ctx || !out) return SW_ERR_INVALID_ARGUMENT;
-	unsigned int errs[4] = {0, 0, 0, 0};
-	SW_CUDA(ctx, cudaMemcpyAsync(errs, ctx->error_counter.ptr, 16, cudaMemcpyDeviceToHost, ctx->stream));
+	uint64_t counters[COUNTER_WORDS] = {};
+	SW_CUDA(ctx, cudaMemcpyAsync(counters, ctx->error_counter.ptr, sizeof(counters), cudaMemcpyDeviceToHost, ctx->stream));
 	SW_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
 	*out = ctx->stats;
-	out->bad_texel_fetches = errs[0];
-	out->pixel_writes = uint64_t(errs[2]) | (uint64_t(errs[3]) << 32);
+	out->bad_texel_fetches = uint32_t(counters[0]);
+	out->pixel_writes = 0;
+	for (uint32_t i = 0; i < SW_WRITE_COUNTERS; ++i) out->pixel_writes += counters[(i + 1) * SW_WRITE_COUNTER_STRIDE];
 	return SW_OK;
 }
 
