@@ -630,6 +630,10 @@ __global__ void __launch_bounds__(256) raster_setup_kernel(RasterArgs a)
 			rd.tex_offset = d.tex_offset;
 			rd.tex_w = d.tex_size[0];
 			rd.tex_h = d.tex_size[1];
+			// addresses are u32 (as usize), affine ones i32 (negative as usize: outside any texture)
+			const uint64_t area = uint64_t(d.tex_size[0]) * d.tex_size[1];
+			const uint64_t reach = d.mode == SW_RASTER_AFFINE ? uint64_t(1) << 31 : uint64_t(1) << 32;
+			rd.max_texel = uint32_t((area < reach ? area : reach) - 1);
 			rd.reserved = 0;
 			rd.mode = d.mode;
 			rd.blend = uint16_t(d.blend);
@@ -676,87 +680,174 @@ __device__ __forceinline__ void blend_into(typename P::T& dst, typename P::T tex
 	}
 }
 
-// Texel address of span pixel i (rasterizer.rs:424-445, 558-572, 705-719): u32 arithmetic for the
-// perspective modes, i32 for affine, then as usize.
-__device__ __forceinline__ uint64_t pixel_address(const RasterRow& r, uint32_t mode, int32_t i, uint32_t tex_w)
+// (1 << Z_CALC_SHIFT) / zdiv, 0 < zdiv <= 2^24. From 512 on the quotient is at most 2^22: the float estimate's error (one
+// unit in the last place of the reciprocal) and its rounding to an integer keep it within one of the quotient, and
+// the remainder corrects it. That is one operation of the quarter-rate unit instead of the general division's three.
+__device__ __forceinline__ uint32_t z_of(uint32_t zdiv)
 {
-	const int32_t t0 = wadd(r.a1, wmul(i, r.b1));
-	const int32_t t1 = wadd(r.a2, wmul(i, r.b2));
-	if (mode == SW_RASTER_FULL_PERSPECTIVE)
-	{
-		const int32_t inv_z = wadd(r.a0, wmul(i, r.b0));
-		const uint32_t zdiv = uint32_t(inv_z) >> INV_Z_PRE_SHIFT;
-		const uint32_t z = (1u << Z_CALC_SHIFT) / (zdiv ? zdiv : 1u);
-		const uint32_t pu = uint32_t((uint64_t(z) * uint64_t(int64_t(t0))) >> TC_FINAL_SHIFT);
-		const uint32_t pv = uint32_t((uint64_t(z) * uint64_t(int64_t(t1))) >> TC_FINAL_SHIFT);
-		return uint32_t(pu + pv * tex_w);
-	}
-	if (mode == SW_RASTER_LINE_Z_CORRECTED) return uint32_t(t0 >> 16) + uint32_t(t1 >> 16) * tex_w;
-	return uint64_t(int64_t(wadd(t0 >> 16, wmul(t1 >> 16, int32_t(tex_w)))));
+	if (zdiv < 512u) return (1u << Z_CALC_SHIFT) / (zdiv ? zdiv : 1u);
+	float inv;
+	asm("rcp.approx.f32 %0, %1;" : "=f"(inv) : "f"(__uint2float_rn(zdiv)));
+	uint32_t q = __float_as_uint(fadd(fmul(inv, 2147483648.0f), 8388608.0f)) & 0x7FFFFFu;
+	const int32_t r = int32_t((1u << Z_CALC_SHIFT) - q * zdiv); // in (-zdiv, 2 * zdiv)
+	if (r < 0)
+		--q;
+	else if (uint32_t(r) >= zdiv)
+		++q;
+	return q;
 }
 
-// A thread's strip of one triangle row (fill_triangle_part's pixel loop, rasterizer.rs:1213-1279):
-// texture coordinates and light of span pixel i are start + i * step (the reference's per-pixel
-// additions), the Color32 texel is lit per lane ((texel * light) >> 16, the alpha lane by 0) and
-// written with the draw's blend; alpha test and alpha blend use the unlit texel's alpha.
-template <class P, int STRIP>
-__device__ __forceinline__ void triangle_strip(const RasterArgs& a, const RasterDraw& d, const RasterRow& row, int xb,
-	typename P::T* pix, unsigned int& errors, unsigned int& writes)
+// The pixels of a warp: TILE_W x RPW of its tile, pixel k of a lane in row k / PPR at column lane + 32 (k % PPR), so the
+// lanes' pixels are neighbours in every load and store.
+template <int TILE_W, int STRIP>
+struct WarpPixels
 {
-	const TriSteps ts = a.tri_steps[uint32_t(row.b2)];
-	uint32_t tex[STRIP];
-	bool ok[STRIP];
-#pragma unroll
-	for (int k = 0; k < STRIP; ++k)
-	{
-		const int x = xb + k;
-		ok[k] = x >= row.xs && x < row.xe;
-		tex[k] = 0;
-		if (ok[k])
+	static constexpr int PPR = TILE_W / 32;   // a lane's pixels per row
+	static constexpr int RPW = STRIP / PPR;   // rows
+	static_assert(TILE_W % 32 == 0 && STRIP % PPR == 0, "whole rows per warp");
+};
+
+// A polygon draw's rows (`rows`, one per warp row) over a warp's pixels: span pixel i = x - xs has the interpolants
+// start + i * step (wrapping, as the reference's repeated additions), its texel address (rasterizer.rs:424-445,
+// 558-572, 705-719) in u32 arithmetic for the perspective modes and in i32 for affine, then as usize. All covered
+// pixels' loads are issued together, then blended.
+template <class P, int TILE_W, int STRIP>
+__device__ __forceinline__ void polygon_pixels(const RasterDraw& d, const RasterRow* rows, const typename P::T* arena,
+	const typename P::T* skybox, int x0, typename P::T (&pix)[STRIP], unsigned int& errors, unsigned int& writes)
+{
+	typedef typename P::T T;
+	constexpr int PPR = WarpPixels<TILE_W, STRIP>::PPR, RPW = WarpPixels<TILE_W, STRIP>::RPW;
+	const T* base = (d.tex_source == SW_TEXSRC_SKYBOX ? skybox : arena) + d.tex_offset;
+	const uint32_t tex_w = d.tex_w, max_texel = d.max_texel;
+	T tex[STRIP];
+	uint32_t covered = 0; // bit k: pixel k is in its row's span
+	auto fetch = [&](int k, uint32_t at) {
+		if (at > max_texel)
 		{
-			const int32_t i = x - row.xs;
-			const int32_t u = wadd(row.a0, wmul(i, ts.d_tc_dx[0])) >> 16;
-			const int32_t v = wadd(row.b0, wmul(i, ts.d_tc_dx[1])) >> 16;
-			uint64_t ua = uint64_t(int64_t(wadd(u, wmul(v, int32_t(d.tex_w)))));
-			if (ua >= uint64_t(d.tex_w) * d.tex_h)
+			++errors;
+			at = 0;
+		}
+		tex[k] = base[at];
+		covered |= 1u << k;
+	};
+	if (d.mode == SW_RASTER_FULL_PERSPECTIVE)
+	{
+#pragma unroll
+		for (int r = 0; r < RPW; ++r)
+		{
+			const RasterRow row = rows[r];
+#pragma unroll
+			for (int j = 0; j < PPR; ++j)
 			{
-				++errors;
-				ua = 0;
+				const int x = x0 + 32 * j, i = x - row.xs;
+				if (i < 0 || x >= row.xe) continue;
+				const uint64_t z = z_of(uint32_t(wadd(row.a0, wmul(i, row.b0))) >> INV_Z_PRE_SHIFT);
+				fetch(r * PPR + j, uint32_t((z * uint64_t(int64_t(wadd(row.a1, wmul(i, row.b1))))) >> TC_FINAL_SHIFT) +
+						uint32_t((z * uint64_t(int64_t(wadd(row.a2, wmul(i, row.b2))))) >> TC_FINAL_SHIFT) * tex_w);
 			}
-			tex[k] = __ldg(a.lite + d.tex_offset + ua);
 		}
 	}
+	else
+	{
 #pragma unroll
-	for (int k = 0; k < STRIP; ++k)
-		if (ok[k])
+		for (int r = 0; r < RPW; ++r)
 		{
-			const int32_t i = xb + k - row.xs;
-			const CI t = ci_from_c32(tex[k]);
-			// line_light lanes [b, g, r, 0] = [light2, light1, light0, 0] (ColorVecI::from_color_i32x3)
-			const CI lit{{wmul(t.v[0], wadd(row.a2, wmul(i, ts.d_light_dx[2]))) >> 16,
-				wmul(t.v[1], wadd(row.b1, wmul(i, ts.d_light_dx[1]))) >> 16,
-				wmul(t.v[2], wadd(row.a1, wmul(i, ts.d_light_dx[0]))) >> 16, 0}};
-			typename P::T& dst = pix[k];
-			switch (d.blend)
-			{
-			case SW_BLEND_NONE: dst = P::from_ci(lit); break;
-			case SW_BLEND_AVERAGE: dst = P::average(dst, P::from_ci(lit)); break;
-			case SW_BLEND_ADDITIVE: dst = P::saturated_sum(dst, P::from_ci(lit)); break;
-			case SW_BLEND_ALPHA_TEST:
-				if ((tex[k] & 0xFF000000u) > 0x7F000000u) dst = P::from_ci(lit);
-				break;
-			default:
-			{
-				const int32_t alpha = int32_t(tex[k] >> 24);
-				const CI dv = P::to_ci(dst);
-				CI r;
+			const RasterRow row = rows[r];
 #pragma unroll
-				for (int l = 0; l < 4; ++l) r.v[l] = wadd(wmul(dv.v[l], wsub(255, alpha)), wmul(lit.v[l], alpha)) >> 8;
-				dst = P::from_ci(r);
+			for (int j = 0; j < PPR; ++j)
+			{
+				const int x = x0 + 32 * j, i = x - row.xs;
+				if (i < 0 || x >= row.xe) continue;
+				fetch(r * PPR + j, uint32_t(wadd(row.a1, wmul(i, row.b1)) >> 16) + uint32_t(wadd(row.a2, wmul(i, row.b2)) >> 16) * tex_w);
 			}
-			}
-			++writes;
 		}
+	}
+	writes += __popc(covered);
+	const uint32_t blend = d.blend;
+	if (blend == SW_BLEND_NONE)
+	{
+#pragma unroll
+		for (int k = 0; k < STRIP; ++k)
+			if ((covered >> k) & 1u) pix[k] = tex[k];
+	}
+	else
+	{
+#pragma unroll
+		for (int k = 0; k < STRIP; ++k)
+			if ((covered >> k) & 1u) blend_into<P>(pix[k], tex[k], blend);
+	}
+}
+
+// A triangle's rows over a warp's pixels (fill_triangle_part's pixel loop, rasterizer.rs:1213-1279): texture coordinates
+// and light of span pixel i are start + i * step (the reference's per-pixel additions), the Color32 texel is lit
+// per lane ((texel * light) >> 16, the alpha lane by 0) and written with the draw's blend; alpha test and alpha
+// blend use the unlit texel's alpha.
+template <class P, int TILE_W, int STRIP>
+__device__ __forceinline__ void triangle_pixels(const RasterArgs& a, const RasterDraw& d, const RasterRow* rows, int x0,
+	typename P::T (&pix)[STRIP], unsigned int& errors, unsigned int& writes)
+{
+	constexpr int PPR = WarpPixels<TILE_W, STRIP>::PPR, RPW = WarpPixels<TILE_W, STRIP>::RPW;
+	const uint32_t* base = a.lite + d.tex_offset;
+	const uint64_t area = uint64_t(d.tex_w) * d.tex_h;
+#pragma unroll
+	for (int r = 0; r < RPW; ++r)
+	{
+		const RasterRow row = rows[r];
+		if (row.xs >= row.xe) continue;
+		const TriSteps ts = a.tri_steps[uint32_t(row.b2)];
+		uint32_t tex[PPR];
+		bool ok[PPR];
+#pragma unroll
+		for (int j = 0; j < PPR; ++j)
+		{
+			const int x = x0 + 32 * j, i = x - row.xs;
+			ok[j] = i >= 0 && x < row.xe;
+			tex[j] = 0;
+			if (ok[j])
+			{
+				const int32_t u = wadd(row.a0, wmul(i, ts.d_tc_dx[0])) >> 16;
+				const int32_t v = wadd(row.b0, wmul(i, ts.d_tc_dx[1])) >> 16;
+				uint64_t ua = uint64_t(int64_t(wadd(u, wmul(v, int32_t(d.tex_w)))));
+				if (ua >= area)
+				{
+					++errors;
+					ua = 0;
+				}
+				tex[j] = __ldg(base + ua);
+			}
+		}
+#pragma unroll
+		for (int j = 0; j < PPR; ++j)
+			if (ok[j])
+			{
+				const int32_t i = x0 + 32 * j - row.xs;
+				const CI t = ci_from_c32(tex[j]);
+				// line_light lanes [b, g, r, 0] = [light2, light1, light0, 0] (ColorVecI::from_color_i32x3)
+				const CI lit{{wmul(t.v[0], wadd(row.a2, wmul(i, ts.d_light_dx[2]))) >> 16,
+					wmul(t.v[1], wadd(row.b1, wmul(i, ts.d_light_dx[1]))) >> 16,
+					wmul(t.v[2], wadd(row.a1, wmul(i, ts.d_light_dx[0]))) >> 16, 0}};
+				typename P::T& dst = pix[r * PPR + j];
+				switch (d.blend)
+				{
+				case SW_BLEND_NONE: dst = P::from_ci(lit); break;
+				case SW_BLEND_AVERAGE: dst = P::average(dst, P::from_ci(lit)); break;
+				case SW_BLEND_ADDITIVE: dst = P::saturated_sum(dst, P::from_ci(lit)); break;
+				case SW_BLEND_ALPHA_TEST:
+					if ((tex[j] & 0xFF000000u) > 0x7F000000u) dst = P::from_ci(lit);
+					break;
+				default:
+				{
+					const int32_t alpha = int32_t(tex[j] >> 24);
+					const CI dv = P::to_ci(dst);
+					CI b;
+#pragma unroll
+					for (int l = 0; l < 4; ++l) b.v[l] = wadd(wmul(dv.v[l], wsub(255, alpha)), wmul(lit.v[l], alpha)) >> 8;
+					dst = P::from_ci(b);
+				}
+				}
+				++writes;
+			}
+	}
 }
 
 // The bloom downscale of a tile's final colour64 pixels (downscale_hdr_buffer, postprocessor.rs:792-844):
@@ -768,15 +859,15 @@ __device__ __forceinline__ void triangle_strip(const RasterArgs& a, const Raster
 template <int TILE_W, int TILE_H, int STRIP>
 __device__ __forceinline__ void bloom_epilogue(const RasterArgs& a, const uint64_t* pix, int tx0, int ty0, int tid, void* staging)
 {
-	constexpr int TPR = TILE_W / STRIP;
+	constexpr int PPR = WarpPixels<TILE_W, STRIP>::PPR, RPW = WarpPixels<TILE_W, STRIP>::RPW;
 	static_assert(TILE_W % 8 == 0 && TILE_H % 8 == 0, "bloom cells must not straddle tiles");
 	__shared__ int32_t s_ls[TILE_H / 2][4];
 	uint64_t* s_pix = static_cast<uint64_t*>(staging);
 	__syncthreads(); // the staging area is free
 	{
-		const int ly = tid / TPR, lx = (tid % TPR) * STRIP;
+		const int row = (tid >> 5) * RPW, column = tid & 31;
 #pragma unroll
-		for (int k = 0; k < STRIP; ++k) s_pix[ly * TILE_W + lx + k] = pix[k];
+		for (int k = 0; k < STRIP; ++k) s_pix[(row + k / PPR) * TILE_W + column + 32 * (k % PPR)] = pix[k];
 	}
 	for (int i = tid; i < (TILE_H / 2) * 4; i += 256) (&s_ls[0][0])[i] = 0;
 	__syncthreads();
@@ -826,9 +917,10 @@ __global__ void __launch_bounds__(256) raster_bin_kernel(RasterArgs a)
 	{
 		const uint32_t di = chunk + threadIdx.x;
 		bool hit = false;
+		RasterBox b{0, 0, 0, 0, 0u, 0u};
 		if (di < num_draws)
 		{
-			const RasterBox b = a.boxes[di];
+			b = a.boxes[di];
 			hit = b.x0 < bx1 && b.x1 > bx0 && b.y0 < by1 && b.y1 > by0 && b.x0 < b.x1 && b.y0 < b.y1;
 		}
 		const unsigned mask = __ballot_sync(0xFFFFFFFFu, hit);
@@ -841,7 +933,11 @@ __global__ void __launch_bounds__(256) raster_bin_kernel(RasterArgs a)
 			if (w < warp) base += s_counts[w];
 			sum += s_counts[w];
 		}
-		if (hit) list[base + __popc(mask & ((1u << lane) - 1u))] = di;
+		if (hit)
+		{
+			const uint32_t pos = base + __popc(mask & ((1u << lane) - 1u));
+			list[pos] = di;
+		}
 		total += sum;
 		__syncthreads(); // s_counts is rewritten by the next chunk
 	}
@@ -849,118 +945,64 @@ __global__ void __launch_bounds__(256) raster_bin_kernel(RasterArgs a)
 	pdl_trigger();
 }
 
-// The scale-2 bloom downscale without shared memory, when a tile row's threads share a warp with the
-// next row's (TILE_W / STRIP <= 16): the thread of an even row takes the odd row's STRIP pixels from
-// its partner by a shuffle, box-averages its STRIP / 2 cells and stores them; the line's lane sums of
-// the row pair are reduced over its threads by shuffles and added to the global sums, one atomic per
-// lane. Same integer arithmetic as bloom_epilogue, so the same values.
+// The scale-2 bloom downscale without shared memory, when a warp has whole row pairs: a lane has both rows of its
+// columns and takes the neighbouring column's sums from its partner by shuffles; the even lanes box-average and
+// store the cells, and the line's lane sums are reduced over the warp and added to the global sums, one atomic per
+// colour lane. Same integer arithmetic as bloom_epilogue, so the same values.
 template <int TILE_W, int STRIP>
-__device__ __forceinline__ void bloom_epilogue_s2(const RasterArgs& a, const uint64_t* pix, int tx0, int ty0, int tid)
+__device__ __forceinline__ void bloom_epilogue_s2(const RasterArgs& a, const uint64_t* pix, int tx0, int wy0, int lane)
 {
-	constexpr int TPR = TILE_W / STRIP;
-	static_assert(TPR <= 16 && (TPR & (TPR - 1)) == 0 && STRIP % 2 == 0, "row pairs within a warp");
-	const int ly = tid / TPR, lx = (tid % TPR) * STRIP;
-	uint64_t other[STRIP];
+	constexpr int PPR = WarpPixels<TILE_W, STRIP>::PPR, RPW = WarpPixels<TILE_W, STRIP>::RPW;
+	static_assert(RPW % 2 == 0, "row pairs within a warp");
 #pragma unroll
-	for (int k = 0; k < STRIP; ++k) other[k] = __shfl_xor_sync(0xFFFFFFFFu, pix[k], TPR);
-	int32_t line[4] = {0, 0, 0, 0};
-	const bool even = (ly & 1) == 0;
-	const uint32_t by = uint32_t((ty0 + ly) / 2);
-	if (even && by < a.bloom_h)
+	for (int r = 0; r < RPW; r += 2)
 	{
+		const uint32_t by = uint32_t((wy0 + r) / 2);
+		if (by >= a.bloom_h) break;
+		int32_t line[4] = {0, 0, 0, 0};
 #pragma unroll
-		for (int c = 0; c < STRIP / 2; ++c)
+		for (int j = 0; j < PPR; ++j)
 		{
-			const uint32_t bx = uint32_t((tx0 + lx) / 2 + c);
-			if (bx >= a.bloom_w) continue;
-			int32_t sum[4] = {0, 0, 0, 0};
-			const uint64_t q[4] = {pix[2 * c], pix[2 * c + 1], other[2 * c], other[2 * c + 1]};
-#pragma unroll
-			for (int j = 0; j < 4; ++j)
-			{
-				const CI v = ci_from_c64(q[j]);
-#pragma unroll
-				for (int l = 0; l < 4; ++l) sum[l] = wadd(sum[l], v.v[l]);
-			}
+			const CI top = ci_from_c64(pix[r * PPR + j]), bottom = ci_from_c64(pix[(r + 1) * PPR + j]);
+			const uint32_t bx = uint32_t((tx0 + lane + 32 * j) / 2);
 			CI avg;
 #pragma unroll
 			for (int l = 0; l < 4; ++l)
 			{
-				avg.v[l] = wmul(sum[l], 64) >> 8; // scaler 256 / (2 * 2)
-				line[l] = wadd(line[l], avg.v[l]);
+				const int32_t sum = wadd(top.v[l], bottom.v[l]);
+				avg.v[l] = wmul(wadd(sum, __shfl_xor_sync(0xFFFFFFFFu, sum, 1)), 64) >> 8; // scaler 256 / (2 * 2)
 			}
-			a.bloom_out[uint64_t(by) * a.bloom_w + bx] = ci_to_c64(avg);
+			if ((lane & 1) == 0 && bx < a.bloom_w)
+			{
+#pragma unroll
+				for (int l = 0; l < 4; ++l) line[l] = wadd(line[l], avg.v[l]);
+				a.bloom_out[uint64_t(by) * a.bloom_w + bx] = ci_to_c64(avg);
+			}
 		}
-	}
-	// the row pair's threads are TPR consecutive lanes (the odd row's add zeros)
 #pragma unroll
-	for (int l = 0; l < 4; ++l)
-		for (int o = TPR / 2; o > 0; o >>= 1) line[l] = wadd(line[l], __shfl_xor_sync(0xFFFFFFFFu, line[l], o));
-	if (even && (tid % TPR) == 0 && by < a.bloom_h)
-	{
-#pragma unroll
-		for (int l = 0; l < 4; ++l) atomicAdd(&a.bloom_line_sums[by * 4 + l], line[l]);
+		for (int l = 0; l < 4; ++l) line[l] = __reduce_add_sync(0xFFFFFFFFu, line[l]);
+		if (lane < 4) atomicAdd(&a.bloom_line_sums[by * 4 + lane], lane == 0 ? line[0] : lane == 1 ? line[1] : lane == 2 ? line[2] : line[3]);
 	}
 }
 
 // Tile shapes of the tile pass (the autotuner's choice, SwTuning.raster_tile): TILE_W x TILE_H pixels,
-// 256 threads, each thread a 1 x STRIP strip of one row. Every shape gives the same frame.
+// 256 threads of STRIP pixels. Every shape gives the same frame.
 struct TileShape
 {
 	int w, h, strip;
 };
 constexpr TileShape TILE_SHAPES[SW_RASTER_TILE_VARIANTS] = {{64, 16, 4}, {32, 32, 4}, {128, 8, 4}, {64, 32, 8}, {32, 16, 2}};
 
-// STRIP pixels of a row from / to memory: 16 bytes at a time where `vec` says that the address allows it and the
-// whole strip lies in the row.
-template <class T, int STRIP>
-__device__ __forceinline__ void load_strip(T (&pix)[STRIP], const T* p, int n, bool vec)
-{
-	constexpr int W = 16 / int(sizeof(T));
-	if constexpr (STRIP % W == 0)
-		if (vec && n >= STRIP)
-		{
-#pragma unroll
-			for (int k = 0; k < STRIP; k += W) *reinterpret_cast<uint4*>(&pix[k]) = *reinterpret_cast<const uint4*>(p + k);
-			return;
-		}
-#pragma unroll
-	for (int k = 0; k < STRIP; ++k)
-		if (k < n) pix[k] = p[k];
-}
-template <class T, int STRIP>
-__device__ __forceinline__ void store_strip(const T (&pix)[STRIP], T* p, int n, bool vec)
-{
-	constexpr int W = 16 / int(sizeof(T));
-	if constexpr (STRIP % W == 0)
-		if (vec && n >= STRIP)
-		{
-#pragma unroll
-			for (int k = 0; k < STRIP; k += W) *reinterpret_cast<uint4*>(p + k) = *reinterpret_cast<const uint4*>(&pix[k]);
-			return;
-		}
-#pragma unroll
-	for (int k = 0; k < STRIP; ++k)
-		if (k < n) p[k] = pix[k];
-}
-template <class T>
-__device__ __forceinline__ bool rows_aligned(const T* p, uint32_t pitch)
-{
-	return ((reinterpret_cast<uintptr_t>(p) | (uintptr_t(pitch) * sizeof(T))) & 15) == 0;
-}
-
-// Bound by latency: list -> box -> row and draw records -> texels are four dependent round trips per tile, so what
+// Bound by latency: boxes -> row and draw records -> texels are three dependent round trips per tile, so what
 // counts is how many warps are in flight and that none waits for another (with the tile's draws compacted and staged
 // by the CTA between barriers, 26 KB of shared memory and four CTAs per SM, a pass over a sheet of 46.9 M colour64
 // pixels took 103 us more of 1,620, and a 1920x1080 frame 4 us more of 49). Six CTAs per SM (40 registers, a few bytes spilled) measured 1% faster than four.
 template <class P, int TILE_W, int TILE_H, int STRIP>
-__global__ void __launch_bounds__(256, 6) raster_tiles_kernel(RasterArgs a)
+__global__ void __launch_bounds__(256, 4) raster_tiles_kernel(RasterArgs a)
 {
 	static_assert((TILE_W / STRIP) * TILE_H == 256, "256 threads per tile");
-	constexpr int TPR = TILE_W / STRIP; // threads per tile row
-	constexpr int RPW = 32 / TPR;       // rows per warp
-	constexpr int BATCH = 32 / RPW;     // hits whose rows the warp stages at a time, one row record per lane
-	static_assert(32 % TPR == 0, "whole rows per warp");
+	constexpr int PPR = WarpPixels<TILE_W, STRIP>::PPR, RPW = WarpPixels<TILE_W, STRIP>::RPW;
+	constexpr int BATCH = 32 / RPW; // hits whose rows the warp stages at a time, one row record per lane
 	typedef typename P::T T;
 	struct WarpShared
 	{
@@ -976,54 +1018,55 @@ __global__ void __launch_bounds__(256, 6) raster_tiles_kernel(RasterArgs a)
 	const int ty0 = int(blockIdx.x / tiles_x) * TILE_H;
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	WarpShared& sw = reinterpret_cast<WarpShared*>(s_mem)[warp];
-	const int ly = tid / TPR;
 	pdl_wait(); // the surface build (launched before this kernel) has completed
-	const int xb = tx0 + (tid % TPR) * STRIP; // first pixel of this thread's strip
-	const int y = ty0 + ly;
-	const bool row_valid = y < a.height;
-	const int in_row = row_valid ? a.width - xb : 0; // the strip's pixels inside the frame (at most STRIP of them)
+	const int x0 = tx0 + lane; // the lane's first column
 	const int tx1 = min(tx0 + TILE_W, a.width);
 	const int wy0 = ty0 + warp * RPW, wy1 = min(wy0 + RPW, a.height); // the warp's rows
 
-	T* fb = static_cast<T*>(a.framebuffer) + int64_t(y) * a.width + xb;
-	const bool fb_vec = rows_aligned(static_cast<const T*>(a.framebuffer), uint32_t(a.width));
+	T* fb = static_cast<T*>(a.framebuffer);
 	const T* arena = static_cast<const T*>(a.arena);
 	const T* skybox = static_cast<const T*>(a.skybox);
 	T pix[STRIP];
 	// ColorVec::from_color_f32x3(&[32.0, 16.0, 8.0]).into(), partial_renderer.rs:255
 	const T background = P::FORMAT == SW_PIXEL_C64 ? T(8ull | (16ull << 16) | (32ull << 32)) : T(0x00201008u);
 #pragma unroll
-	for (int k = 0; k < STRIP; ++k) pix[k] = a.clear_background && k < in_row ? background : T(0);
-	if (!a.clear_background) load_strip(pix, fb, in_row, fb_vec);
+	for (int k = 0; k < STRIP; ++k)
+	{
+		pix[k] = T(0);
+		const int x = x0 + 32 * (k % PPR), y = wy0 + k / PPR;
+		if (x < a.width && y < a.height) pix[k] = a.clear_background ? background : fb[uint64_t(y) * uint32_t(a.width) + x];
+	}
 	unsigned int local_errors = 0, local_writes = 0;
 
-	// the draws to scan: the tile's bin's list (draw order), or every draw
+	// the draws to scan: the tile's bin's list (draw order; its first 32 draws' boxes lie beside it, so a short list
+	// costs one round trip), or every draw; lane i's draw of the 32 scanned next is fetched while the 32 before
+	// are drawn
 	const uint32_t* list = nullptr;
 	uint32_t list_len;
-	if (a.bin_lists)
-	{
-		const uint32_t bin = uint32_t(tx0 / RASTER_BIN_W) + uint32_t(ty0 / RASTER_BIN_H) * a.bins_x;
-		list = a.bin_lists + uint64_t(bin) * a.bin_cap;
-		list_len = a.bin_counts[bin];
-	}
-	else
-		list_len = a.counts ? a.counts->num_draws : a.num_draws;
-	if (wy0 >= wy1) list_len = 0;
-	// lane i's draw of the 32 scanned next, fetched while the 32 before are drawn
-	uint32_t next_di = 0;
 	RasterBox next_box{0, 0, 0, 0, 0u, 0u};
 	auto fetch = [&](uint32_t k) {
 		next_box = RasterBox{0, 0, 0, 0, 0u, 0u};
 		if (k < list_len)
 		{
-			next_di = list ? list[k] : k;
-			next_box = a.boxes[next_di];
+			const uint32_t di = list ? list[k] : k;
+			next_box = a.boxes[di];
+			next_box.draw = di;
 		}
 	};
-	fetch(uint32_t(lane));
+	if (a.bin_lists)
+	{
+		const uint32_t bin = uint32_t(tx0 / RASTER_BIN_W) + uint32_t(ty0 / RASTER_BIN_H) * a.bins_x;
+		list = a.bin_lists + uint64_t(bin) * a.bin_cap;
+		list_len = wy0 < wy1 ? a.bin_counts[bin] : 0u;
+		fetch(uint32_t(lane));
+	}
+	else
+	{
+		list_len = wy0 < wy1 ? (a.counts ? a.counts->num_draws : a.num_draws) : 0u;
+		fetch(uint32_t(lane));
+	}
 	for (uint32_t chunk = 0; chunk < list_len; chunk += 32)
 	{
-		const uint32_t di = next_di;
 		const RasterBox b = next_box;
 		if (chunk + 32 < list_len) fetch(chunk + 32 + uint32_t(lane));
 		// (an empty box is 0, 0, 0, 0)
@@ -1031,7 +1074,7 @@ __global__ void __launch_bounds__(256, 6) raster_tiles_kernel(RasterArgs a)
 		const unsigned mask = __ballot_sync(0xFFFFFFFFu, hit);
 		if (!mask) continue;
 		if (hit)
-			sw.hit[__popc(mask & ((1u << lane) - 1u))] = make_uint4(di, b.row_off, uint32_t(int32_t(b.y0)), uint32_t(int32_t(b.y1)));
+			sw.hit[__popc(mask & ((1u << lane) - 1u))] = make_uint4(b.draw, b.row_off, uint32_t(int32_t(b.y0)), uint32_t(int32_t(b.y1)));
 		__syncwarp();
 		const int total = __popc(mask);
 		for (int b0 = 0; b0 < total; b0 += BATCH)
@@ -1051,57 +1094,33 @@ __global__ void __launch_bounds__(256, 6) raster_tiles_kernel(RasterArgs a)
 				if (lane < n) sw.rd[lane] = a.rdraws[sw.hit[b0 + lane].x];
 			}
 			__syncwarp();
-			if (row_valid)
-				for (int h = 0; h < n; ++h)
-				{
-					const RasterRow row = sw.row[h][lane / TPR];
-					if (xb + STRIP <= row.xs || xb >= row.xe) continue;
-					const RasterDraw& d = sw.rd[h];
-					if (d.mode == SW_RASTER_TRIANGLE)
-					{
-						triangle_strip<P, STRIP>(a, d, row, xb, pix, local_errors, local_writes);
-						continue;
-					}
-					// Up to four independent texel loads, then the blends in pixel order.
-					T tex[STRIP];
-					bool ok[STRIP];
-#pragma unroll
-					for (int k = 0; k < STRIP; ++k)
-					{
-						const int x = xb + k;
-						ok[k] = x >= row.xs && x < row.xe;
-						tex[k] = T(0);
-						if (ok[k])
-						{
-							uint64_t ua = pixel_address(row, d.mode, x - row.xs, d.tex_w);
-							if (ua >= uint64_t(d.tex_w) * d.tex_h)
-							{
-								++local_errors;
-								ua = 0;
-							}
-							tex[k] = (d.tex_source == SW_TEXSRC_SKYBOX ? skybox : arena)[d.tex_offset + ua];
-						}
-					}
-#pragma unroll
-					for (int k = 0; k < STRIP; ++k)
-						if (ok[k])
-						{
-							blend_into<P>(pix[k], tex[k], d.blend);
-							++local_writes;
-						}
-				}
+			for (int h = 0; h < n; ++h)
+			{
+				const RasterDraw& d = sw.rd[h];
+				if (d.mode == SW_RASTER_TRIANGLE)
+					triangle_pixels<P, TILE_W, STRIP>(a, d, sw.row[h], x0, pix, local_errors, local_writes);
+				else
+					polygon_pixels<P, TILE_W, STRIP>(d, sw.row[h], arena, skybox, x0, pix, local_errors, local_writes);
+			}
 			__syncwarp(); // the staged records are overwritten by the next batch or chunk
 		}
 	}
-	store_strip(pix, fb, in_row, fb_vec);
-	if (a.out)
-		store_strip(pix, static_cast<T*>(a.out) + int64_t(y) * a.out_pitch + xb, in_row, rows_aligned(static_cast<const T*>(a.out), a.out_pitch));
+#pragma unroll
+	for (int k = 0; k < STRIP; ++k)
+	{
+		const int x = x0 + 32 * (k % PPR), y = wy0 + k / PPR;
+		if (x < a.width && y < a.height)
+		{
+			fb[uint64_t(y) * uint32_t(a.width) + x] = pix[k];
+			if (a.out) static_cast<T*>(a.out)[uint64_t(y) * a.out_pitch + x] = pix[k];
+		}
+	}
 	if constexpr (P::FORMAT == SW_PIXEL_C64)
 	{
-		if constexpr (TILE_W / STRIP <= 16)
+		if constexpr (RPW % 2 == 0)
 		{
 			if (a.bloom_scale == 2)
-				bloom_epilogue_s2<TILE_W, STRIP>(a, reinterpret_cast<const uint64_t*>(pix), tx0, ty0, tid);
+				bloom_epilogue_s2<TILE_W, STRIP>(a, reinterpret_cast<const uint64_t*>(pix), tx0, wy0, lane);
 			else if (a.bloom_scale)
 				bloom_epilogue<TILE_W, TILE_H, STRIP>(a, pix, tx0, ty0, tid, s_mem);
 		}

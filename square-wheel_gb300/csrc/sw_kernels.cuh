@@ -227,7 +227,8 @@ struct RasterDraw
 	uint32_t tex_w, tex_h;
 	uint32_t mode;
 	uint16_t blend, tex_source; // SwBlend, SwTexSource
-	uint64_t reserved;
+	uint32_t max_texel;         // the largest texel address inside the texture
+	uint32_t reserved;
 };
 
 // Pixel bounds of a draw, [x0, x1) x [y0, y1), all 0 when empty; row y's record is rows[row_off + y] (u32 arithmetic).
@@ -235,7 +236,7 @@ struct __align__(16) RasterBox
 {
 	int16_t x0, y0, x1, y1;
 	uint32_t row_off;
-	uint32_t reserved;
+	uint32_t draw; // its index, in a bin's list of boxes
 };
 
 #define SW_WRITE_COUNTERS 512u
