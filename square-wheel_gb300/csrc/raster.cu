@@ -937,6 +937,11 @@ __global__ void __launch_bounds__(256) raster_bin_kernel(RasterArgs a)
 		{
 			const uint32_t pos = base + __popc(mask & ((1u << lane) - 1u));
 			list[pos] = di;
+			if (pos < 32)
+			{
+				b.draw = di;
+				a.bin_first[blockIdx.x * 32 + pos] = b;
+			}
 		}
 		total += sum;
 		__syncthreads(); // s_counts is rewritten by the next chunk
@@ -1056,9 +1061,10 @@ __global__ void __launch_bounds__(256, 4) raster_tiles_kernel(RasterArgs a)
 	if (a.bin_lists)
 	{
 		const uint32_t bin = uint32_t(tx0 / RASTER_BIN_W) + uint32_t(ty0 / RASTER_BIN_H) * a.bins_x;
+		const RasterBox first = a.bin_first[bin * 32 + uint32_t(lane)];
 		list = a.bin_lists + uint64_t(bin) * a.bin_cap;
 		list_len = wy0 < wy1 ? a.bin_counts[bin] : 0u;
-		fetch(uint32_t(lane));
+		if (uint32_t(lane) < list_len) next_box = first;
 	}
 	else
 	{

@@ -280,6 +280,7 @@ struct RasterArgs
 	// tile scans its bin's list instead of every draw. NULL lists: every tile scans every draw.
 	uint32_t* bin_lists;
 	uint32_t* bin_counts;
+	RasterBox* bin_first; // the boxes of the first 32 draws of every bin's list
 	uint32_t bin_cap, bins_x, bins_y;
 };
 

@@ -85,10 +85,10 @@ struct SwCtx
 	DevBuf texels, texture_mips, emissive, emissive_mips, lightmaps, dir_lightmaps;
 	DevBuf lm_compressed; // sw_set_lightmaps_compressed: the compressed lumps as uploaded
 	// the tile pass's bins (raster_bin_kernel): bins_x * bins_y lists of bin_cap draw indices and counts
-	DevBuf bin_lists, bin_counts;
+	DevBuf bin_lists, bin_counts, bin_first;
 	uint32_t bin_cap = 0, bins_x = 0, bins_y = 0;
 	// the bins of a whole frame's nested views (portal textures), reused view after view
-	DevBuf vbin_lists, vbin_counts;
+	DevBuf vbin_lists, vbin_counts, vbin_first;
 	uint32_t vbin_cap = 0;
 	uint64_t vbin_cells = 0;
 	DevBuf skybox32, skybox64; // sw_set_skybox: the same texels in Color32 and Color64
@@ -262,6 +262,7 @@ RasterArgs raster_args(SwCtx* ctx)
 	a.write_counters = static_cast<unsigned long long*>(ctx->error_counter.ptr) + SW_WRITE_COUNTER_STRIDE;
 	a.bin_lists = static_cast<uint32_t*>(ctx->bin_lists.ptr);
 	a.bin_counts = static_cast<uint32_t*>(ctx->bin_counts.ptr);
+	a.bin_first = static_cast<RasterBox*>(ctx->bin_first.ptr);
 	a.bin_cap = ctx->bin_cap;
 	a.bins_x = ctx->bins_x;
 	a.bins_y = ctx->bins_y;
@@ -353,6 +354,7 @@ int ensure_bins(SwCtx* ctx, uint32_t width, uint32_t height, uint64_t draws)
 	int r;
 	if ((r = ensure(ctx, ctx->bin_lists, size_t(bx) * by * cap * 4))) return r;
 	if ((r = ensure(ctx, ctx->bin_counts, size_t(bx) * by * 4))) return r;
+	if ((r = ensure(ctx, ctx->bin_first, size_t(bx) * by * 32 * sizeof(RasterBox)))) return r;
 	ctx->bin_cap = cap;
 	ctx->bins_x = bx;
 	ctx->bins_y = by;
@@ -376,6 +378,7 @@ int ensure_view_bins(SwCtx* ctx, const SwView* views, uint32_t num_views)
 	int r;
 	if ((r = ensure(ctx, ctx->vbin_lists, size_t(cells) * cap * 4))) return r;
 	if ((r = ensure(ctx, ctx->vbin_counts, size_t(cells) * 4))) return r;
+	if ((r = ensure(ctx, ctx->vbin_first, size_t(cells) * 32 * sizeof(RasterBox)))) return r;
 	ctx->vbin_cap = cap;
 	ctx->vbin_cells = cells;
 	return SW_OK;
@@ -654,13 +657,13 @@ int sw_destroy(SwCtx* ctx)
 	cudaSetDevice(ctx->device);
 	if (ctx->stream) cudaStreamSynchronize(ctx->stream);
 	if (ctx->aux) cudaStreamSynchronize(ctx->aux);
-	DevBuf* bufs[] = {&ctx->texels, &ctx->texture_mips, &ctx->emissive, &ctx->emissive_mips, &ctx->lightmaps, &ctx->lm_compressed, &ctx->bin_lists, &ctx->bin_counts, &ctx->skybox32,
+	DevBuf* bufs[] = {&ctx->texels, &ctx->texture_mips, &ctx->emissive, &ctx->emissive_mips, &ctx->lightmaps, &ctx->lm_compressed, &ctx->bin_lists, &ctx->bin_counts, &ctx->bin_first, &ctx->skybox32,
 		&ctx->skybox64, &ctx->frame_in,
 		&ctx->dir_lightmaps, &ctx->lights, &ctx->surfaces, &ctx->work_prefix, &ctx->arena, &ctx->draws, &ctx->vertices,
 		&ctx->draw_rows, &ctx->rdraws, &ctx->rows, &ctx->boxes, &ctx->tri_steps, &ctx->tri_vertices, &ctx->lite, &ctx->ldr[0], &ctx->ldr[1], &ctx->framebuffer, &ctx->bloom0, &ctx->bloom1, &ctx->line_sums,
 		&ctx->line_sums_f, &ctx->error_counter, &ctx->up_src, &ctx->up_dst, &ctx->map_polygons,
 		&ctx->map_vertices, &ctx->vslab, &ctx->shadow_storage, &ctx->shadow_descs, &ctx->shadow_chunks, &ctx->effect_buf, &ctx->sim_state, &ctx->sim_buf, &ctx->vbin_lists,
-		&ctx->vbin_counts};
+		&ctx->vbin_counts, &ctx->vbin_first};
 	for (DevBuf* b : bufs) release(*b);
 	for (const SwCtx::HostRange& h : ctx->registered) cudaHostUnregister(h.ptr);
 	if (ctx->gexec) cudaGraphExecDestroy(ctx->gexec);
@@ -1825,6 +1828,7 @@ int enqueue_frame(SwCtx* ctx, const SwFrameInput& f, const unsigned char* h, con
 			va.framebuffer = target;
 			va.bin_lists = static_cast<uint32_t*>(ctx->vbin_lists.ptr);
 			va.bin_counts = static_cast<uint32_t*>(ctx->vbin_counts.ptr);
+			va.bin_first = static_cast<RasterBox*>(ctx->vbin_first.ptr);
 			va.bin_cap = ctx->vbin_cap;
 			va.bins_x = raster_bins(int32_t(v.width), RASTER_BIN_W);
 			va.bins_y = raster_bins(int32_t(v.height), RASTER_BIN_H);
