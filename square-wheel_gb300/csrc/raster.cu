@@ -687,7 +687,7 @@ __device__ __forceinline__ uint32_t z_of(uint32_t zdiv)
 {
 	if (zdiv < 512u) return (1u << Z_CALC_SHIFT) / (zdiv ? zdiv : 1u);
 	float inv;
-	asm("rcp.approx.f32 %0, %1;" : "=f"(inv) : "f"(__uint2float_rn(zdiv)));
+	asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(__uint2float_rn(zdiv)));
 	uint32_t q = __float_as_uint(fadd(fmul(inv, 2147483648.0f), 8388608.0f)) & 0x7FFFFFu;
 	const int32_t r = int32_t((1u << Z_CALC_SHIFT) - q * zdiv); // in (-zdiv, 2 * zdiv)
 	if (r < 0)
