@@ -554,64 +554,84 @@ __device__ RasterRow row_setup(const SwDrawCmd& d, const DrawEq& e, const Raster
 	return r;
 }
 
-// Raster setup of one draw per CTA. The draw and its vertices are staged in shared memory; thread 0
-// runs the edge walk into shared memory (its loop reads vertices on the walk's dependency chain, which
-// from shared memory costs a few cycles per step) and writes the draw's tile-binning box (conservative:
-// x is linear in the row, so its extremes over a part are at the part's first and last rows) and the
-// per-draw record of the tile kernel; then every thread sets up rows of the draw (its row records,
-// numbered by the host in draw order) from those parts.
-__global__ void __launch_bounds__(256) raster_setup_kernel(RasterArgs a)
+// Raster setup, DRAWS draws per CTA: one (every thread takes rows of it) or eight (a warp each). The draw and its
+// vertices are staged in shared memory; the group's first warp runs the edge walk there (its loop reads vertices on
+// the walk's dependency chain) and thread 0 writes the draw's tile-binning box (conservative: x is linear in the row,
+// so its extremes over a part are at the part's first and last rows) and the per-draw record of the tile kernel; then
+// every thread of the group sets up rows of the draw (its row records, numbered by the host in draw order).
+// Bound by latency: with one draw per CTA 304 draws are in flight, which is what a frame of a few hundred polygons of up
+// to a screen's height needs; 4,096 draws of 90 rows took 72 us that way and take 30 with a warp each, 2,363 with
+// triangles among them 97 and 42. At 512 draws a lone pass is 8% slower with a warp each (100 us against 92), although
+// overlapped passes gain 9%; at 300 a lone frame loses 11% and overlapped ones gain nothing.
+struct SetupShared
 {
-	__shared__ __align__(8) SwDrawCmd s_d;
-	__shared__ SwVertex16 s_v[SW_MAX_POLYGON_VERTICES];
-	__shared__ SwTriVertex s_tv[3];
-	__shared__ RasterPart s_parts[SW_RASTER_MAX_PARTS];
-	__shared__ DrawRows s_dr;
-	__shared__ uint32_t s_np, s_steps_count;
-	__shared__ WalkStep s_steps[MAX_WALK_STEPS];
-	// One draw per CTA; with the draw count on the device (GPU-side preparation) a fixed grid strides.
+	__align__(8) SwDrawCmd d;
+	SwVertex16 v[SW_MAX_POLYGON_VERTICES];
+	SwTriVertex tv[3];
+	RasterPart parts[SW_RASTER_MAX_PARTS];
+	DrawRows dr;
+	uint32_t np, steps_count;
+	WalkStep steps[MAX_WALK_STEPS];
+};
+
+template <int DRAWS>
+__global__ void __launch_bounds__(256, DRAWS == 1 ? 2 : 3) raster_setup_kernel(RasterArgs a)
+{
+	static_assert(DRAWS == 1 || DRAWS == 8, "a CTA or a warp per draw");
+	constexpr uint32_t THREADS = 256 / DRAWS; // per draw
+	__shared__ SetupShared s_all[DRAWS];
+	const uint32_t group = threadIdx.x / THREADS, thread = threadIdx.x % THREADS;
+	SetupShared& sh = s_all[group];
+	SwDrawCmd& s_d = sh.d;
+	auto sync = [] {
+		if constexpr (DRAWS == 1)
+			__syncthreads();
+		else
+			__syncwarp();
+	};
+	// With the draw count on the device (GPU-side preparation) a fixed grid strides.
 	const uint32_t num_draws = a.counts ? a.counts->num_draws : a.num_draws;
-	for (uint32_t di = blockIdx.x; di < num_draws; di += gridDim.x)
+	for (uint32_t di = blockIdx.x * DRAWS + group; di < num_draws; di += gridDim.x * DRAWS)
 	{
-		static_assert(sizeof(SwDrawCmd) % 4 == 0 && sizeof(SwDrawCmd) / 4 <= 256, "draw record");
-		if (threadIdx.x < sizeof(SwDrawCmd) / 4)
-			reinterpret_cast<uint32_t*>(&s_d)[threadIdx.x] = reinterpret_cast<const uint32_t*>(a.draws + di)[threadIdx.x];
-		if (threadIdx.x == 0) s_dr = a.draw_rows[di];
-		__syncthreads();
+		static_assert(sizeof(SwDrawCmd) % 4 == 0, "draw record");
+		for (uint32_t i = thread; i < sizeof(SwDrawCmd) / 4; i += THREADS)
+			reinterpret_cast<uint32_t*>(&s_d)[i] = reinterpret_cast<const uint32_t*>(a.draws + di)[i];
+		if (thread == 0) sh.dr = a.draw_rows[di];
+		sync();
 		const bool tri = s_d.mode == SW_RASTER_TRIANGLE;
 		if (tri)
 		{
-			if (threadIdx.x < 3) s_tv[threadIdx.x] = a.tri_vertices[s_d.first_vertex + threadIdx.x];
+			if (thread < 3) sh.tv[thread] = a.tri_vertices[s_d.first_vertex + thread];
 		}
-		else if (threadIdx.x < s_d.vertex_count && threadIdx.x < SW_MAX_POLYGON_VERTICES)
-			s_v[threadIdx.x] = a.vertices[s_d.first_vertex + threadIdx.x];
-		__syncthreads();
+		else if (thread < s_d.vertex_count && thread < SW_MAX_POLYGON_VERTICES)
+			sh.v[thread] = a.vertices[s_d.first_vertex + thread];
+		sync();
 		uint32_t walked = 0;
-		if (!tri && threadIdx.x < 32) walked = edge_walk_warp(s_d, s_v, a.height, s_parts, s_steps, &s_steps_count);
-		if (threadIdx.x == 0)
+		if (!tri && thread < 32) walked = edge_walk_warp(s_d, sh.v, a.height, sh.parts, sh.steps, &sh.steps_count);
+		if (thread == 0)
 		{
 			const SwDrawCmd& d = s_d;
 			uint32_t np;
 			if (tri)
 			{
-				np = triangle_setup(s_tv, int32_t(d.tex_size[0]), int32_t(d.tex_size[1]), a.height, s_parts);
+				np = triangle_setup(sh.tv, int32_t(d.tex_size[0]), int32_t(d.tex_size[1]), a.height, sh.parts);
 				for (uint32_t pi = 0; pi < np; ++pi)
 				{
 					TriSteps ts;
-					ts.d_tc_dx[0] = s_parts[pi].tc_right0[0];
-					ts.d_tc_dx[1] = s_parts[pi].tc_right0[1];
-					for (int i = 0; i < 3; ++i) ts.d_light_dx[i] = s_parts[pi].d_light_dx[i];
+					ts.d_tc_dx[0] = sh.parts[pi].tc_right0[0];
+					ts.d_tc_dx[1] = sh.parts[pi].tc_right0[1];
+					for (int i = 0; i < 3; ++i) ts.d_light_dx[i] = sh.parts[pi].d_light_dx[i];
 					ts.reserved = 0;
 					a.tri_steps[uint64_t(di) * 2 + pi] = ts;
 				}
 			}
 			else
 				np = walked;
-			s_np = np;
+			sh.np = np;
 			int32_t bx0 = INT32_MAX, bx1 = INT32_MIN, by0 = INT32_MAX, by1 = INT32_MIN;
 			for (uint32_t pi = 0; pi < np; ++pi)
 			{
-				const RasterPart& p = s_parts[pi];
+				const RasterPart& p = sh.parts[pi];
 				const int32_t last = p.y_end_int - 1 - p.y_start_int;
 				bx0 = min(bx0, min(p.x_left0 >> 16, wadd(p.x_left0, wmul(last, p.dx_dy_left)) >> 16));
 				bx1 = max(bx1, max(p.x_right0 >> 16, wadd(p.x_right0, wmul(last, p.dx_dy_right)) >> 16));
@@ -620,7 +640,7 @@ __global__ void __launch_bounds__(256) raster_setup_kernel(RasterArgs a)
 			}
 			bx0 = max(bx0, 0);
 			bx1 = min(bx1, a.width);
-			const DrawRows dr = s_dr;
+			const DrawRows dr = sh.dr;
 			// Rows outside the host's row range have no record; clamp the box to it.
 			by0 = max(by0, dr.y0);
 			by1 = min(by1, dr.y0 + int32_t(dr.nrows));
@@ -640,11 +660,11 @@ __global__ void __launch_bounds__(256) raster_setup_kernel(RasterArgs a)
 			rd.tex_source = uint16_t(d.tex_source);
 			a.rdraws[di] = rd;
 		}
-		__syncthreads();
-		const uint32_t np = s_np;
+		sync();
+		const uint32_t np = sh.np;
 		const DrawEq e = draw_equations(s_d);
-		const DrawRows dr = s_dr;
-		for (uint32_t k = threadIdx.x; k < dr.nrows; k += blockDim.x)
+		const DrawRows dr = sh.dr;
+		for (uint32_t k = thread; k < dr.nrows; k += THREADS)
 		{
 			const int32_t y = dr.y0 + int32_t(k);
 			RasterRow row;
@@ -652,7 +672,7 @@ __global__ void __launch_bounds__(256) raster_setup_kernel(RasterArgs a)
 			row.a0 = row.b0 = row.a1 = row.b1 = row.a2 = row.b2 = 0;
 			for (uint32_t pi = 0; pi < np; ++pi)
 			{
-				const RasterPart& p = s_parts[pi];
+				const RasterPart& p = sh.parts[pi];
 				if (y >= p.y_start_int && y < p.y_end_int)
 				{
 					row = s_d.mode == SW_RASTER_TRIANGLE ? triangle_row(p, y, a.width, di * 2 + pi) : row_setup(s_d, e, p, y, a.width);
@@ -661,7 +681,7 @@ __global__ void __launch_bounds__(256) raster_setup_kernel(RasterArgs a)
 			}
 			a.rows[dr.row_base + k] = row;
 		}
-		__syncthreads(); // the shared records are reused by the CTA's next draw
+		sync(); // the shared records are reused by the group's next draw
 	}
 }
 
@@ -1498,12 +1518,17 @@ int launch_shadow_rebase(unsigned long long* storage, uint64_t num_texels, cudaS
 
 int launch_raster_setup(const RasterArgs& args, cudaStream_t stream)
 {
+	// A CTA per draw while the CTAs fit on the GPU a few times over, else a warp per draw (both sides measured: the
+	// kernel's comment).
+	constexpr uint32_t WARP_DRAWS_FROM = 1024;
 	if (args.counts)
 	{
-		if (args.setup_blocks > 0) raster_setup_kernel<<<args.setup_blocks, 256, 0, stream>>>(args);
+		if (args.setup_blocks > 0) raster_setup_kernel<1><<<args.setup_blocks, 256, 0, stream>>>(args);
 	}
+	else if (args.num_draws >= WARP_DRAWS_FROM)
+		raster_setup_kernel<8><<<(args.num_draws + 7) / 8, 256, 0, stream>>>(args);
 	else if (args.num_draws > 0)
-		raster_setup_kernel<<<args.num_draws, 256, 0, stream>>>(args);
+		raster_setup_kernel<1><<<args.num_draws, 256, 0, stream>>>(args);
 	return int(cudaGetLastError());
 }
 
