@@ -10,11 +10,9 @@
 // padding pixels are zeroed once at allocation and never written, which gives the zero padding of the
 // convolution and of its transpose.
 //
-// conv_kernel: one CTA = 4 output rows x 128 pixels of one image. One thread bulk-copies (TMA, untiled)
-// the 6 input rows x chunks x 130 pixels and the packed weights into shared memory, issues
-// 4 rows x 9 taps x (chunks / 2) MMAs of 128 x N x 16 into TMEM (4 x N columns), and commits to an
-// mbarrier; 4 warps then read the accumulators (warp w = TMEM lanes 32w.., i.e. pixels 32w..) and run
-// the epilogue: bias + ReLU (forward), ReLU mask (input gradient), or the output stage (pixel shuffle +
+// conv_kernel: persistent CTAs with rows of 128 pixels of their own; input rows come in by tiled TMA, their MMAs of
+// 128 x 3N x 16 accumulate into a ring of output rows in TMEM, and epilogue warps (warp w = TMEM lanes 32 * (w % 4)..,
+// i.e. pixels) apply bias + ReLU (forward), the ReLU mask (input gradient) or the output stage (pixel shuffle +
 // bilinear residual, written as Color32 for inference or as the loss gradient for training).
 // wgrad_kernel: weight gradient dW[co][dy][dx][ci] = sum_p G[p][co] X[p + (dy, dx)][ci] with both operands
 // MN-major: D rows = (dy, chunk, ci % 8) groups at a uniform shared-memory stride, D columns = co, one
@@ -169,35 +167,68 @@ __device__ __forceinline__ RowRange cta_rows(uint32_t total)
 	return RowRange{uint32_t(uint64_t(blockIdx.x) * total / gridDim.x), uint32_t(uint64_t(blockIdx.x + 1) * total / gridDim.x)};
 }
 
-// Epilogue of one output row for the 128 pixels of a tile: thread = pixel x, v = the row's N accumulators
-// (all N loaded; `half` selects the work share of the two warps reading the same TMEM lane quadrant):
-//   EPI_RELU / EPI_MASK: channels [half * N / 2, (half + 1) * N / 2);
-//   EPI_INFER: output row 2y + half;  EPI_LOSS: half 0 only (the loss gradient planes need whole pixels).
-template <int N, int EPI, int half>
-__device__ __forceinline__ void conv_epilogue(const ConvArgs& a, const float (&v)[N], const float (&bias)[N], uint32_t img,
-	int x, int y, float& loss)
+// What the epilogue of one output pixel reads from global memory: the stored activations whose sign gates the gradient
+// (EPI_MASK), the source pixels of the bilinear upsample (EPI_INFER, EPI_LOSS) and the four target pixels (EPI_LOSS).
+// None of it depends on the accumulators, so it is loaded before the wait for them.
+template <int N, int EPI>
+struct EpiOperands
+{
+	uint4 mask[EPI == EPI_MASK ? N / 8 : 1];
+	uint32_t src[EPI == EPI_INFER || EPI == EPI_LOSS ? 9 : 1]; // rows y - 1, y, y + 1, columns x - 1, x, x + 1, edges clamped
+	uint2 target[EPI == EPI_LOSS ? 2 : 1];
+};
+
+template <int N, int EPI>
+__device__ __forceinline__ void load_operands(const ConvArgs& a, uint32_t img, int x, int y, EpiOperands<N, EPI>& op)
+{
+	if (x >= int(a.in.width) || y >= int(a.in.height)) return;
+	if (EPI == EPI_MASK)
+	{
+		const uint16_t* msk = a.mask.data + planes_index(a.mask, img, y, 0, x);
+#pragma unroll
+		for (int c8 = 0; c8 < N / 8; ++c8) op.mask[c8] = *reinterpret_cast<const uint4*>(msk + c8 * (size_t(a.mask.wp) * 8));
+	}
+	else if (EPI == EPI_INFER || EPI == EPI_LOSS)
+	{
+		const CropGpu c = a.crops[img];
+		const int lx = c.x + x, ly = c.y + y;
+		const int xs[3] = {max(lx - 1, 0), lx, min(lx + 1, int(c.lo_w) - 1)};
+		const int ys[3] = {max(ly - 1, 0), ly, min(ly + 1, int(c.lo_h) - 1)};
+#pragma unroll
+		for (int j = 0; j < 3; ++j)
+#pragma unroll
+			for (int i = 0; i < 3; ++i) op.src[j * 3 + i] = c.lo[size_t(ys[j]) * c.lo_pitch + xs[i]];
+		if (EPI == EPI_LOSS)
+#pragma unroll
+			for (int sy = 0; sy < 2; ++sy)
+				op.target[sy] = *reinterpret_cast<const uint2*>(c.hi + size_t(2 * ly + sy) * c.hi_pitch + 2 * lx);
+	}
+}
+
+// Epilogue of channels c0 .. c0 + 15 of one output pixel: v = their accumulators, bias = theirs.
+template <int N, int EPI>
+__device__ __forceinline__ void conv_epilogue(const ConvArgs& a, const EpiOperands<N, EPI>& op, const float (&v)[16],
+	const float* bias, int c0, uint32_t img, int x, int y, float& loss)
 {
 	if (x >= int(a.in.width) || y >= int(a.in.height)) return; // padding pixels stay zero
 	if (EPI == EPI_RELU || EPI == EPI_MASK)
 	{
-		uint16_t* out = a.out.data + planes_index(a.out, img, y, 0, x);
 		const size_t cstride = size_t(a.out.wp) * 8;
-		const uint16_t* msk = EPI == EPI_MASK ? a.mask.data + planes_index(a.mask, img, y, 0, x) : nullptr;
+		uint16_t* out = a.out.data + planes_index(a.out, img, y, 0, x) + (c0 / 8) * cstride;
 #pragma unroll
-		for (int cc = 0; cc < N / 16; ++cc)
+		for (int c8 = 0; c8 < 2; ++c8)
 		{
-			const int c8 = half * (N / 16) + cc;
 			uint32_t o[4];
 			if (EPI == EPI_RELU)
 			{
 #pragma unroll
 				for (int q = 0; q < 4; ++q)
-					o[q] = pack2(fmaxf(v[c8 * 8 + 2 * q] + bias[c8 * 8 + 2 * q], 0.0f),
-						fmaxf(v[c8 * 8 + 2 * q + 1] + bias[c8 * 8 + 2 * q + 1], 0.0f));
+					o[q] = pack2(fmaxf(v[c8 * 8 + 2 * q] + bias[c0 + c8 * 8 + 2 * q], 0.0f),
+						fmaxf(v[c8 * 8 + 2 * q + 1] + bias[c0 + c8 * 8 + 2 * q + 1], 0.0f));
 			}
 			else
 			{
-				const uint4 m = *reinterpret_cast<const uint4*>(msk + c8 * cstride);
+				const uint4 m = op.mask[EPI == EPI_MASK ? c0 / 8 + c8 : 0];
 				const uint32_t mw[4] = {m.x, m.y, m.z, m.w};
 #pragma unroll
 				for (int q = 0; q < 4; ++q)
@@ -215,31 +246,17 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, const float (&v
 	{
 		// Output stage: channel c*4 + sy*2 + sx is colour c of output pixel (2x + sx, 2y + sy), added to
 		// the bilinear 2x upsample of the source (weights 3/4, 1/4; edges clamped).
-		if (EPI == EPI_LOSS && half) return;
-		const CropGpu c = a.crops[img];
-		const int lx = c.x + x, ly = c.y + y;
-		const int xs[3] = {max(lx - 1, 0), lx, min(lx + 1, int(c.lo_w) - 1)};
-		const int ys[3] = {max(ly - 1, 0), ly, min(ly + 1, int(c.lo_h) - 1)};
 		float g[16];
 #pragma unroll
 		for (int j = 0; j < 16; ++j) g[j] = 0.0f;
 		const bool in_loss = EPI == EPI_LOSS && x >= int(a.margin) && x < int(a.in.width - a.margin) &&
 			y >= int(a.margin) && y < int(a.in.height - a.margin);
+		const uint32_t p11 = op.src[4], p10 = op.src[3], p12 = op.src[5];
 #pragma unroll
 		for (int sy = 0; sy < 2; ++sy)
 		{
-			if (EPI == EPI_INFER && sy != half) continue;
-			const uint32_t* r1 = c.lo + size_t(ly) * c.lo_pitch;
-			const uint32_t* r2 = c.lo + size_t(ys[sy ? 2 : 0]) * c.lo_pitch;
-			const uint32_t p11 = r1[lx], p10 = r1[xs[0]], p12 = r1[xs[2]];
-			const uint32_t p21 = r2[lx], p20 = r2[xs[0]], p22 = r2[xs[2]];
-			uint32_t tp[2] = {0u, 0u};
-			if (EPI == EPI_LOSS)
-			{
-				const uint2 t2 = *reinterpret_cast<const uint2*>(c.hi + size_t(2 * ly + sy) * c.hi_pitch + 2 * lx);
-				tp[0] = t2.x;
-				tp[1] = t2.y;
-			}
+			const uint32_t p21 = op.src[sy ? 7 : 1], p20 = op.src[sy ? 6 : 0], p22 = op.src[sy ? 8 : 2];
+			const uint32_t tp[2] = {op.target[EPI == EPI_LOSS ? sy : 0].x, op.target[EPI == EPI_LOSS ? sy : 0].y};
 			uint32_t px[2];
 #pragma unroll
 			for (int sx = 0; sx < 2; ++sx)
@@ -265,7 +282,8 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, const float (&v
 				px[sx] = bytes;
 			}
 			if (EPI == EPI_INFER)
-				*reinterpret_cast<uint2*>(a.hi_out + size_t(2 * ly + sy) * a.hi_pitch + 2 * lx) = make_uint2(px[0], px[1]);
+				*reinterpret_cast<uint2*>(a.hi_out + size_t(2 * (a.crops[img].y + y) + sy) * a.hi_pitch + 2 * (a.crops[img].x + x)) =
+					make_uint2(px[0], px[1]);
 		}
 		if (EPI == EPI_LOSS)
 		{
@@ -295,32 +313,22 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, const float (&v
 //   warp 1 (lane 0 issues; the warp owns the TMEM allocation): per input row waits for it (and, when it
 //     starts a new output row, for that row's accumulator to be free), issues the MMAs and commits the
 //     row to rowbar[k % NBAR]: that releases the input row's slot and completes output row y_in - 1;
-//   warps 2..9: per output row: TMEM -> registers (warp w reads lanes 32*(w%4).., i.e. pixels), zero
-//     the accumulator, release it, run the epilogue and store (the two warps of a lane quadrant split
-//     the columns and the epilogue work).
+//   warps 2..9: two groups of four (warp w reads TMEM lanes 32*(w%4).., i.e. pixels) taking alternate output
+//     rows: what the row's epilogue reads from global memory is loaded first, then TMEM -> registers, the
+//     accumulator is zeroed and released, and the epilogue stores the row.
 // The issuing thread's own instruction latency bounds the MMA rate, so the common case (three
 // contributions, no ring wrap) is straight-line code with compile-time descriptor offsets.
+// At a training step's sizes a CTA has three or four rows, so the kernel is bound by the latency of one row's chain
+// (load, MMAs, epilogue). A training step of 16 crops took 181 us with all eight warps on one row and the operands
+// loaded after the accumulators, and takes 163 this way.
 // Every wait is bounded: on expiry the role stops, the error flag is set, and the CTA still waits for
 // its own MMAs and copies before freeing TMEM.
 constexpr int CONV_THREADS = 320;
 constexpr int CONV_EPI_WARPS = 8;
 constexpr int NBAR = 16; // row-completion barriers (more than the rows the MMA issuer can run ahead)
 
-// Named barrier 1 of the 8 epilogue warps; epi_any is the same barrier returning the OR of `v` over them
-// (so all eight take the same branch).
-__device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
-__device__ __forceinline__ bool epi_any(bool v)
-{
-	uint32_t r;
-	asm volatile("{\n\t.reg .pred q, p;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.or.pred p, 1, 256, q;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-				 : "=r"(r)
-				 : "r"(v ? 1u : 0u)
-				 : "memory");
-	return r != 0;
-}
-
 template <int C8, int N, int EPI>
-__global__ void __launch_bounds__(CONV_THREADS, 1) conv_kernel(const __grid_constant__ ConvArgs a)
+__global__ void __launch_bounds__(CONV_THREADS, 2) conv_kernel(const __grid_constant__ ConvArgs a)
 {
 	constexpr int KSTEPS = C8 / 2;      // 16-channel steps per horizontal tap
 	constexpr int NB = 3 * N;           // MMA N for a whole input row
@@ -340,6 +348,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) conv_kernel(const __grid_cons
 	uint64_t* donebar = wbar + 1;
 	uint32_t* s_tmem = reinterpret_cast<uint32_t*>(donebar + 1);
 	float* s_red = reinterpret_cast<float*>(s_tmem + 4); // [CONV_EPI_WARPS]
+	float* s_bias = s_red + CONV_EPI_WARPS;              // [N]
 
 	const int tid = threadIdx.x, lane = tid & 31;
 	const int warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0); // known to be the same in the whole warp
@@ -351,7 +360,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) conv_kernel(const __grid_cons
 	{
 		for (int i = 0; i < NSTAGE; ++i) mbar_init(&full[i], 1);
 		for (int i = 0; i < NBAR; ++i) mbar_init(&rowbar[i], 1);
-		for (int i = 0; i < R; ++i) mbar_init(&acce[i], CONV_EPI_WARPS);
+		for (int i = 0; i < R; ++i) mbar_init(&acce[i], CONV_EPI_WARPS / 2);
 		mbar_init(wbar, 1);
 		mbar_init(donebar, 1);
 		fence_mbar_init();
@@ -491,53 +500,53 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) conv_kernel(const __grid_cons
 	}
 	else
 	{
-		const int quad = warp & 3, half = (warp - 2) >> 2;
+		const int quad = warp & 3;
+		const uint32_t group = uint32_t(warp - 2) >> 2;
 		const uint32_t lane_base = uint32_t(quad * 32) << 16;
-		float bias[N];
-#pragma unroll
-		for (int c = 0; c < N; ++c) bias[c] = EPI == EPI_MASK ? 0.0f : a.bias[c];
+		if (EPI != EPI_MASK)
+		{
+			// the same values from either group; a warp reads what its own lanes wrote
+			if (lane < N) s_bias[lane] = a.bias[lane];
+			__syncwarp();
+		}
 		float loss = 0.0f;
 		uint32_t o = 0, k_base = 0;
+		EpiOperands<N, EPI> op, next;
 		for (uint32_t r = rows.begin; r < rows.end && !failed;)
 		{
 			const uint32_t strip = r / H, y_lo = r % H, y_hi = min(H, y_lo + (rows.end - r));
 			r += y_hi - y_lo;
 			const uint32_t img = strip / tiles_x;
 			const int x = int(strip % tiles_x) * TILE_X + quad * 32 + lane;
-			for (uint32_t y = y_lo; y < y_hi; ++y, ++o)
+			const uint32_t y_first = y_lo + ((o ^ group) & 1u); // this group's rows: those of its counter's parity
+			if (y_first < y_hi) load_operands<N, EPI>(a, img, x, int(y_first), next);
+			for (uint32_t y = y_first; y < y_hi; y += 2)
 			{
+				op = next;
+				if (y + 2 < y_hi) load_operands<N, EPI>(a, img, x, int(y + 2), next);
 				// output row y is complete once input row y + 1 (ring entry k_base + y - y_lo + 2) is committed
 				const uint32_t kc = k_base + (y - y_lo) + 2;
-				const bool ok = mbar_wait_bounded(&rowbar[kc % NBAR], (kc / NBAR) & 1, POLL_LIMIT);
-				if (epi_any(!ok))
+				if (!mbar_wait_warp(&rowbar[kc % NBAR], (kc / NBAR) & 1, POLL_LIMIT))
 				{
 					failed = true;
 					break;
 				}
 				fence_after_sync();
-				const uint32_t b = (R - o % R) % R;
-				float v[N];
+				const uint32_t b = (R - (o + (y - y_lo)) % R) % R;
+				float v[N / 16][16];
 #pragma unroll
-				for (int c8 = 0; c8 < N / 8; ++c8)
-				{
-					float t8[8];
-					tmem_ld8(tmem + lane_base + b * N + c8 * 8, t8);
-#pragma unroll
-					for (int e = 0; e < 8; ++e) v[c8 * 8 + e] = t8[e];
-				}
+				for (int c = 0; c < N / 16; ++c) tmem_ld(tmem + lane_base + b * N + c * 16, v[c]);
 				tmem_ld_wait();
-				epi_sync(); // both warps of the quadrant have read the accumulator
 #pragma unroll
-				for (int c8 = 0; c8 < N / 16; ++c8) tmem_zero8(tmem + lane_base + b * N + (half * (N / 16) + c8) * 8);
+				for (int c8 = 0; c8 < N / 8; ++c8) tmem_zero8(tmem + lane_base + b * N + c8 * 8);
 				tmem_st_wait();
 				fence_before_sync();
 				__syncwarp();
 				if (lane == 0) mbar_arrive(&acce[b]);
-				if (half)
-					conv_epilogue<N, EPI, 1>(a, v, bias, img, x, int(y), loss);
-				else
-					conv_epilogue<N, EPI, 0>(a, v, bias, img, x, int(y), loss);
+#pragma unroll
+				for (int c = 0; c < N / 16; ++c) conv_epilogue<N, EPI>(a, op, v[c], s_bias, c * 16, img, x, int(y), loss);
 			}
+			o += y_hi - y_lo;
 			k_base += (y_hi - y_lo) + 2;
 		}
 		if (EPI == EPI_LOSS)
