@@ -15,8 +15,8 @@
 // i.e. pixels) apply bias + ReLU (forward), the ReLU mask (input gradient) or the output stage (pixel shuffle +
 // bilinear residual, written as Color32 for inference or as the loss gradient for training).
 // wgrad_kernel: weight gradient dW[co][dy][dx][ci] = sum_p G[p][co] X[p + (dy, dx)][ci] with both operands
-// MN-major: D rows = (dy, chunk, ci % 8) groups at a uniform shared-memory stride, D columns = co, one
-// accumulator per dx, K = 16 pixels per MMA; per-CTA partial sums are reduced in a fixed order.
+// MN-major: D rows = (input row, chunk, ci % 8) groups at a uniform shared-memory stride, D columns = (gradient row,
+// co), one accumulator per dx, K = 16 pixels per MMA; per-CTA partial sums are reduced in a fixed order.
 #include "sw_kernels.cuh"
 #include "tc05.cuh"
 
@@ -42,8 +42,6 @@ namespace
 
 constexpr int TILE_X = 128;            // pixels per M tile
 constexpr int ROWS = 4;                // output rows per CTA
-constexpr int XS = TILE_X + 2;         // staged pixels per row and chunk (one halo pixel each side)
-constexpr uint32_t XS_BYTES = XS * 16; // 2080
 constexpr uint32_t POLL_LIMIT = 1u << 21;
 constexpr int NUM_LAYERS = 4;
 
@@ -1094,12 +1092,16 @@ __global__ void __launch_bounds__(F_THREADS, 1) fused_upscale_kernel(const __gri
 
 // ---- weight gradient ----
 
+struct WgradLayer
+{
+	Planes x; // layer input
+	Planes g; // pre-activation gradient
+	float* partial; // per CTA: [3 dx][wgrad_rows(C8X)][NG] then the bias partials [NG]
+};
 struct WgradArgs
 {
-	Planes x; // layer input (C8X chunks)
-	Planes g; // pre-activation gradient (NG / 8 chunks)
-	float* partial;    // per CTA: [3 dx][wgrad_rows(C8X)][NG] then the bias partials [NG]
-	uint32_t tiles_x, row_blocks;
+	WgradLayer layer[NUM_LAYERS];
+	uint32_t blocks; // per layer: images * height / ROWS
 	int* error;
 };
 
@@ -1107,84 +1109,71 @@ struct WgradArgs
 __host__ __device__ constexpr uint32_t wgrad_rows(int c8x) { return 3 * c8x * 8; }
 __host__ __device__ constexpr uint32_t wgrad_partial_floats(int c8x, int ng) { return 3 * wgrad_rows(c8x) * ng + ng; }
 
-template <int C8X, int NG>
-__global__ void __launch_bounds__(128) wgrad_kernel(WgradArgs a)
+// Crops are one tile wide and their planes CXS pixels, so a row (all its chunks) is one run of memory, and so are
+// neighbouring rows.
+static_assert(SW_UPSCALER_CROP_W == TILE_X && SW_UPSCALER_CROP_H % ROWS == 0, "a CTA's rows are whole rows of one crop");
+constexpr int WG_XROWS = ROWS + 2; // staged input rows
+constexpr int WG_STEPS = ROWS / 2; // two gradient rows per MMA
+constexpr uint32_t WG_X_BYTES = WG_XROWS * 4 * CXS_BYTES, WG_G_BYTES = ROWS * 4 * CXS_BYTES;
+constexpr uint32_t WG_TMEM_COLS = 256;
+struct WgradSmem
 {
-	constexpr int DY = 16 / C8X;         // dy groups stacked in M (only the first 3 are taps)
-	constexpr int XROWS = ROWS + DY - 1; // staged input rows
-	constexpr int G8 = NG / 8;
-	constexpr uint32_t X_BYTES = XROWS * C8X * XS_BYTES;
-	constexpr uint32_t G_BYTES = ROWS * G8 * XS_BYTES;
-	constexpr uint32_t TMEM_COLS = 3 * NG <= 64 ? 64 : 128;
-	extern __shared__ __align__(1024) unsigned char smem[];
-	unsigned char* s_x = smem;
-	unsigned char* s_g = smem + X_BYTES;
-	uint64_t* bars = reinterpret_cast<uint64_t*>(smem + X_BYTES + G_BYTES);
-	uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + 2);
-	float* s_bias = reinterpret_cast<float*>(bars + 4); // [128]
+	static constexpr uint32_t X = 0, G = WG_X_BYTES, BARS = G + WG_G_BYTES; // bars: [WG_STEPS] rows loaded, then MMAs done
+	static constexpr uint32_t TMEM = BARS + (WG_STEPS + 1) * 8, BIAS = TMEM + 8, TOTAL = BIAS + 128 * 4;
+};
 
+// One layer's share of a CTA: ROWS rows of one crop.
+template <int C8X, int NG>
+__device__ __forceinline__ bool wgrad_rows_block(const WgradLayer& a, uint32_t bid, unsigned char* smem, uint32_t tmem)
+{
+	constexpr int XM = 16 / C8X; // input rows stacked in M; the first four meet a gradient row
+	constexpr int G8 = NG / 8;
+	constexpr uint32_t X_ROW = C8X * CXS_BYTES, G_ROW = G8 * CXS_BYTES;
+	constexpr uint32_t MR = wgrad_rows(C8X);
+	constexpr uint32_t LINE = NG + 4; // floats between the rows of the sums (conflict-free 16-byte accesses)
+	// the rows of M that meet no gradient row read whatever lies behind the staged rows
+	static_assert(XM >= 4 && (ROWS - 2 + XM) * X_ROW <= WgradSmem::BARS && WG_XROWS * X_ROW <= WG_X_BYTES, "staged rows");
+	static_assert(3 * 2 * NG <= int(WG_TMEM_COLS) && 3 * MR * LINE * 4 <= WgradSmem::BARS, "accumulators");
+	unsigned char* s_x = smem + WgradSmem::X;
+	unsigned char* s_g = smem + WgradSmem::G;
+	uint64_t* bars = reinterpret_cast<uint64_t*>(smem + WgradSmem::BARS);
+	float* s_bias = reinterpret_cast<float*>(smem + WgradSmem::BIAS);
 	const int tid = threadIdx.x, lane = tid & 31;
 	const int warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0); // known to be the same in the whole warp
-	uint32_t bid = blockIdx.x;
-	const uint32_t tx = bid % a.tiles_x;
-	bid /= a.tiles_x;
-	const uint32_t rb = bid % a.row_blocks;
-	const uint32_t img = bid / a.row_blocks;
-	const int x0 = int(tx) * TILE_X, y0 = int(rb) * ROWS;
-
+	const uint32_t row_blocks = a.x.height / ROWS;
+	const uint32_t img = bid / row_blocks;
+	const int y0 = int(bid % row_blocks) * ROWS;
+	bool ok = true;
 	if (tid == 0)
-	{
-		mbar_init(&bars[0], 1);
-		mbar_init(&bars[1], 1);
-		fence_mbar_init();
-	}
-	if (warp == 0)
-	{
-		tmem_alloc(s_tmem, TMEM_COLS);
-		tmem_relinquish();
-	}
-	fence_before_sync();
-	__syncthreads();
-	fence_after_sync();
-	const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, *s_tmem, 0);
-	pdl_trigger();
-	pdl_wait(); // the planes are written
-
-	if (tid == 0)
-	{
-		mbar_expect_tx(&bars[0], X_BYTES + G_BYTES);
-		for (int r = 0; r < XROWS; ++r)
-			for (int c = 0; c < C8X; ++c)
-				bulk_g2s(s_x + (r * C8X + c) * XS_BYTES, a.x.data + planes_index(a.x, img, y0 - 1 + r, c, x0 - 1), XS_BYTES, &bars[0]);
-		for (int r = 0; r < ROWS; ++r)
-			for (int c = 0; c < G8; ++c)
-				bulk_g2s(s_g + (r * G8 + c) * XS_BYTES, a.g.data + planes_index(a.g, img, y0 + r, c, x0 - 1), XS_BYTES, &bars[0]);
-	}
-	const bool loaded = mbar_wait_bounded(&bars[0], 0, POLL_LIMIT);
-	if (__syncthreads_or(!loaded))
-	{
-		if (tid == 0) atomicExch(a.error, 3);
-		mbar_wait_bounded(&bars[0], 0, POLL_LIMIT);
-		__syncthreads();
-		if (warp == 0) tmem_dealloc(tmem, TMEM_COLS);
-		return;
-	}
+		for (int t = 0; t < WG_STEPS; ++t)
+		{
+			// the input rows y0 + 2t - 1 .. y0 + 2t + 2 that are not staged yet, and gradient rows y0 + 2t, y0 + 2t + 1
+			const int first = t ? 2 * t + 2 : 0, n = t ? 2 : 4;
+			mbar_expect_tx(&bars[t], n * X_ROW + 2 * G_ROW);
+			bulk_g2s(s_x + first * X_ROW, a.x.data + planes_index(a.x, img, y0 - 1 + first, 0, -1), n * X_ROW, &bars[t]);
+			bulk_g2s(s_g + 2 * t * G_ROW, a.g.data + planes_index(a.g, img, y0 + 2 * t, 0, -1), 2 * G_ROW, &bars[t]);
+		}
 	if (warp == 0)
 	{
 		const uint32_t issue = lane == 0 ? 1u : 0u;
-		fence_after_sync();
-		constexpr uint32_t idesc = make_idesc_bf16(128, NG, 1, 1);
-		// A = X^T: rows (dy, chunk, ci % 8), 8-row groups XS_BYTES apart; K = 16 pixels, LBO = 8 pixels.
-		const uint64_t xb = make_sdesc(smem_addr(s_x), 128, XS_BYTES);
-		// B = G^T: columns co, 8-column groups XS_BYTES apart; the same 16 pixels.
-		const uint64_t gb = make_sdesc(smem_addr(s_g), 128, XS_BYTES);
-		for (int rr = 0; rr < ROWS; ++rr)
+		constexpr uint32_t idesc = make_idesc_bf16(128, 2 * NG, 1, 1);
+		// A = X^T: rows (input row, chunk, ci % 8), 8-row groups CXS_BYTES apart; K = 16 pixels, LBO = 8 pixels.
+		const uint64_t xb = make_sdesc(smem_addr(s_x), 128, CXS_BYTES);
+		// B = G^T: columns (gradient row, co), 8-column groups CXS_BYTES apart; the same 16 pixels.
+		const uint64_t gb = make_sdesc(smem_addr(s_g), 128, CXS_BYTES);
+		for (int t = 0; t < WG_STEPS; ++t)
+		{
+			if (!mbar_wait_warp(&bars[t], 0, POLL_LIMIT)) ok = false;
+			if (!ok) continue; // every copy has to be waited for before the CTA may leave
+			fence_after_sync();
+#pragma unroll 2
 			for (int kc = 0; kc < TILE_X / 16; ++kc)
 #pragma unroll
 				for (int d = 0; d < 3; ++d)
-					mma_bf16(tmem + d * NG, xb + (((rr * C8X) * XS_BYTES + (d + 16 * kc) * 16) >> 4),
-						gb + (((rr * G8) * XS_BYTES + (1 + 16 * kc) * 16) >> 4), idesc, rr || kc ? 1u : 0u, issue);
-		mma_commit(&bars[1], issue);
+					mma_bf16(tmem + d * 2 * NG, xb + ((2 * t * X_ROW + (d + 16 * kc) * 16) >> 4),
+						gb + ((2 * t * G_ROW + (1 + 16 * kc) * 16) >> 4), idesc, t || kc ? 1u : 0u, issue);
+		}
+		mma_commit(&bars[WG_STEPS], issue);
 	}
 	// Bias gradient partials from the staged gradient rows (pixels 0..127 of the tile).
 	{
@@ -1193,40 +1182,55 @@ __global__ void __launch_bounds__(128) wgrad_kernel(WgradArgs a)
 		const int c8 = co / 8, e = co % 8;
 		float s = 0.0f;
 		for (int r = 0; r < ROWS; ++r)
-			for (int p = part; p < TILE_X; p += PARTS)
-				s += bf2f(*reinterpret_cast<const uint16_t*>(s_g + (r * G8 + c8) * XS_BYTES + (1 + p) * 16 + e * 2));
+		{
+			if (!mbar_wait_bounded(&bars[r / 2], 0, POLL_LIMIT)) ok = false;
+			if (ok)
+				for (int p = part; p < TILE_X; p += PARTS)
+					s += bf2f(*reinterpret_cast<const uint16_t*>(s_g + r * G_ROW + c8 * CXS_BYTES + (1 + p) * 16 + e * 2));
+		}
 		s_bias[tid] = s;
 	}
-	const bool done = mbar_wait_bounded(&bars[1], 0, POLL_LIMIT);
-	if (__syncthreads_or(!done))
-	{
-		if (tid == 0) atomicExch(a.error, 4);
-		mbar_wait_bounded(&bars[1], 0, POLL_LIMIT);
-		fence_before_sync();
-		__syncthreads();
-		fence_after_sync();
-		if (warp == 0) tmem_dealloc(tmem, TMEM_COLS);
-		return;
-	}
+	if (!mbar_wait_bounded(&bars[WG_STEPS], 0, POLL_LIMIT)) ok = false;
+	if (__syncthreads_or(!ok)) return false;
 	fence_after_sync();
-	constexpr uint32_t MR = wgrad_rows(C8X);
-	float* out = a.partial + size_t(blockIdx.x) * wgrad_partial_floats(C8X, NG);
+	// Input row i with gradient row j of a step is tap row dy = i - j: row (dy, chunk, ci % 8) of the sum is accumulator row
+	// m of the first gradient row and m + C8X * 8 of the second. Added in shared memory (the operands are no longer read),
+	// from where whole lines are written.
+	float* sums = reinterpret_cast<float*>(smem);
 	const uint32_t m = warp * 32 + lane;
 	const uint32_t lane_base = uint32_t(warp * 32) << 16;
-	for (int d = 0; d < 3 && warp * 32 < MR; ++d)
-	{
 #pragma unroll
-		for (int c8 = 0; c8 < G8; ++c8)
-		{
-			float t8[8];
-			tmem_ld8(tmem + lane_base + d * NG + c8 * 8, t8);
-			tmem_ld_wait();
-			if (m >= MR) continue;
-			float4* o = reinterpret_cast<float4*>(out + (size_t(d) * MR + m) * NG + c8 * 8);
-			o[0] = make_float4(t8[0], t8[1], t8[2], t8[3]);
-			o[1] = make_float4(t8[4], t8[5], t8[6], t8[7]);
-		}
+	for (int j = 0; j < 2; ++j)
+	{
+		const uint32_t row = m - j * C8X * 8; // of the sum; wraps for the rows below
+		if (warp * 32 < int(MR) + j * C8X * 8)
+#pragma unroll
+			for (int d = 0; d < 3; ++d)
+#pragma unroll
+				for (int c = 0; c < NG; c += 16)
+				{
+					float v[16];
+					tmem_ld(tmem + lane_base + (d * 2 + j) * NG + c, v);
+					tmem_ld_wait();
+					if (row >= MR) continue;
+					float4* o = reinterpret_cast<float4*>(sums + (d * MR + row) * LINE + c);
+#pragma unroll
+					for (int q = 0; q < 4; ++q)
+					{
+						float4 w = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+						if (j)
+						{
+							const float4 f = o[q];
+							w = make_float4(f.x + w.x, f.y + w.y, f.z + w.z, f.w + w.w);
+						}
+						o[q] = w;
+					}
+				}
+		__syncthreads();
 	}
+	float* out = a.partial + size_t(bid) * wgrad_partial_floats(C8X, NG);
+	for (uint32_t i = tid; i < 3 * MR * (NG / 4); i += 128)
+		reinterpret_cast<float4*>(out)[i] = *reinterpret_cast<const float4*>(sums + i / (NG / 4) * LINE + i % (NG / 4) * 4);
 	if (tid < NG)
 	{
 		constexpr int PARTS = 128 / NG;
@@ -1234,22 +1238,54 @@ __global__ void __launch_bounds__(128) wgrad_kernel(WgradArgs a)
 		for (int q = 0; q < PARTS; ++q) s += s_bias[q * NG + tid];
 		out[3 * MR * NG + tid] = s;
 	}
+	return true;
+}
+
+// The weight gradients of all four layers, ROWS rows of a crop and one layer per CTA, last layer first. Bound by the
+// rate of the MMAs (52 cycles each for 2 * NG <= 64 columns, whatever their number, so two gradient rows share one:
+// 48 per CTA instead of 96) and by loading, multiplying and storing one after the other in the two CTAs of an SM.
+// A training step of 16 crops took 163 us with a launch per layer between the input gradients and a copy per row
+// and chunk, 157 with one launch and whole rows, and takes 145 with two gradient rows per MMA.
+__global__ void __launch_bounds__(128, 2) wgrad_kernel(const __grid_constant__ WgradArgs a)
+{
+	extern __shared__ __align__(1024) unsigned char smem[];
+	uint64_t* bars = reinterpret_cast<uint64_t*>(smem + WgradSmem::BARS);
+	uint32_t* s_tmem = reinterpret_cast<uint32_t*>(smem + WgradSmem::TMEM);
+	const int warp = __shfl_sync(0xFFFFFFFFu, int(threadIdx.x >> 5), 0); // known to be the same in the whole warp
+	if (threadIdx.x == 0)
+	{
+		for (int i = 0; i <= WG_STEPS; ++i) mbar_init(&bars[i], 1);
+		fence_mbar_init();
+	}
+	if (warp == 0)
+	{
+		tmem_alloc(s_tmem, WG_TMEM_COLS);
+		tmem_relinquish();
+	}
+	fence_before_sync();
+	__syncthreads();
+	fence_after_sync();
+	const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, *s_tmem, 0);
+	pdl_trigger();
+	pdl_wait(); // the planes are written
+	const uint32_t l = NUM_LAYERS - 1 - blockIdx.x / a.blocks, bid = blockIdx.x % a.blocks;
+	static_assert(LAYERS[0].c8_in == 2 && LAYERS[0].n_out == 32 && LAYERS[1].c8_in == 4 && LAYERS[1].n_out == 32 &&
+			LAYERS[2].c8_in == 4 && LAYERS[2].n_out == 32 && LAYERS[3].c8_in == 4 && LAYERS[3].n_out == 16, "instances");
+	const bool ok = l == 3 ? wgrad_rows_block<4, 16>(a.layer[3], bid, smem, tmem)
+		: l == 0           ? wgrad_rows_block<2, 32>(a.layer[0], bid, smem, tmem)
+						   : wgrad_rows_block<4, 32>(a.layer[l], bid, smem, tmem);
+	if (!ok && threadIdx.x == 0) atomicExch(a.error, 3);
 	fence_before_sync();
 	__syncthreads();
 	if (warp == 0)
 	{
 		fence_after_sync();
-		tmem_dealloc(tmem, TMEM_COLS);
+		tmem_dealloc(tmem, WG_TMEM_COLS);
 	}
 }
 
-template <int C8X, int NG>
-__host__ __device__ constexpr uint32_t wgrad_smem_bytes()
-{
-	return (ROWS + 16 / C8X - 1) * C8X * XS_BYTES + ROWS * (NG / 8) * XS_BYTES + 32 + 512;
-}
+// ---- conversion, Adam, reduction ----
 
-// Input conversion: Color32 window of each crop -> chunk 0 of the row planes (b, g, r, 0...) / 255.
 __global__ void convert_input_kernel(const CropGpu* crops, Planes p)
 {
 	const uint32_t img = blockIdx.y;
@@ -1609,28 +1645,26 @@ int launch_conv(SwUpscaler* u, ConvArgs a, cudaStream_t s)
 constexpr uint32_t WGRAD_CTAS_PER_CROP =
 	(SW_UPSCALER_CROP_W + TILE_X - 1) / TILE_X * ((SW_UPSCALER_CROP_H + ROWS - 1) / ROWS);
 
-template <int C8X, int NG>
-int launch_wgrad(SwUpscaler* u, const Planes& x, const Planes& g, int layer, cudaStream_t s)
+int launch_wgrad(SwUpscaler* u, const Planes (&x)[NUM_LAYERS], const Planes (&g)[NUM_LAYERS], cudaStream_t s)
 {
 	WgradArgs a;
-	a.x = x;
-	a.g = g;
-	a.partial = static_cast<float*>(u->partial[layer].ptr);
-	a.tiles_x = (x.width + TILE_X - 1) / TILE_X;
-	a.row_blocks = (x.height + ROWS - 1) / ROWS;
-	a.error = static_cast<int*>(u->error.ptr);
-	constexpr uint32_t smem = wgrad_smem_bytes<C8X, NG>();
-	static bool configured[8] = {};
-	const int key = (C8X / 2 - 1) * 2 + (NG / 16 - 1);
-	if (!configured[key])
+	a.blocks = x[0].images * WGRAD_CTAS_PER_CROP;
+	for (int l = 0; l < NUM_LAYERS; ++l)
 	{
-		UP_CUDA(u, cudaFuncSetAttribute(wgrad_kernel<C8X, NG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-		configured[key] = true;
+		a.layer[l] = WgradLayer{x[l], g[l], static_cast<float*>(u->partial[l].ptr)};
+		if (x[l].chunks != uint32_t(LAYERS[l].c8_in) || g[l].chunks != uint32_t(LAYERS[l].n_out / 8) || x[l].wp != CXS || g[l].wp != CXS)
+			return fail(u, SW_ERR_KERNEL, "layer %d: planes of another shape", l);
+		if (size_t(a.blocks) * wgrad_partial_floats(LAYERS[l].c8_in, LAYERS[l].n_out) * 4 > u->partial[l].bytes)
+			return fail(u, SW_ERR_LIMIT, "weight-gradient partial buffer too small");
 	}
-	const uint32_t blocks = x.images * a.tiles_x * a.row_blocks; // images * WGRAD_CTAS_PER_CROP for training crops
-	if (size_t(blocks) * wgrad_partial_floats(C8X, NG) * 4 > u->partial[layer].bytes)
-		return fail(u, SW_ERR_LIMIT, "weight-gradient partial buffer too small");
-	UP_CUDA(u, launch_dependent(wgrad_kernel<C8X, NG>, dim3(blocks), dim3(128), smem, s, a));
+	a.error = static_cast<int*>(u->error.ptr);
+	static bool configured = false;
+	if (!configured)
+	{
+		UP_CUDA(u, cudaFuncSetAttribute(wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WgradSmem::TOTAL));
+		configured = true;
+	}
+	UP_CUDA(u, launch_dependent(wgrad_kernel, dim3(a.blocks * NUM_LAYERS), dim3(128), WgradSmem::TOTAL, s, a));
 	return SW_OK;
 }
 
@@ -1806,21 +1840,19 @@ int forward_backward(SwUpscaler* u, const SwUpscalerCrop* crops, uint32_t n, uin
 
 	const uint32_t count = n * (W - 2 * M) * (H - 2 * M) * 4 * 3;
 	*loss_count = count;
-	// layer 3 (32 -> 12): weight gradient, input gradient into G[2] masked by A[2]
-	if ((r = launch_wgrad<4, 16>(u, A[2], g4, 3, s))) return r;
+	// layer 3 (32 -> 12): input gradient into G[2] masked by A[2]
 	ConvArgs b{};
 	b.in = g4, b.out = G[2], b.mask = A[2], b.wpack = static_cast<uint16_t*>(u->wbwd[3].ptr);
 	if ((r = launch_conv<2, 32, EPI_MASK>(u, b, s))) return r;
 	// layer 2
-	if ((r = launch_wgrad<4, 32>(u, A[1], G[2], 2, s))) return r;
 	b.in = G[2], b.out = G[1], b.mask = A[1], b.wpack = static_cast<uint16_t*>(u->wbwd[2].ptr);
 	if ((r = launch_conv<4, 32, EPI_MASK>(u, b, s))) return r;
 	// layer 1
-	if ((r = launch_wgrad<4, 32>(u, A[0], G[1], 1, s))) return r;
 	b.in = G[1], b.out = G[0], b.mask = A[0], b.wpack = static_cast<uint16_t*>(u->wbwd[1].ptr);
 	if ((r = launch_conv<4, 32, EPI_MASK>(u, b, s))) return r;
-	// layer 0 (3 -> 32): weight gradient only
-	if ((r = launch_wgrad<2, 32>(u, x0, G[0], 0, s))) return r;
+	// the weight gradients of every layer; layer 0 (3 -> 32) has no other
+	const Planes wx[NUM_LAYERS] = {x0, A[0], A[1], A[2]}, wg[NUM_LAYERS] = {G[0], G[1], G[2], g4};
+	if ((r = launch_wgrad(u, wx, wg, s))) return r;
 	return SW_OK;
 }
 
