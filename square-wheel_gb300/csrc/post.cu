@@ -291,15 +291,21 @@ __global__ void __launch_bounds__(256) pp_downscale_kernel(PostArgs a)
 }
 
 // pp_blur_kernel: the separable blur of the downscaled bloom buffer, once per cell (perform_blur_impl,
-// postprocessor.rs:846-956): one block per BL_W x BL_H tile of cells stages its cells with a radius halo
+// postprocessor.rs:846-956): one block per tile of BL_W x blur_tile_lines cells stages its cells with a radius halo
 // on every side (source indices clamped to the buffer as the reference's blur clamps them), runs the
 // horizontal pass over every staged line and the vertical pass (bloom_scale folded into its weights)
 // over the tile, and writes the blurred cells to bloom1.
-constexpr uint32_t BL_W = 64, BL_H = 16;
+constexpr uint32_t BL_W = 64;
+
+// Lines of a tile: the more, the less of the horizontal pass is halo; the fewer, the more CTAs there are (a 2560x1440
+// frame at scale 4 has 230 tiles of 16 lines, which took 21.6-22.3 us with the rest of the postprocess, and 450 of 8:
+// 20.2; 1920x1080 at scale 2 with 510 and 1,020: 38.4 and 37.6 us a frame). From radius 9 on a tile of 8 would be
+// two thirds halo and more.
+__host__ __device__ __forceinline__ uint32_t blur_tile_lines(uint32_t radius) { return radius <= 8 ? 8 : 16; }
 
 __host__ __device__ __forceinline__ uint32_t blur_tile_smem(uint32_t radius)
 {
-	const uint32_t lines = BL_H + 2 * radius, cols = BL_W + 2 * radius;
+	const uint32_t lines = blur_tile_lines(radius) + 2 * radius, cols = BL_W + 2 * radius;
 	return (lines * cols + lines * BL_W) * 16u; // cells as four i32 lanes
 }
 
@@ -312,80 +318,86 @@ __device__ __forceinline__ int4 lanes_of(unsigned long long c)
 // A blur pass's result as the reference stores it: (sum >> 14) into a Colour64 lane, (v as u64).min(65535).
 __device__ __forceinline__ int32_t pass_lane(int32_t sum) { return int32_t(min(uint32_t(sum >> 14), 65535u)); }
 
+// Bound by its instructions: a thread keeps its column for every line, so no index is divided (with flat indices over the
+// tile's lines the divisions were a quarter of 244 instructions per cell).
 __global__ void __launch_bounds__(256) pp_blur_kernel(PostArgs a)
 {
 	extern __shared__ __align__(16) int4 s_cells[];
-	const uint32_t cx0 = blockIdx.x * BL_W, cy0 = blockIdx.y * BL_H;
-	pdl_wait(); // the downscale (the raster tile pass or pp_downscale_kernel) has completed
+	static_assert(BL_W == 64, "four lines of columns per step");
+	const uint32_t tile_lines = blur_tile_lines(a.radius);
+	const uint32_t cx0 = blockIdx.x * BL_W, cy0 = blockIdx.y * tile_lines;
 	const int32_t r = int32_t(a.radius);
-	const uint32_t cols = min(BL_W, a.bw - cx0), lines = min(BL_H, a.bh - cy0);
-	const uint32_t slines = lines + 2 * uint32_t(r), scols = cols + 2 * uint32_t(r);
-	int4* s_b = s_cells;                  // slines x scols downscaled cells, unpacked once
-	int4* s_h = s_b + slines * scols;     // slines x cols, horizontally blurred (already clamped lanes)
+	const uint32_t cols = min(BL_W, a.bw - cx0), lines = min(tile_lines, a.bh - cy0);
+	const uint32_t slines = lines + 2 * uint32_t(r), pitch = BL_W + 2 * uint32_t(r);
+	const uint32_t col = threadIdx.x % BL_W, line0 = threadIdx.x / BL_W;
+	int4* s_b = s_cells;              // slines x pitch downscaled cells, unpacked once
+	int4* s_h = s_b + slines * pitch; // slines x BL_W, horizontally blurred (already clamped lanes)
+	pdl_wait(); // the downscale (the raster tile pass or pp_downscale_kernel) has completed
 	{
-		// four loads in flight per thread; staged cell (l, c) is cell (clamp(cy0 - r + l), clamp(cx0 - r + c))
-		const uint32_t total = slines * scols;
+		// staged cell (l, c) is cell (clamp(cy0 - r + l), clamp(cx0 - r + c))
 		const unsigned long long* src = reinterpret_cast<const unsigned long long*>(a.bloom0);
-		for (uint32_t i0 = threadIdx.x; i0 < total; i0 += 4 * blockDim.x)
+		auto cell = [&](uint32_t l, uint32_t c) {
+			const int32_t by = min(max(int32_t(cy0) - r + int32_t(l), 0), int32_t(a.bh) - 1);
+			const int32_t bx = min(max(int32_t(cx0) - r + int32_t(c), 0), int32_t(a.bw) - 1);
+			return __ldg(src + uint32_t(by) * uint64_t(a.bw) + uint32_t(bx));
+		};
+		// the first 64 columns, four loads in flight per thread
+		for (uint32_t l0 = line0; l0 < slines; l0 += 16)
 		{
 			unsigned long long v[4];
 #pragma unroll
 			for (int k = 0; k < 4; ++k)
-			{
-				const uint32_t i = i0 + k * blockDim.x;
-				if (i < total)
-				{
-					const uint32_t l = i / scols, c = i % scols;
-					const int32_t by = min(max(int32_t(cy0) - r + int32_t(l), 0), int32_t(a.bh) - 1);
-					const int32_t bx = min(max(int32_t(cx0) - r + int32_t(c), 0), int32_t(a.bw) - 1);
-					v[k] = __ldg(src + uint64_t(by) * a.bw + uint32_t(bx));
-				}
-			}
+				if (l0 + k * 4 < slines) v[k] = cell(l0 + k * 4, col);
 #pragma unroll
 			for (int k = 0; k < 4; ++k)
-				if (i0 + k * blockDim.x < total) s_b[i0 + k * blockDim.x] = lanes_of(v[k]);
+				if (l0 + k * 4 < slines) s_b[(l0 + k * 4) * pitch + col] = lanes_of(v[k]);
 		}
+		// the 2 r (at most 32) columns behind them
+		const uint32_t c = threadIdx.x % 32;
+		if (c < 2 * uint32_t(r))
+			for (uint32_t l = threadIdx.x / 32; l < slines; l += 8) s_b[l * pitch + BL_W + c] = lanes_of(cell(l, BL_W + c));
 	}
 	__syncthreads();
 	// horizontal pass over every staged line: cell c of the tile sits at staged column c + r
-	for (uint32_t i = threadIdx.x; i < slines * cols; i += blockDim.x)
-	{
-		const uint32_t l = i / cols, c = i % cols;
-		const int4* line = s_b + l * scols + c + uint32_t(r);
-		const int4 cc = line[0];
-		const int32_t k0 = a.kernel_h[r];
-		int32_t s0 = wmul(cc.x, k0), s1 = wmul(cc.y, k0), s2 = wmul(cc.z, k0), s3 = wmul(cc.w, k0);
-		for (int32_t dx = 1; dx <= r; ++dx)
+	if (col < cols)
+		for (uint32_t l = line0; l < slines; l += 4)
 		{
-			const int4 c0 = line[-dx], c1 = line[dx];
-			const int32_t k = a.kernel_h[dx + r];
-			s0 = wadd(s0, wmul(wadd(c0.x, c1.x), k));
-			s1 = wadd(s1, wmul(wadd(c0.y, c1.y), k));
-			s2 = wadd(s2, wmul(wadd(c0.z, c1.z), k));
-			s3 = wadd(s3, wmul(wadd(c0.w, c1.w), k));
+			const int4* line = s_b + l * pitch + col + uint32_t(r);
+			const int4 cc = line[0];
+			const int32_t k0 = a.kernel_h[r];
+			int32_t s0 = wmul(cc.x, k0), s1 = wmul(cc.y, k0), s2 = wmul(cc.z, k0), s3 = wmul(cc.w, k0);
+			for (int32_t dx = 1; dx <= r; ++dx)
+			{
+				const int4 c0 = line[-dx], c1 = line[dx];
+				const int32_t k = a.kernel_h[dx + r];
+				s0 = wadd(s0, wmul(wadd(c0.x, c1.x), k));
+				s1 = wadd(s1, wmul(wadd(c0.y, c1.y), k));
+				s2 = wadd(s2, wmul(wadd(c0.z, c1.z), k));
+				s3 = wadd(s3, wmul(wadd(c0.w, c1.w), k));
+			}
+			s_h[l * BL_W + col] = make_int4(pass_lane(s0), pass_lane(s1), pass_lane(s2), pass_lane(s3));
 		}
-		s_h[i] = make_int4(pass_lane(s0), pass_lane(s1), pass_lane(s2), pass_lane(s3));
-	}
 	__syncthreads();
 	// vertical pass: line cy0 + l is staged at l + r
-	for (uint32_t i = threadIdx.x; i < lines * cols; i += blockDim.x)
-	{
-		const uint32_t l = i / cols, c = i % cols;
-		const int4 cc = s_h[(l + r) * cols + c];
-		const int32_t k0 = a.kernel_v[r];
-		int32_t s0 = wmul(cc.x, k0), s1 = wmul(cc.y, k0), s2 = wmul(cc.z, k0), s3 = wmul(cc.w, k0);
-		for (int32_t dy = 1; dy <= r; ++dy)
+	if (col < cols)
+		for (uint32_t l = line0; l < lines; l += 4)
 		{
-			const int4 c0 = s_h[(l + r - dy) * cols + c], c1 = s_h[(l + r + dy) * cols + c];
-			const int32_t k = a.kernel_v[dy + r];
-			s0 = wadd(s0, wmul(wadd(c0.x, c1.x), k));
-			s1 = wadd(s1, wmul(wadd(c0.y, c1.y), k));
-			s2 = wadd(s2, wmul(wadd(c0.z, c1.z), k));
-			s3 = wadd(s3, wmul(wadd(c0.w, c1.w), k));
+			const int4* at = s_h + (l + r) * BL_W + col;
+			const int4 cc = at[0];
+			const int32_t k0 = a.kernel_v[r];
+			int32_t s0 = wmul(cc.x, k0), s1 = wmul(cc.y, k0), s2 = wmul(cc.z, k0), s3 = wmul(cc.w, k0);
+			for (int32_t dy = 1; dy <= r; ++dy)
+			{
+				const int4 c0 = at[-dy * int32_t(BL_W)], c1 = at[dy * int32_t(BL_W)];
+				const int32_t k = a.kernel_v[dy + r];
+				s0 = wadd(s0, wmul(wadd(c0.x, c1.x), k));
+				s1 = wadd(s1, wmul(wadd(c0.y, c1.y), k));
+				s2 = wadd(s2, wmul(wadd(c0.z, c1.z), k));
+				s3 = wadd(s3, wmul(wadd(c0.w, c1.w), k));
+			}
+			a.bloom1[uint64_t(cy0 + l) * a.bw + cx0 + col] = uint64_t(uint32_t(pass_lane(s0))) | (uint64_t(uint32_t(pass_lane(s1))) << 16) |
+				(uint64_t(uint32_t(pass_lane(s2))) << 32) | (uint64_t(uint32_t(pass_lane(s3))) << 48);
 		}
-		a.bloom1[uint64_t(cy0 + l) * a.bw + cx0 + c] = uint64_t(uint32_t(pass_lane(s0))) | (uint64_t(uint32_t(pass_lane(s1))) << 16) |
-			(uint64_t(uint32_t(pass_lane(s2))) << 32) | (uint64_t(uint32_t(pass_lane(s3))) << 48);
-	}
 	pdl_trigger();
 }
 
@@ -634,7 +646,7 @@ int launch_bloom_pass(const PostArgs& a, cudaStream_t stream, bool downscale)
 	{
 		const uint32_t smem = blur_tile_smem(a.radius);
 		if (int e = allow_smem(pp_blur_kernel, smem)) return e;
-		const dim3 grid((a.bw + BL_W - 1) / BL_W, (a.bh + BL_H - 1) / BL_H);
+		const dim3 grid((a.bw + BL_W - 1) / BL_W, (a.bh + blur_tile_lines(a.radius) - 1) / blur_tile_lines(a.radius));
 		if (int e = int(launch_dependent(pp_blur_kernel, grid, dim3(256), smem, stream, a))) return e;
 		bloom = a.bloom1;
 	}
