@@ -11,13 +11,13 @@
 //     start and step of the mode's interpolants (the span setup of rasterizer.rs:329-422 / 513-556 /
 //     686-703), evaluated once per (draw, row) over the whole span with the frame as clip rectangle
 //     (the reference's num_threads == 1 ClipRect).
-//   raster_tiles: one 256-thread CTA per 64x16 tile, each thread a 1x4 pixel strip of one row; every warp
-//     works on its own two rows and never waits for the others. It streams over its bin's draws in submission
+//   raster_tiles: one 256-thread CTA per 64x32 tile (or another shape), each thread 8 of its pixels; every warp
+//     works on its own rows and never waits for the others. It streams over its bin's draws in submission
 //     order, 32 at a time: each lane tests one draw's box against the warp's rows and a ballot compacts the
-//     hits in order; the lanes then fetch the hits' rows and draw records together (16 hits a round trip) into
+//     hits in order; the lanes then fetch the hits' rows and draw records together (as many at a time as have a lane per row) into
 //     shared memory, and every thread walks the hits in order for its strip: for span pixel i it takes start +
 //     i*step (the reference's repeated wrapping addition), the per-pixel z division and the texel address,
-//     issues its four texel loads at once and blends them in submission order into registers. Blending order
+//     issues its texel loads at once and blends them in submission order into registers. Blending order
 //     is the reference's, the frame buffer is read and written once, and coverage and texel addresses are
 //     bit-exact.
 #include "sw_kernels.cuh"
@@ -1095,12 +1095,13 @@ struct TileShape
 {
 	int w, h, strip;
 };
-constexpr TileShape TILE_SHAPES[SW_RASTER_TILE_VARIANTS] = {{64, 16, 4}, {32, 32, 4}, {128, 8, 4}, {64, 32, 8}, {32, 16, 2}};
+constexpr TileShape TILE_SHAPES[SW_RASTER_TILE_VARIANTS] = {{64, 32, 8}, {32, 32, 4}, {128, 8, 4}, {64, 16, 4}, {32, 16, 2}};
 
 // Bound by latency: boxes -> row and draw records -> texels are three dependent round trips per tile, so what
 // counts is how many warps are in flight and that none waits for another (with the tile's draws compacted and staged
 // by the CTA between barriers, 26 KB of shared memory and four CTAs per SM, a pass over a sheet of 46.9 M colour64
-// pixels took 103 us more of 1,620, and a 1920x1080 frame 4 us more of 49). Six CTAs per SM (40 registers, a few bytes spilled) measured 1% faster than four.
+// pixels took 103 us more of 1,620, and a 1920x1080 frame 4 us more of 49). Five CTAs per SM spill: 1,042 us where four
+// take 980.
 template <class P, int TILE_W, int TILE_H, int STRIP>
 __global__ void __launch_bounds__(256, 4) raster_tiles_kernel(RasterArgs a)
 {
@@ -1710,10 +1711,20 @@ int launch_raster_tiles(const RasterArgs& args, uint32_t pixel_format, uint32_t 
 {
 	switch (variant)
 	{
-	case 0: launch_tiles_variant<0>(args, pixel_format, stream); break;
+	case 0:
+		// Untuned: a tile is a chain of dependent round trips, so a thread has eight pixels on it (a pass over 4,096
+		// surfaces and their 46.6 M pixels takes 980 us, with four 1,042; a 1920x1080 frame 37.0 and 37.8 us; 128 x 16
+		// and 32 x 64 tiles with eight 996 and 988 us, 64 x 64 with sixteen 1,158). Triangles lie in clusters, whose
+		// warps draw them one after another: half the rows per warp are faster there (3840x2160 with 2,363 draws, most
+		// of them triangles: 79 us, with eight pixels 109).
+		if (args.num_tri_vertices)
+			launch_tiles_variant<3>(args, pixel_format, stream);
+		else
+			launch_tiles_variant<0>(args, pixel_format, stream);
+		break;
+	case 3: launch_tiles_variant<0>(args, pixel_format, stream); break;
 	case 1: launch_tiles_variant<1>(args, pixel_format, stream); break;
 	case 2: launch_tiles_variant<2>(args, pixel_format, stream); break;
-	case 3: launch_tiles_variant<3>(args, pixel_format, stream); break;
 	case 4: launch_tiles_variant<4>(args, pixel_format, stream); break;
 	default: return int(cudaErrorInvalidValue);
 	}
