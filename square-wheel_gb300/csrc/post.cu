@@ -41,24 +41,27 @@ __device__ __forceinline__ CV tonemap(CV c, const PostArgs& a, float4 isc)
 // min(c / (c * inv_255 + inv_scale), 255), the quotient rounded once as __fdiv_rn rounds it. The byte only depends on
 // the quotient's integer part, so an approximate quotient decides it unless it lies next to an integer: the
 // approximate reciprocal is off by at most one unit in its last place and the product by half of one, 4.6e-5 for
-// quotients up to 256, and the rounded quotient by 8e-6; within 1e-4 of an integer (one lane in 5,000), or where the
-// divisor is no normal number, `unsure` is set and the caller divides exactly. 0 / x and saturated lanes need no
-// second look; an infinite quotient saturates as in the conversion of the exact one. c, inv_255, inv_scale >= 0.
-__device__ __forceinline__ uint32_t tonemap_byte(float c, float inv_255, float inv_scale, bool& unsure)
+// quotients up to 256, and the rounded quotient by 8e-6. `edge` collects the largest distance of a quotient from the
+// middle of its unit interval: above 0.4999 (one lane in 5,000) the caller divides exactly. Below 0.5 and above 255.5
+// nothing depends on the quotient, so it is clamped there; an infinite quotient saturates as in the conversion of the
+// exact one, an infinite divisor gives 0 both ways. c >= 0, tonemap_plain_factors.
+__device__ __forceinline__ uint32_t tonemap_byte(float c, float inv_255, float inv_scale, float& edge)
 {
 	const float den = mad2(c, inv_255, inv_scale);
 	float inv;
 	asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(den));
-	const float q = fminf(fmul(c, inv), 255.5f);
-	const float nearest = fsub(fadd(q, 8388608.0f), 8388608.0f); // q rounded to an integer (0 <= q < 2^22)
-	unsure = unsure || (fabsf(fsub(q, nearest)) < 1e-4f && c != 0.0f) || !(den >= 1.17549435e-38f);
-	return __float_as_uint(__fadd_rd(q, 8388608.0f));
+	const float q = fmaxf(fminf(fmul(c, inv), 255.5f), 0.5f);
+	const float t = __fadd_rd(q, 8388608.0f);
+	edge = fmaxf(edge, fabsf(fsub(q, fsub(t, 8388607.5f)))); // both differences are exact
+	return __float_as_uint(t);
 }
-// Whether the frame's factors allow tonemap_byte and an alpha of 255 (tonemap): always, but for odd modulations.
+// Whether the frame's factors allow tonemap_byte and an alpha of 255 (tonemap): always, but for odd modulations. Every
+// divisor is at least its inv_scale, a normal number then.
 __device__ __forceinline__ bool tonemap_plain_factors(const PostArgs& a, float4 isc)
 {
-	return a.inv_255[3] == 0.0f && isc.w == 0.0f && a.inv_255[0] >= 0.0f && a.inv_255[1] >= 0.0f && a.inv_255[2] >= 0.0f && isc.x >= 0.0f &&
-		isc.y >= 0.0f && isc.z >= 0.0f;
+	constexpr float NORMAL = 1.17549435e-38f, LARGEST = 3.402823466e+38f;
+	return a.inv_255[3] == 0.0f && isc.w == 0.0f && a.inv_255[0] >= 0.0f && a.inv_255[1] >= 0.0f && a.inv_255[2] >= 0.0f &&
+		a.inv_255[0] <= LARGEST && a.inv_255[1] <= LARGEST && a.inv_255[2] <= LARGEST && isc.x >= NORMAL && isc.y >= NORMAL && isc.z >= NORMAL;
 }
 
 // The three colour lanes of a Color64 as floats (2^23 + v is exact for 16 bits; no conversion unit).
@@ -78,15 +81,15 @@ __device__ __forceinline__ CV3 cv3_sma(CV3 a, float s, CV3 b) { return CV3{mad2(
 template <int N>
 __device__ __forceinline__ void tonemap_c32(const CV3 (&c)[N], const PostArgs& a, float4 isc, uint32_t (&o)[N])
 {
-	bool unsure = false;
+	float edge = 0.0f;
 #pragma unroll
 	for (int k = 0; k < N; ++k)
 	{
-		const uint32_t b = tonemap_byte(c[k].b, a.inv_255[0], isc.x, unsure), g = tonemap_byte(c[k].g, a.inv_255[1], isc.y, unsure),
-					   r = tonemap_byte(c[k].r, a.inv_255[2], isc.z, unsure);
+		const uint32_t b = tonemap_byte(c[k].b, a.inv_255[0], isc.x, edge), g = tonemap_byte(c[k].g, a.inv_255[1], isc.y, edge),
+					   r = tonemap_byte(c[k].r, a.inv_255[2], isc.z, edge);
 		o[k] = __byte_perm(__byte_perm(b, g, 0x0040), r, 0x0410) | 0xFF000000u;
 	}
-	if (unsure)
+	if (edge > 0.4999f)
 	{
 #pragma unroll
 		for (int k = 0; k < N; ++k) o[k] = cv_to_c32(tonemap(CV{c[k].b, c[k].g, c[k].r, 0.0f}, a, isc));
@@ -469,7 +472,7 @@ __device__ __forceinline__ void bloom_sum4(const PostArgs& a, const unsigned lon
 // (postprocessor.rs:346-726, :997-1024), 4 horizontally adjacent pixels per thread over the flat pixel
 // space (one 32-byte HDR load pair and one 16-byte store when the row width is a multiple of 4). Bound by its
 // arithmetic: with three IEEE divisions and up to 8 bloom cells per pixel, 2560x1440 with linear bloom at scale 4 took
-// 31.7 us under the profiler, now 21.8 us (44 MB); 1920x1080 with nearest bloom 10.2 us, now 10.0 us.
+// 31.7 us under the profiler, now 20.4 us (44 MB); 1920x1080 with nearest bloom takes 10.7 us.
 template <int S, bool LINEAR>
 __global__ void __launch_bounds__(256) pp_tonemap_bloom_kernel(PostArgs a, const uint64_t* bloom)
 {
