@@ -1716,12 +1716,19 @@ int launch_raster_tiles(const RasterArgs& args, uint32_t pixel_format, uint32_t 
 		// surfaces and their 46.6 M pixels takes 980 us, with four 1,042; a 1920x1080 frame 37.0 and 37.8 us; 128 x 16
 		// and 32 x 64 tiles with eight 996 and 988 us, 64 x 64 with sixteen 1,158). Triangles lie in clusters, whose
 		// warps draw them one after another: half the rows per warp are faster there (3840x2160 with 2,363 draws, most
-		// of them triangles: 79 us, with eight pixels 109).
-		if (args.num_tri_vertices)
+		// of them triangles: 79 us, with eight pixels 109). And a frame whose large tiles are less than the CTAs that
+		// fit at once (four per SM) is left with idle SMs (1366x768, 528 of 608: raster 20.4 us, 16.3 with small
+		// tiles; 640x480 frames one after another 31.3 us each, 28.2).
+	{
+		constexpr uint32_t RESIDENT = 152 * 4;
+		constexpr TileShape t = TILE_SHAPES[0];
+		const uint64_t tiles = uint64_t((args.width + t.w - 1) / t.w) * uint64_t((args.height + t.h - 1) / t.h);
+		if (args.num_tri_vertices || tiles < RESIDENT)
 			launch_tiles_variant<3>(args, pixel_format, stream);
 		else
 			launch_tiles_variant<0>(args, pixel_format, stream);
 		break;
+	}
 	case 3: launch_tiles_variant<0>(args, pixel_format, stream); break;
 	case 1: launch_tiles_variant<1>(args, pixel_format, stream); break;
 	case 2: launch_tiles_variant<2>(args, pixel_format, stream); break;

@@ -47,3 +47,22 @@ def test_frames_with_and_without_triangles(gpu_ok, w, h, shape):
             assert np.array_equal(want, got), f"{(want != got).sum()} pixels differ"
     finally:
         r.close()
+
+
+@pytest.mark.parametrize("w,h", [(1600, 768), (1600, 769), (1217, 1024)])
+def test_frames_around_a_wave_of_tiles(gpu_ok, w, h):
+    """600 large tiles (small ones are taken), 625 and 640."""
+    fmt = abi.SW_PIXEL_C32
+    arena, draws, verts = scenes.make_raster_scene(81, w, h, 30, blends=(0, 1, 2, 3, 4), pixel_format=fmt)
+    fp = gpu.frame_params(w, h, fmt, (0, 0, 0))
+    r = gpu.GpuRenderer(synth.BatchedSurfaces(seed=1, count=1, max_side=8).static_data())
+    try:
+        r.frame_begin(fp)
+        r.set_surfaces(arena)
+        r.submit_draws(draws, verts)
+        got, want = np.zeros((h, w), np.uint32), np.zeros((h, w), np.uint32)
+        r.render(got)
+        assert oracle.rasterize(draws, verts, arena, fp, want) == 0
+        assert np.array_equal(want, got), f"{(want != got).sum()} pixels differ"
+    finally:
+        r.close()
