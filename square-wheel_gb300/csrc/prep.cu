@@ -9,7 +9,7 @@
 // evaluates the host's per-polygon expressions (host/prep_math.h, compiled for the device without FMA
 // contraction and with IEEE division and square root) with the sequential loops turned into exact
 // lane-parallel equivalents. The serial parts of the reference - the running surface offset and the
-// submission order - become prefix sums in prep_compact_kernel: one CTA scans the
+// submission order - become prefix sums in the compaction kernels: a CTA scans the
 // candidates in allocation order (surface index, texel offset) and the drawn leafs' polygons in draw
 // order (draw index, first vertex, first row record), and writes the surface records, descriptors,
 // draws, vertices and row ranges the surface build and the rasteriser read, plus the counts they
