@@ -371,7 +371,7 @@ __device__ __forceinline__ CV shade_texel(const SurfaceKernelArgs& a, const Surf
 				mad2(tn.x, u_norm.z, mad2(tn.y, v_norm.z, fmul(tn.z, bnormal.z))));
 		}
 		V3 refl = mkv3(0.0f, 0.0f, 0.0f);
-		float refl_len2 = MIN_POSITIVE_VALUE;
+		float refl_len2 = 1.0f;
 		float sk = 0.0f, inv_rough = 0.0f;
 		if (spec != 0)
 		{
@@ -389,6 +389,17 @@ __device__ __forceinline__ CV shade_texel(const SurfaceKernelArgs& a, const Surf
 			const V3 to_light = v3sub(mkv3(L.position[0], L.position[1], L.position[2]), pos);
 			const float tl_len2 = fmaxf(v3dot(to_light, to_light), MIN_POSITIVE_VALUE);
 			const float sdf = fmul(light_shadow_factor(a, s.g->lights[li], to_light), fmaxf(fsub(inv_fast(tl_len2), L.inv_square_radius), 0.0f));
+			// A factor of 0 (the texel lies outside the light's radius or in its shadow) adds zeros, unless a factor beside
+			// it is infinite or NaN. Within these bounds none is: the diffuse cosine is below 1e27, the specular one below
+			// 1e36, its intensity at most the roughness' reciprocal (127 or infinite); the light's colour is finite. Such a
+			// light is left here: of 62.4 us for 512 colour32 surfaces with six lights each 23 went into lights, most of them
+			// out of reach; now 54.6. (A bound on the texel's values alone would be hoisted out of the loop into a register
+			// too many, and so would the test before the shadow's: 1.5% of the time of batches without lights.)
+			if (sdf == 0.0f && tl_len2 > 1e-18f && tl_len2 < 1e18f && fabsf(v3dot(normal, to_light)) < 1e18f)
+			{
+				const float len2 = fmul(refl_len2, tl_len2);
+				if (fabsf(v3dot(refl, to_light)) < 1e18f && len2 > 1e-36f && len2 < 1e36f && fabsf(fmul(inv_rough, tl_len2)) < 1e36f) continue;
+			}
 			float di = 0.0f;
 			if (spec != 2) di = fmaxf(fmul(v3dot(normal, to_light), inv_sqrt_fast(tl_len2)), 0.0f);
 			float si = 0.0f;
