@@ -5,8 +5,8 @@
 // 137-729, write_into_framebuffer :1511-1536).
 //
 // Two launches:
-//   raster_setup: one CTA per draw. Thread 0 runs the reference's edge walk (rasterizer.rs:160-270)
-//     into the draw's parts and derives its tile-binning box; then the CTA's threads take the draw's
+//   raster_setup: a CTA or a warp per draw. A warp runs the reference's edge walk (rasterizer.rs:160-270)
+//     into the draw's parts and derives its tile-binning box; then the draw's threads take its
 //     (row) records (row ranges and record offsets come from the host): the span [xs, xe) and the
 //     start and step of the mode's interpolants (the span setup of rasterizer.rs:329-422 / 513-556 /
 //     686-703), evaluated once per (draw, row) over the whole span with the frame as clip rectangle
@@ -14,8 +14,8 @@
 //   raster_tiles: one 256-thread CTA per 64x32 tile (or another shape), each thread 8 of its pixels; every warp
 //     works on its own rows and never waits for the others. It streams over its bin's draws in submission
 //     order, 32 at a time: each lane tests one draw's box against the warp's rows and a ballot compacts the
-//     hits in order; the lanes then fetch the hits' rows and draw records together (as many at a time as have a lane per row) into
-//     shared memory, and every thread walks the hits in order for its strip: for span pixel i it takes start +
+//     hits in order; the lanes then fetch the hits' rows and draw records together (as many at a time as
+//     have a lane per row) into shared memory, and every thread walks the hits in order for its strip: for span pixel i it takes start +
 //     i*step (the reference's repeated wrapping addition), the per-pixel z division and the texel address,
 //     issues its texel loads at once and blends them in submission order into registers. Blending order
 //     is the reference's, the frame buffer is read and written once, and coverage and texel addresses are
