@@ -15,9 +15,9 @@
 //     works on its own rows and never waits for the others. It streams over its bin's draws in submission
 //     order, 32 at a time: each lane tests one draw's box against the warp's rows and a ballot compacts the
 //     hits in order; the lanes then fetch the hits' rows and draw records together (as many at a time as
-//     have a lane per row) into shared memory, and every thread walks the hits in order for its strip: for span pixel i it takes start +
-//     i*step (the reference's repeated wrapping addition), the per-pixel z division and the texel address,
-//     issues its texel loads at once and blends them in submission order into registers. Blending order
+//     have a lane per row) into shared memory, and every thread walks the hits in order for its pixels: for span
+//     pixel i it takes start + i*step (the reference's repeated wrapping addition), the per-pixel z division and
+//     the texel address, issues its texel loads at once and blends them in submission order into registers. Blending order
 //     is the reference's, the frame buffer is read and written once, and coverage and texel addresses are
 //     bit-exact.
 #include "sw_kernels.cuh"
