@@ -410,8 +410,9 @@ int sw_submit_draws_ex(SwCtx* ctx, const SwDrawCmd* draws, uint32_t num_draws, c
 int sw_set_lite_textures(SwCtx* ctx, const uint32_t* pixels, uint64_t num_pixels);
 
 /* Rasterise the submitted draws (Renderer::draw_frame, renderer.rs:106-124) into the context's
- * framebuffer. If dst != NULL the frame (pixel_format of sw_frame_begin) is also copied there:
- * dst_is_device != 0 means a device pointer, otherwise host memory; pitch is in pixels. */
+ * framebuffer. If dst != NULL the frame (pixel_format of sw_frame_begin) is also written there:
+ * dst_is_device != 0 means a device pointer (any address cudaMemcpy2DAsync takes; memory of the context's
+ * device at a multiple of the pixel size needs no separate copy), otherwise host memory; pitch is in pixels. */
 int sw_render(SwCtx* ctx, void* dst, uint32_t pitch, int dst_is_device);
 
 /* Postprocessor::perform_postprocessing (src/square_wheel/postprocessor.rs:68-204) on the context's

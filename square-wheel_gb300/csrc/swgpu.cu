@@ -11,8 +11,12 @@
 //   (width*height pixels), bloom buffers and the exposure-average scratch.
 // Host->device uploads go through pinned staging buffers on the context's stream. Every descriptor is
 // validated on the host before launch so that no kernel can read outside its buffers.
+#include "launch_rules.h"
 #include "sw_kernels.cuh"
 #include "../host/prep_math.h"
+
+#include <cuda.h>
+#include <cudaTypedefs.h>
 
 #include "../../include/swlearn.h"
 
@@ -60,6 +64,7 @@ struct ViewGraphKey
 	uint32_t raster_tile, pixel_format, postprocess, dst_pitch;
 	void* dst;
 	int32_t dst_is_device;
+	uint32_t direct; // the tile pass stores to dst (stores_to)
 	uint32_t slot;
 	uint32_t in_flight; // the frame runs in flight with the next one (average event in the graph)
 };
@@ -272,11 +277,59 @@ RasterArgs raster_args(SwCtx* ctx)
 
 
 
-// A frame that ends with rasterisation and goes to device memory: the tile pass writes it there beside the frame
-// buffer (which the next frame and sw_postprocess read), instead of a copy that reads the frame buffer again.
-void frame_to_device(RasterArgs& a, void* dst, uint32_t pitch, int dst_is_device)
+uint32_t bpp_of(uint32_t format) { return format == SW_PIXEL_C64 ? 8u : 4u; }
+
+// A function of the driver (the same for every device), NULL where the driver has none of that name.
+template <class F>
+F driver_function(const char* name, unsigned version)
 {
-	if (!dst || !dst_is_device) return;
+	void* fn = nullptr;
+	cudaDriverEntryPointQueryResult q;
+	if (cudaGetDriverEntryPointByVersion(name, &fn, version, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
+		return reinterpret_cast<F>(fn);
+	cudaGetLastError();
+	return nullptr;
+}
+
+// What the driver knows about a caller's pointer (all false for memory it does not know).
+PointerInfo pointer_info(const void* ptr)
+{
+	PointerInfo info{};
+	static const auto query = driver_function<PFN_cuPointerGetAttributes_v7000>("cuPointerGetAttributes", 7000);
+	static const auto current = driver_function<PFN_cuCtxGetCurrent_v4000>("cuCtxGetCurrent", 4000);
+	if (!query || !current) return info;
+	CUpointer_attribute names[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED, CU_POINTER_ATTRIBUTE_ACCESS_FLAGS,
+		CU_POINTER_ATTRIBUTE_CONTEXT, CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+		CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+	uint32_t type = 0, managed = 0;
+	uint64_t access = 0, begin = 0, bytes = 0;
+	CUcontext owner = nullptr, ctx = nullptr;
+	int device = -1;
+	void* values[] = {&type, &managed, &access, &owner, &device, &begin, &bytes};
+	if (query(7, names, values, CUdeviceptr(reinterpret_cast<uintptr_t>(ptr))) != CUDA_SUCCESS || current(&ctx) != CUDA_SUCCESS) return info;
+	info.device_memory = type == CU_MEMORYTYPE_DEVICE;
+	info.managed = managed != 0;
+	info.writable = access == CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE;
+	info.own_context = !owner || owner == ctx;
+	info.device = device;
+	info.begin = begin;
+	info.bytes = bytes;
+	return info;
+}
+
+// Whether a frame that ends with rasterisation goes to a device destination that the tile pass can store to
+// (otherwise it is copied there).
+bool stores_to(SwCtx* ctx, const SwFrameParams& p, void* dst, uint32_t pitch, int dst_is_device)
+{
+	return dst && dst_is_device &&
+		can_store_frame(pointer_info(dst), ctx->device, uint64_t(reinterpret_cast<uintptr_t>(dst)), pitch, p.width, p.height,
+			bpp_of(p.pixel_format));
+}
+
+// The tile pass writes the frame to `dst` beside the frame buffer (which the next frame and sw_postprocess read), instead
+// of a copy that reads the frame buffer again.
+void frame_to_device(RasterArgs& a, void* dst, uint32_t pitch)
+{
 	a.out = dst;
 	a.out_pitch = pitch;
 }
@@ -525,8 +578,6 @@ int check_kernel(SwCtx* ctx, int launch_result, const char* what)
 		return fail(ctx, SW_ERR_CUDA, "%s launch failed: %s", what, cudaGetErrorString(cudaError_t(launch_result)));
 	return SW_OK;
 }
-
-uint32_t bpp_of(uint32_t format) { return format == SW_PIXEL_C64 ? 8u : 4u; }
 
 bool all_finite(const float* v, int n)
 {
@@ -1196,7 +1247,8 @@ int sw_render(SwCtx* ctx, void* dst, uint32_t pitch, int dst_is_device)
 		ctx->fb_valid = true;
 	}
 	RasterArgs a = raster_args(ctx);
-	frame_to_device(a, dst, pitch, dst_is_device);
+	const bool direct = stores_to(ctx, ctx->frame, dst, pitch, dst_is_device);
+	if (direct) frame_to_device(a, dst, pitch);
 	SW_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->ev_setup, 0));
 	stage_begin(ctx, STAGE_RASTER);
 	r = check_kernel(ctx, launch_raster_tiles(a, fmt, ctx->tuning.raster_tile, ctx->stream), "raster");
@@ -1205,7 +1257,7 @@ int sw_render(SwCtx* ctx, void* dst, uint32_t pitch, int dst_is_device)
 	SW_CUDA(ctx, cudaEventRecord(ctx->ev_tiles, ctx->stream));
 	ctx->tiles_recorded = true;
 	ctx->frame_open = false;
-	if (dst && !dst_is_device) return copy_out(ctx, dst, pitch, 0, ctx->framebuffer.ptr, w, w, h, bpp);
+	if (dst && !direct) return copy_out(ctx, dst, pitch, dst_is_device, ctx->framebuffer.ptr, w, w, h, bpp);
 	return SW_OK;
 }
 
@@ -1784,8 +1836,9 @@ int fuse_bloom_downscale(SwCtx* ctx, RasterArgs& ra, PostArgs& pa, cudaStream_t 
 // Recording average_ready inside a frame graph is an event record node.
 unsigned average_flags(const SwCtx* ctx) { return ctx->capturing ? cudaEventRecordExternal : cudaEventRecordDefault; }
 
+// `direct`: stores_to() of the frame's destination.
 int enqueue_frame(SwCtx* ctx, const SwFrameInput& f, const unsigned char* h, const size_t* off, uint64_t rows,
-	const PostArgs* post)
+	const PostArgs* post, bool direct)
 {
 	cudaStream_t s = ctx->stream, aux = ctx->aux;
 	// every per-frame array in one copy: the device buffer has the staging block's layout
@@ -1851,8 +1904,8 @@ int enqueue_frame(SwCtx* ctx, const SwFrameInput& f, const unsigned char* h, con
 		pp = *post;
 		if ((r = fuse_bloom_downscale(ctx, ra, pp, s))) return r;
 	}
-	else
-		frame_to_device(ra, f.dst, f.dst_pitch, f.dst_is_device);
+	else if (direct)
+		frame_to_device(ra, f.dst, f.dst_pitch);
 	stage_begin(ctx, STAGE_RASTER);
 	r = check_kernel(ctx, launch_raster_tiles(ra, f.params.pixel_format, ctx->tuning.raster_tile, s), "raster");
 	stage_end(ctx, STAGE_RASTER);
@@ -1866,6 +1919,8 @@ int enqueue_frame(SwCtx* ctx, const SwFrameInput& f, const unsigned char* h, con
 		stage_end(ctx, STAGE_POST);
 		if (r) return r;
 	}
+	else if (f.dst && f.dst_is_device && !direct)
+		return copy_out(ctx, f.dst, f.dst_pitch, 1, ctx->framebuffer.ptr, f.params.width, f.params.width, f.params.height, bpp);
 	return SW_OK;
 }
 } // namespace
@@ -2145,8 +2200,9 @@ int sw_draw_frame(SwCtx* ctx, const SwFrameInput* in)
 
 	// 3. capture the device work and update (or instantiate) the frame graph; with the graph off, the
 	// same work is launched directly (with per-stage timing events when timing is on)
+	const bool direct = !f.postprocess && stores_to(ctx, p, f.dst, f.dst_pitch, f.dst_is_device);
 	auto enqueue = [&]() {
-		return enqueue_frame(ctx, f, h, off, rows, f.postprocess ? &pa : nullptr);
+		return enqueue_frame(ctx, f, h, off, rows, f.postprocess ? &pa : nullptr, direct);
 	};
 	if (ctx->graph_enabled)
 	{
@@ -2576,6 +2632,8 @@ int sw_draw_frame_view(SwCtx* ctx, const SwViewFrameInput* in)
 	key.dst = f.dst;
 	key.dst_pitch = f.dst_pitch;
 	key.dst_is_device = f.dst_is_device;
+	// (asked on every call: the same address may be other memory now)
+	key.direct = !f.postprocess && stores_to(ctx, p, f.dst, f.dst_pitch, f.dst_is_device) ? 1u : 0u;
 	key.slot = slot;
 	key.in_flight = pslot >= 0 ? 1u : 0u;
 
@@ -2604,8 +2662,8 @@ int sw_draw_frame_view(SwCtx* ctx, const SwViewFrameInput* in)
 			{
 				if ((rr = fuse_bloom_downscale(ctx, ra2, pp2, s))) return rr;
 			}
-			else
-				frame_to_device(ra2, f.dst, f.dst_pitch, f.dst_is_device);
+			else if (key.direct)
+				frame_to_device(ra2, f.dst, f.dst_pitch);
 			if ((rr = check_kernel(ctx, launch_raster_tiles(ra2, p.pixel_format, ctx->tuning.raster_tile, s), "raster")))
 				return rr;
 			if (f.postprocess)
@@ -2615,6 +2673,9 @@ int sw_draw_frame_view(SwCtx* ctx, const SwViewFrameInput* in)
 						 "postprocess")))
 					return rr;
 			}
+			else if (f.dst && f.dst_is_device && !key.direct &&
+				(rr = copy_out(ctx, f.dst, f.dst_pitch, 1, ctx->framebuffer.ptr, p.width, p.width, p.height, bpp)))
+				return rr;
 			SW_CUDA(ctx, cudaMemcpyAsync(ctx->h_counts + slot, counts, sizeof(SwViewCounts), cudaMemcpyDeviceToHost, s));
 			return SW_OK;
 		};
