@@ -723,9 +723,8 @@ int sw_read_shadow_maps(SwCtx* ctx, float* dst, uint64_t max_texels);
 /* ---- launch configuration (no reference counterpart) ---- */
 #define SW_RASTER_TILE_VARIANTS 5
 typedef struct SwTuning {
-	/* tile shape of the tile pass, 256 threads each: 0 = 64x32 pixels (8 per thread), or 64x16 (4) in
-	 * frames with triangle draws and small frames, 1 = 32x32 (4), 2 = 128x8 (4), 3 = 64x32 (8),
-	 * 4 = 32x16 (2); all give the same frame */
+	/* tile shape of the tile pass, 256 threads each: 0 = 64x16 pixels (4 per thread), 1 = 32x32 (4), 2 = 128x8 (4),
+	 * 3 = 64x32 (4, twice), 4 = 32x16 (2); all give the same frame */
 	uint32_t raster_tile;
 	/* persistent grid of the surface build: blocks per SM, 1..64 */
 	uint32_t surface_blocks_per_sm;

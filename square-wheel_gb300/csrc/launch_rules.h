@@ -7,6 +7,15 @@
 namespace swgpu
 {
 
+// Tile shapes of the tile pass, as SwTuning.raster_tile numbers them: w x h pixels, 256 threads with `strip` pixels each
+// at a time, `passes` times one below the other. Every shape gives the same frame.
+struct TileShape
+{
+	int w, h, strip, passes;
+};
+constexpr uint32_t NUM_TILE_SHAPES = 5;
+constexpr TileShape TILE_SHAPES[NUM_TILE_SHAPES] = {{64, 16, 4, 1}, {32, 32, 4, 1}, {128, 8, 4, 1}, {64, 32, 4, 2}, {32, 16, 2, 1}};
+
 // What the driver reports about a pointer of the caller's.
 struct PointerInfo
 {

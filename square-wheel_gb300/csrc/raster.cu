@@ -11,7 +11,7 @@
 //     start and step of the mode's interpolants (the span setup of rasterizer.rs:329-422 / 513-556 /
 //     686-703), evaluated once per (draw, row) over the whole span with the frame as clip rectangle
 //     (the reference's num_threads == 1 ClipRect).
-//   raster_tiles: one 256-thread CTA per 64x32 tile (or another shape), each thread 8 of its pixels; every warp
+//   raster_tiles: one 256-thread CTA per 64x16 tile (or another shape), each thread 4 of its pixels; every warp
 //     works on its own rows and never waits for the others. It streams over its bin's draws in submission
 //     order, 32 at a time: each lane tests one draw's box against the warp's rows and a ballot compacts the
 //     hits in order; the lanes then fetch the hits' rows and draw records together (as many at a time as
@@ -20,6 +20,7 @@
 //     the texel address, issues its texel loads at once and blends them in submission order into registers. Blending order
 //     is the reference's, the frame buffer is read and written once, and coverage and texel addresses are
 //     bit-exact.
+#include "launch_rules.h"
 #include "sw_kernels.cuh"
 #include "warp_prep.cuh"
 
@@ -1089,20 +1090,17 @@ __device__ __forceinline__ void bloom_epilogue_s2(const RasterArgs& a, const uin
 	}
 }
 
-// Tile shapes of the tile pass (the autotuner's choice, SwTuning.raster_tile): TILE_W x TILE_H pixels,
-// 256 threads of STRIP pixels. Every shape gives the same frame.
-struct TileShape
-{
-	int w, h, strip;
-};
-constexpr TileShape TILE_SHAPES[SW_RASTER_TILE_VARIANTS] = {{64, 32, 8}, {32, 32, 4}, {128, 8, 4}, {64, 16, 4}, {32, 16, 2}};
+static_assert(NUM_TILE_SHAPES == SW_RASTER_TILE_VARIANTS, "tile shapes");
 
 // Bound by latency: boxes -> row and draw records -> texels are three dependent round trips per tile, so what
 // counts is how many warps are in flight and that none waits for another (with the tile's draws compacted and staged
 // by the CTA between barriers, 26 KB of shared memory and four CTAs per SM, a pass over a sheet of 46.9 M colour64
-// pixels took 103 us more of 1,620, and a 1920x1080 frame 4 us more of 49). Five CTAs per SM spill: 1,042 us where four
-// take 980.
-template <class P, int TILE_W, int TILE_H, int STRIP>
+// pixels took 103 us more of 1,620, and a 1920x1080 frame 4 us more of 49). A thread has four pixels: with eight the
+// sheet's frame takes 980 us where it takes 1,042, but the code of a draw, unrolled over a thread's pixels, is twice as
+// long and no longer fits the SM's first instruction cache together with other draws' modes and blends. 110 M pixel
+// writes by 4,000 overlapping draws of all modes and blends on 1920x1080 then take 1,560 us instead of 431, and 300 small
+// draws in one corner 55 us instead of 32.
+template <class P, int TILE_W, int TILE_H, int STRIP, int PASSES>
 __global__ void __launch_bounds__(256, 4) raster_tiles_kernel(RasterArgs a)
 {
 	static_assert((TILE_W / STRIP) * TILE_H == 256, "256 threads per tile");
@@ -1120,118 +1118,124 @@ __global__ void __launch_bounds__(256, 4) raster_tiles_kernel(RasterArgs a)
 
 	const int tiles_x = (a.width + TILE_W - 1) / TILE_W;
 	const int tx0 = int(blockIdx.x % tiles_x) * TILE_W;
-	const int ty0 = int(blockIdx.x / tiles_x) * TILE_H;
+	const int tile_y0 = int(blockIdx.x / tiles_x) * TILE_H * PASSES;
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	WarpShared& sw = reinterpret_cast<WarpShared*>(s_mem)[warp];
 	pdl_wait(); // the surface build (launched before this kernel) has completed
 	const int x0 = tx0 + lane; // the lane's first column
 	const int tx1 = min(tx0 + TILE_W, a.width);
-	const int wy0 = ty0 + warp * RPW, wy1 = min(wy0 + RPW, a.height); // the warp's rows
 
 	T* fb = static_cast<T*>(a.framebuffer);
 	const T* arena = static_cast<const T*>(a.arena);
 	const T* skybox = static_cast<const T*>(a.skybox);
-	T pix[STRIP];
 	// ColorVec::from_color_f32x3(&[32.0, 16.0, 8.0]).into(), partial_renderer.rs:255
 	const T background = P::FORMAT == SW_PIXEL_C64 ? T(8ull | (16ull << 16) | (32ull << 32)) : T(0x00201008u);
-#pragma unroll
-	for (int k = 0; k < STRIP; ++k)
-	{
-		pix[k] = T(0);
-		const int x = x0 + 32 * (k % PPR), y = wy0 + k / PPR;
-		if (x < a.width && y < a.height) pix[k] = a.clear_background ? background : fb[uint64_t(y) * uint32_t(a.width) + x];
-	}
 	unsigned int local_errors = 0, local_writes = 0;
 
-	// the draws to scan: the tile's bin's list (draw order; its first 32 draws' boxes lie beside it, so a short list
-	// costs one round trip), or every draw; lane i's draw of the 32 scanned next is fetched while the 32 before
-	// are drawn
-	const uint32_t* list = nullptr;
-	uint32_t list_len;
-	RasterBox next_box{0, 0, 0, 0, 0u, 0u};
-	auto fetch = [&](uint32_t k) {
-		next_box = RasterBox{0, 0, 0, 0, 0u, 0u};
-		if (k < list_len)
-		{
-			const uint32_t di = list ? list[k] : k;
-			next_box = a.boxes[di];
-			next_box.draw = di;
-		}
-	};
-	if (a.bin_lists)
+#pragma unroll 1
+	for (int pass = 0; pass < PASSES; ++pass)
 	{
-		const uint32_t bin = uint32_t(tx0 / RASTER_BIN_W) + uint32_t(ty0 / RASTER_BIN_H) * a.bins_x;
-		const RasterBox first = a.bin_first[bin * 32 + uint32_t(lane)];
-		list = a.bin_lists + uint64_t(bin) * a.bin_cap;
-		list_len = wy0 < wy1 ? a.bin_counts[bin] : 0u;
-		if (uint32_t(lane) < list_len) next_box = first;
-	}
-	else
-	{
-		list_len = wy0 < wy1 ? (a.counts ? a.counts->num_draws : a.num_draws) : 0u;
-		fetch(uint32_t(lane));
-	}
-	for (uint32_t chunk = 0; chunk < list_len; chunk += 32)
-	{
-		const RasterBox b = next_box;
-		if (chunk + 32 < list_len) fetch(chunk + 32 + uint32_t(lane));
-		// (an empty box is 0, 0, 0, 0)
-		const bool hit = b.x0 < tx1 && b.x1 > tx0 && b.y0 < wy1 && b.y1 > wy0;
-		const unsigned mask = __ballot_sync(0xFFFFFFFFu, hit);
-		if (!mask) continue;
-		if (hit)
-			sw.hit[__popc(mask & ((1u << lane) - 1u))] = make_uint4(b.draw, b.row_off, uint32_t(int32_t(b.y0)), uint32_t(int32_t(b.y1)));
-		__syncwarp();
-		const int total = __popc(mask);
-		for (int b0 = 0; b0 < total; b0 += BATCH)
-		{
-			const int n = min(BATCH, total - b0);
-			{
-				const int h = lane / RPW, r = lane % RPW;
-				if (h < n)
-				{
-					const uint4 e = sw.hit[b0 + h];
-					const int ry = wy0 + r;
-					RasterRow row;
-					row.xs = row.xe = 0;
-					if (ry >= int(e.z) && ry < int(e.w)) row = a.rows[e.y + uint32_t(ry)];
-					sw.row[h][r] = row;
-				}
-				if (lane < n) sw.rd[lane] = a.rdraws[sw.hit[b0 + lane].x];
-			}
-			__syncwarp();
-			for (int h = 0; h < n; ++h)
-			{
-				const RasterDraw& d = sw.rd[h];
-				if (d.mode == SW_RASTER_TRIANGLE)
-					triangle_pixels<P, TILE_W, STRIP>(a, d, sw.row[h], x0, pix, local_errors, local_writes);
-				else
-					polygon_pixels<P, TILE_W, STRIP>(d, sw.row[h], arena, skybox, x0, pix, local_errors, local_writes);
-			}
-			__syncwarp(); // the staged records are overwritten by the next batch or chunk
-		}
-	}
+		const int ty0 = tile_y0 + pass * TILE_H;
+		if (pass && ty0 >= a.height) break;
+		const int wy0 = ty0 + warp * RPW, wy1 = min(wy0 + RPW, a.height); // the warp's rows
+		T pix[STRIP];
 #pragma unroll
-	for (int k = 0; k < STRIP; ++k)
-	{
-		const int x = x0 + 32 * (k % PPR), y = wy0 + k / PPR;
-		if (x < a.width && y < a.height)
+		for (int k = 0; k < STRIP; ++k)
 		{
-			fb[uint64_t(y) * uint32_t(a.width) + x] = pix[k];
-			if (a.out) static_cast<T*>(a.out)[uint64_t(y) * a.out_pitch + x] = pix[k];
+			pix[k] = T(0);
+			const int x = x0 + 32 * (k % PPR), y = wy0 + k / PPR;
+			if (x < a.width && y < a.height) pix[k] = a.clear_background ? background : fb[uint64_t(y) * uint32_t(a.width) + x];
 		}
-	}
-	if constexpr (P::FORMAT == SW_PIXEL_C64)
-	{
-		if constexpr (RPW % 2 == 0)
+		// the draws to scan: the tile's bin's list (draw order; its first 32 draws' boxes lie beside it, so a short list
+		// costs one round trip), or every draw; lane i's draw of the 32 scanned next is fetched while the 32 before
+		// are drawn
+		const uint32_t* list = nullptr;
+		uint32_t list_len;
+		RasterBox next_box{0, 0, 0, 0, 0u, 0u};
+		auto fetch = [&](uint32_t k) {
+			next_box = RasterBox{0, 0, 0, 0, 0u, 0u};
+			if (k < list_len)
+			{
+				const uint32_t di = list ? list[k] : k;
+				next_box = a.boxes[di];
+				next_box.draw = di;
+			}
+		};
+		if (a.bin_lists)
 		{
-			if (a.bloom_scale == 2)
-				bloom_epilogue_s2<TILE_W, STRIP>(a, reinterpret_cast<const uint64_t*>(pix), tx0, wy0, lane);
+			const uint32_t bin = uint32_t(tx0 / RASTER_BIN_W) + uint32_t(ty0 / RASTER_BIN_H) * a.bins_x;
+			const RasterBox first = a.bin_first[bin * 32 + uint32_t(lane)];
+			list = a.bin_lists + uint64_t(bin) * a.bin_cap;
+			list_len = wy0 < wy1 ? a.bin_counts[bin] : 0u;
+			if (uint32_t(lane) < list_len) next_box = first;
+		}
+		else
+		{
+			list_len = wy0 < wy1 ? (a.counts ? a.counts->num_draws : a.num_draws) : 0u;
+			fetch(uint32_t(lane));
+		}
+		for (uint32_t chunk = 0; chunk < list_len; chunk += 32)
+		{
+			const RasterBox b = next_box;
+			if (chunk + 32 < list_len) fetch(chunk + 32 + uint32_t(lane));
+			// (an empty box is 0, 0, 0, 0)
+			const bool hit = b.x0 < tx1 && b.x1 > tx0 && b.y0 < wy1 && b.y1 > wy0;
+			const unsigned mask = __ballot_sync(0xFFFFFFFFu, hit);
+			if (!mask) continue;
+			if (hit)
+				sw.hit[__popc(mask & ((1u << lane) - 1u))] = make_uint4(b.draw, b.row_off, uint32_t(int32_t(b.y0)), uint32_t(int32_t(b.y1)));
+			__syncwarp();
+			const int total = __popc(mask);
+			for (int b0 = 0; b0 < total; b0 += BATCH)
+			{
+				const int n = min(BATCH, total - b0);
+				{
+					const int h = lane / RPW, r = lane % RPW;
+					if (h < n)
+					{
+						const uint4 e = sw.hit[b0 + h];
+						const int ry = wy0 + r;
+						RasterRow row;
+						row.xs = row.xe = 0;
+						if (ry >= int(e.z) && ry < int(e.w)) row = a.rows[e.y + uint32_t(ry)];
+						sw.row[h][r] = row;
+					}
+					if (lane < n) sw.rd[lane] = a.rdraws[sw.hit[b0 + lane].x];
+				}
+				__syncwarp();
+				for (int h = 0; h < n; ++h)
+				{
+					const RasterDraw& d = sw.rd[h];
+					if (d.mode == SW_RASTER_TRIANGLE)
+						triangle_pixels<P, TILE_W, STRIP>(a, d, sw.row[h], x0, pix, local_errors, local_writes);
+					else
+						polygon_pixels<P, TILE_W, STRIP>(d, sw.row[h], arena, skybox, x0, pix, local_errors, local_writes);
+				}
+				__syncwarp(); // the staged records are overwritten by the next batch or chunk
+			}
+		}
+#pragma unroll
+		for (int k = 0; k < STRIP; ++k)
+		{
+			const int x = x0 + 32 * (k % PPR), y = wy0 + k / PPR;
+			if (x < a.width && y < a.height)
+			{
+				fb[uint64_t(y) * uint32_t(a.width) + x] = pix[k];
+				if (a.out) static_cast<T*>(a.out)[uint64_t(y) * a.out_pitch + x] = pix[k];
+			}
+		}
+		if constexpr (P::FORMAT == SW_PIXEL_C64)
+		{
+			if constexpr (RPW % 2 == 0)
+			{
+				if (a.bloom_scale == 2)
+					bloom_epilogue_s2<TILE_W, STRIP>(a, reinterpret_cast<const uint64_t*>(pix), tx0, wy0, lane);
+				else if (a.bloom_scale)
+					bloom_epilogue<TILE_W, TILE_H, STRIP>(a, pix, tx0, ty0, tid, s_mem);
+			}
 			else if (a.bloom_scale)
 				bloom_epilogue<TILE_W, TILE_H, STRIP>(a, pix, tx0, ty0, tid, s_mem);
 		}
-		else if (a.bloom_scale)
-			bloom_epilogue<TILE_W, TILE_H, STRIP>(a, pix, tx0, ty0, tid, s_mem);
 	}
 	if (local_errors) atomicAdd(a.error_counter, local_errors);
 	// Pixel writes (span pixels processed) for the traffic accounting, one atomic per warp, spread over counters: on a
@@ -1621,9 +1625,9 @@ void launch_tiles_variant(const RasterArgs& args, uint32_t pixel_format, cudaStr
 	const unsigned tiles = unsigned(((args.width + t.w - 1) / t.w) * ((args.height + t.h - 1) / t.h));
 	if (tiles == 0) return;
 	if (pixel_format == SW_PIXEL_C64)
-		launch_dependent(raster_tiles_kernel<PixC64, t.w, t.h, t.strip>, dim3(tiles), dim3(256), 0, stream, args);
+		launch_dependent(raster_tiles_kernel<PixC64, t.w, t.h / t.passes, t.strip, t.passes>, dim3(tiles), dim3(256), 0, stream, args);
 	else
-		launch_dependent(raster_tiles_kernel<PixC32, t.w, t.h, t.strip>, dim3(tiles), dim3(256), 0, stream, args);
+		launch_dependent(raster_tiles_kernel<PixC32, t.w, t.h / t.passes, t.strip, t.passes>, dim3(tiles), dim3(256), 0, stream, args);
 }
 } // namespace
 
@@ -1711,27 +1715,10 @@ int launch_raster_tiles(const RasterArgs& args, uint32_t pixel_format, uint32_t 
 {
 	switch (variant)
 	{
-	case 0:
-		// Untuned: a tile is a chain of dependent round trips, so a thread has eight pixels on it (a pass over 4,096
-		// surfaces and their 46.6 M pixels takes 980 us, with four 1,042; a 1920x1080 frame 37.0 and 37.8 us; 128 x 16
-		// and 32 x 64 tiles with eight 996 and 988 us, 64 x 64 with sixteen 1,158). Triangles lie in clusters, whose
-		// warps draw them one after another: half the rows per warp are faster there (3840x2160 with 2,363 draws, most
-		// of them triangles: 79 us, with eight pixels 109). And a frame whose large tiles are less than the CTAs that
-		// fit at once (four per SM) is left with idle SMs (1366x768, 528 of 608: raster 20.4 us, 16.3 with small
-		// tiles; 640x480 frames one after another 31.3 us each, 28.2).
-	{
-		constexpr uint32_t RESIDENT = 152 * 4;
-		constexpr TileShape t = TILE_SHAPES[0];
-		const uint64_t tiles = uint64_t((args.width + t.w - 1) / t.w) * uint64_t((args.height + t.h - 1) / t.h);
-		if (args.num_tri_vertices || tiles < RESIDENT)
-			launch_tiles_variant<3>(args, pixel_format, stream);
-		else
-			launch_tiles_variant<0>(args, pixel_format, stream);
-		break;
-	}
-	case 3: launch_tiles_variant<0>(args, pixel_format, stream); break;
+	case 0: launch_tiles_variant<0>(args, pixel_format, stream); break;
 	case 1: launch_tiles_variant<1>(args, pixel_format, stream); break;
 	case 2: launch_tiles_variant<2>(args, pixel_format, stream); break;
+	case 3: launch_tiles_variant<3>(args, pixel_format, stream); break;
 	case 4: launch_tiles_variant<4>(args, pixel_format, stream); break;
 	default: return int(cudaErrorInvalidValue);
 	}

@@ -251,7 +251,6 @@ struct RasterArgs
 	uint64_t lite_texels;
 	const DrawRows* draw_rows;
 	uint32_t num_draws;
-	uint32_t num_tri_vertices;  // 0: no triangle draws
 	const SwViewCounts* counts; // GPU-side preparation: num_draws from here (else NULL)
 	uint32_t setup_blocks;      // with counts: raster setup CTAs, each striding over the draws
 	uint32_t total_rows; // row records of all draws

@@ -130,7 +130,7 @@ struct SwCtx
 	DevBuf lite; // sw_set_lite_textures: Color32 textures of triangle draws
 	uint64_t lite_texels = 0;
 	uint64_t num_rows = 0;
-	uint32_t num_draws = 0, num_tri_vertices = 0;
+	uint32_t num_draws = 0;
 	bool draws_valid = false;
 	DevBuf framebuffer;
 	uint32_t fb_width = 0, fb_height = 0, fb_format = SW_PIXEL_C32;
@@ -253,7 +253,6 @@ RasterArgs raster_args(SwCtx* ctx)
 	a.draw_rows = static_cast<const DrawRows*>(ctx->draw_rows.ptr);
 	a.total_rows = uint32_t(ctx->num_rows);
 	a.tri_vertices = static_cast<const SwTriVertex*>(ctx->tri_vertices.ptr);
-	a.num_tri_vertices = ctx->num_tri_vertices;
 	a.lite = static_cast<const uint32_t*>(ctx->lite.ptr);
 	a.lite_texels = ctx->lite_texels;
 	a.tri_steps = static_cast<TriSteps*>(ctx->tri_steps.ptr);
@@ -1217,7 +1216,6 @@ int sw_submit_draws_ex(SwCtx* ctx, const SwDrawCmd* draws, uint32_t num_draws, c
 	if ((r = staging_commit(ctx, ctx->stage_draw_rows, ctx->draw_rows.ptr, num_draws * sizeof(DrawRows), ctx->aux))) return r;
 	ctx->num_rows = row_acc;
 	ctx->num_draws = num_draws;
-	ctx->num_tri_vertices = num_tri_vertices;
 	const RasterArgs a = raster_args(ctx);
 	if ((r = check_kernel(ctx, launch_raster_setup(a, ctx->aux), "raster setup"))) return r;
 	if ((r = check_kernel(ctx, launch_raster_bins(a, ctx->aux), "raster bins"))) return r;
@@ -2184,7 +2182,6 @@ int sw_draw_frame(SwCtx* ctx, const SwFrameInput* in)
 	if ((r = ensure_framebuffer(ctx, p))) return r;
 	ctx->num_rows = rows;
 	ctx->num_draws = f.num_draws;
-	ctx->num_tri_vertices = f.num_tri_vertices;
 	PostArgs pa;
 	void* post_out = nullptr;
 	bool direct_host = false;
@@ -2616,7 +2613,6 @@ int sw_draw_frame_view(SwCtx* ctx, const SwViewFrameInput* in)
 	ra.boxes = reinterpret_cast<RasterBox*>(slab + vs.boxes);
 	ra.counts = counts;
 	ra.num_draws = 0;
-	ra.num_tri_vertices = 0; // the view's draws are polygons
 	ra.setup_blocks = uint32_t(ctx->num_sms) * 2;
 	ra.total_rows = 0;
 	if (f.postprocess)

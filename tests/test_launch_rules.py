@@ -15,6 +15,8 @@ extern "C" int store_frame(int device_memory, int managed, int writable, int own
 	const PointerInfo p{device_memory != 0, managed != 0, writable != 0, own_context != 0, memory_device, begin, bytes};
 	return can_store_frame(p, device, dst, pitch, width, height, bpp) ? 1 : 0;
 }
+extern "C" uint32_t num_shapes() { return NUM_TILE_SHAPES; }
+extern "C" void shape(uint32_t i, int* s) { s[0] = TILE_SHAPES[i].w, s[1] = TILE_SHAPES[i].h, s[2] = TILE_SHAPES[i].strip, s[3] = TILE_SHAPES[i].passes; }
 """
 
 
@@ -56,3 +58,14 @@ def test_device_destinations_that_kernels_store_to(rules, bpp):
             assert not _store(rules, size=dst - BASE + span - 1, **fits)
         assert not _store(rules, dst=BASE - bpp, size=1 << 45, pitch=pitch, width=width, height=height, bpp=bpp)
     assert not _store(rules, size=0, bpp=bpp)
+
+
+def test_tile_shapes_are_the_ones_the_tuning_names(rules):
+    """SwTuning.raster_tile's shapes; no thread has more than four pixels at a time (longer code is fetched more slowly than
+    it saves), and no bloom cell (up to 8 x 8 pixels) straddles two passes."""
+    sizes = [(64, 16), (32, 32), (128, 8), (64, 32), (32, 16)]
+    assert rules.num_shapes() == len(sizes)
+    s = (ctypes.c_int * 4)()
+    for i, (w, h) in enumerate(sizes):
+        rules.shape(i, s)
+        assert tuple(s[:2]) == (w, h) and s[2] <= 4 and 256 * s[2] * s[3] == w * h and h % s[3] == 0 and h // s[3] % 8 == 0
