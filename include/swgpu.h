@@ -728,8 +728,8 @@ typedef struct SwTuning {
 	uint32_t raster_tile;
 	/* persistent grid of the surface build: blocks per SM, 1..64 */
 	uint32_t surface_blocks_per_sm;
-	/* texels per surface-build thread and search, one in each of as many consecutive runs of 32: 1, or at
-	 * least 4 (0 = the default, 1; large batches take up to 8 either way) */
+	/* texels per surface-build thread and search, one in each of as many consecutive runs of 32: 1 or 4
+	 * (0, the default: 1, and up to 8 in batches of several million texels that the host submits) */
 	uint32_t surface_texels_per_thread;
 	uint32_t reserved;
 } SwTuning;

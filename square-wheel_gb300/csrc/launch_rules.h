@@ -2,6 +2,7 @@
 // plain C++, so that they can be checked over their whole range without a GPU.
 #pragma once
 
+#include <algorithm>
 #include <cstdint>
 
 namespace swgpu
@@ -15,6 +16,16 @@ struct TileShape
 };
 constexpr uint32_t NUM_TILE_SHAPES = 5;
 constexpr TileShape TILE_SHAPES[NUM_TILE_SHAPES] = {{64, 16, 4, 1}, {32, 32, 4, 1}, {128, 8, 4, 1}, {64, 32, 4, 2}, {32, 16, 2, 1}};
+
+// Runs of 32 texels that a warp of the surface build takes per search: the tuned number (SwTuning.surface_texels_per_thread,
+// 1 or 4), or with 0 by the work: one while the launch is not several times what the GPU holds at once (a frame's 0.6 M
+// texels hide latency by parallelism), up to 8 for large batches.
+inline uint32_t surface_runs(uint32_t tuned, uint64_t work, int num_sms)
+{
+	if (tuned) return tuned;
+	const uint64_t resident = uint64_t(num_sms) * 2048 * 2;
+	return uint32_t(std::min<uint64_t>(std::max<uint64_t>(work / resident, 1), 8));
+}
 
 // What the driver reports about a pointer of the caller's.
 struct PointerInfo

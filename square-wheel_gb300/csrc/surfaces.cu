@@ -15,6 +15,7 @@
 // surface rows (all but surfaces narrower than 17), the warp builds the line entries they touch together, one
 // component per lane from neighbouring floats, in shared memory, and each texel only mixes its two entries;
 // elsewhere, and for the three floats of a simple lightmap's element, every thread builds its two entries alone. Operations and their order are the reference's either way.
+#include "launch_rules.h"
 #include "sw_kernels.cuh"
 
 #include <cmath>
@@ -573,11 +574,7 @@ int launch_surface_build(const SurfaceKernelArgs& args, uint32_t pixel_format, i
 {
 	const uint64_t work = args.counts ? work_hint : args.total_work - args.work_begin;
 	if (work == 0 && !args.counts) return 0;
-	// Runs of 32 texels per warp and search: one while the launch is not several times what the GPU holds at once
-	// (a frame's 0.6 M texels hide latency by parallelism), up to 8 for large batches; at least 4 when tuned so.
-	const uint64_t resident = uint64_t(num_sms) * 2048 * 2;
-	uint64_t runs = std::min<uint64_t>(std::max<uint64_t>(work / resident, 1), 8);
-	if (texels_per_thread == 4) runs = std::max<uint64_t>(runs, 4);
+	const uint64_t runs = surface_runs(texels_per_thread, work, num_sms);
 	uint64_t blocks_needed = (work + 256 * runs - 1) / (256 * runs);
 	if (args.counts && blocks_needed < uint64_t(num_sms)) blocks_needed = uint64_t(num_sms);
 	// At most blocks_per_sm blocks per SM (several waves of resident blocks); large batches stride.

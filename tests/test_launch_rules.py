@@ -15,6 +15,7 @@ extern "C" int store_frame(int device_memory, int managed, int writable, int own
 	const PointerInfo p{device_memory != 0, managed != 0, writable != 0, own_context != 0, memory_device, begin, bytes};
 	return can_store_frame(p, device, dst, pitch, width, height, bpp) ? 1 : 0;
 }
+extern "C" uint32_t runs(uint32_t tuned, uint64_t work, int num_sms) { return surface_runs(tuned, work, num_sms); }
 extern "C" uint32_t num_shapes() { return NUM_TILE_SHAPES; }
 extern "C" void shape(uint32_t i, int* s) { s[0] = TILE_SHAPES[i].w, s[1] = TILE_SHAPES[i].h, s[2] = TILE_SHAPES[i].strip, s[3] = TILE_SHAPES[i].passes; }
 """
@@ -28,6 +29,7 @@ def rules(tmp_path_factory):
     subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-Werror", "-shared", "-fPIC", "-I", CSRC, str(src), "-o", str(lib)], check=True)
     so = ctypes.CDLL(str(lib))
     so.store_frame.argtypes = [ctypes.c_int] * 5 + [ctypes.c_uint64] * 2 + [ctypes.c_int, ctypes.c_uint64] + [ctypes.c_uint32] * 4
+    so.runs.argtypes = [ctypes.c_uint32, ctypes.c_uint64, ctypes.c_int]
     return so
 
 
@@ -69,3 +71,9 @@ def test_tile_shapes_are_the_ones_the_tuning_names(rules):
     for i, (w, h) in enumerate(sizes):
         rules.shape(i, s)
         assert tuple(s[:2]) == (w, h) and s[2] <= 4 and 256 * s[2] * s[3] == w * h and h % s[3] == 0 and h // s[3] % 8 == 0
+
+
+def test_tuned_surface_runs_are_what_they_say(rules):
+    for work in (1, 1 << 20, 1 << 26, 1 << 40):
+        assert rules.runs(1, work, 152) == 1 and rules.runs(4, work, 152) == 4
+    assert [rules.runs(0, w, 152) for w in (0, 1, 622592, 2 * 622592 - 1, 2 * 622592, 8 * 622592, 1 << 50)] == [1, 1, 1, 1, 2, 8, 8]
