@@ -1283,12 +1283,14 @@ __device__ __forceinline__ float depth_first_line(const RasterPart& p, float dx,
 	return fadd(fadd(fmul(float(p.y_start_int), dy), fmul(0.5f, fadd(dx, dy))), k);
 }
 
-// A part of at most this many texels (rows x widest row) is drawn by the warp that prepared it, one row per
-// lane; a larger one goes to the chunk list: a lane's row is a serial chain of as many steps as the row has
+// A part of at most this many texels (rows x widest row), or of no row this wide, is drawn by the warp that prepared it,
+// one row per lane; another goes to the chunk list: a lane's row is a serial chain of as many steps as the row has
 // texels, each an atomic on a sector of its own, and one warp would run a wall that fills a 1024 x 1024 map
 // alone. With the list a 1920x1080 frame with 4 shadowed lights and a projector takes 136 us instead of 146 us;
-// lines at 256, 512, 2048 and 4096 texels measured the same within 1%.
-constexpr uint32_t SHADOW_DIRECT_TEXELS = 1024;
+// lines at 256, 512, 2048 and 4096 texels measured the same within 1%. A chunk costs 32 columns whatever its width:
+// 900 draws of 1,000 rows take 82 us with the list and 42 without at 2 texels per row, 94 and 80 at 12, 104 and
+// 137 at 24 (5,000 of them 146 and 95, 412 and 375, 742 and 718).
+constexpr uint32_t SHADOW_DIRECT_TEXELS = 1024, SHADOW_LIST_WIDTH = 24;
 
 // The parts of one depth draw, by the warp that walked its edges (the same arguments in every lane). Rows go
 // to lanes 32 at a time: lane i takes the 32-row chunk's first line_inv_z and adds dy i times, which is the
@@ -1309,8 +1311,9 @@ __device__ __forceinline__ void emit_depth_parts(const RasterPart* parts, uint32
 		const int32_t w1 = min(wadd(pt.x_right0, wmul(last, pt.dx_dy_right)) >> 16, size) -
 			max(wadd(pt.x_left0, wmul(last, pt.dx_dy_left)) >> 16, 0);
 		const uint32_t n = (rows + 31) / 32;
+		const uint32_t widest = uint32_t(max(max(w0, w1), 0));
 		uint32_t at = list.capacity;
-		if (uint64_t(rows) * uint32_t(max(max(w0, w1), 0)) > SHADOW_DIRECT_TEXELS)
+		if (widest >= SHADOW_LIST_WIDTH && uint64_t(rows) * widest > SHADOW_DIRECT_TEXELS)
 		{
 			if (lane == 0) at = atomicAdd(list.count, n);
 			at = __shfl_sync(FULL_MASK, at, 0);
