@@ -27,6 +27,7 @@
 #include "../../include/swlearn.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -1509,6 +1510,11 @@ struct SwUpscaler
 	DevMem psnr_sum;
 	unsigned long long* h_psnr = nullptr;
 	cudaEvent_t ev = nullptr;
+	// Shared-memory opt-ins made on this upscaler's device (an attribute of the kernel on one device), and the
+	// convolutions' CTAs per SM with them (0: not yet). Concurrent first calls make them twice.
+	static constexpr int CONV_KEYS = 64;
+	std::atomic<int> conv_per_sm[CONV_KEYS] = {};
+	std::atomic<bool> wgrad_ready{false}, fused_ready{false};
 };
 
 namespace
@@ -1587,15 +1593,19 @@ size_t planes_bytes(uint32_t images, uint32_t width, uint32_t height, uint32_t c
 // x0 + 134), landing in shared memory as [chunk][136 pixels][8 channels].
 int make_row_map(SwUpscaler* u, const Planes& p, CUtensorMap* out)
 {
-	static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
-	if (!encode)
-	{
+	// the driver's function is the same for every device and thread
+	static const PFN_cuTensorMapEncodeTiled_v12000 encode = [] {
 		cudaDriverEntryPointQueryResult q;
 		void* fn = nullptr;
-		UP_CUDA(u, cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q));
-		if (q != cudaDriverEntryPointSuccess || !fn) return fail(u, SW_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
-		encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
-	}
+		if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+			q != cudaDriverEntryPointSuccess)
+		{
+			cudaGetLastError();
+			fn = nullptr;
+		}
+		return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
+	}();
+	if (!encode) return fail(u, SW_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
 	if (p.wp % 8) return fail(u, SW_ERR_KERNEL, "row planes: padded width %u not a multiple of 8", p.wp);
 	const cuuint64_t dims[4] = {64, p.wp / 8, p.chunks, cuuint64_t(p.images) * p.rows_alloc};
 	const cuuint64_t strides[3] = {128, cuuint64_t(p.wp) * 16, cuuint64_t(p.chunks) * p.wp * 16}; // bytes, dims 1..3
@@ -1619,9 +1629,10 @@ int launch_conv(SwUpscaler* u, ConvArgs a, cudaStream_t s)
 	if (r) return r;
 	constexpr uint32_t smem = conv_smem_bytes<C8, N>();
 	constexpr int tmem_cols = int(conv_tmem_cols<N>());
-	static int per_sm[64] = {};
-	const int key = (C8 / 2) * 16 + (N / 16) * 4 + EPI;
-	if (!per_sm[key])
+	constexpr int KEY = (C8 / 2) * 16 + (N / 16) * 4 + EPI;
+	static_assert(KEY < SwUpscaler::CONV_KEYS, "instances");
+	int per_sm = u->conv_per_sm[KEY].load(std::memory_order_relaxed);
+	if (!per_sm)
 	{
 		UP_CUDA(u, cudaFuncSetAttribute(conv_kernel<C8, N, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
 		UP_CUDA(u, cudaFuncSetAttribute(conv_kernel<C8, N, EPI>, cudaFuncAttributePreferredSharedMemoryCarveout,
@@ -1629,10 +1640,11 @@ int launch_conv(SwUpscaler* u, ConvArgs a, cudaStream_t s)
 		int smem_sm = 0;
 		UP_CUDA(u, cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, u->device));
 		const int by_smem = smem_sm / int(smem + 1024); // 1 KB reserved per CTA
-		per_sm[key] = std::max(1, std::min(by_smem, 512 / tmem_cols));
+		per_sm = std::max(1, std::min(by_smem, 512 / tmem_cols));
+		u->conv_per_sm[KEY].store(per_sm, std::memory_order_relaxed);
 	}
 	const uint32_t rows = a.in.images * ((a.in.width + TILE_X - 1) / TILE_X) * a.in.height;
-	const uint32_t blocks = std::max(1u, std::min(uint32_t(u->num_sms * per_sm[key]), (rows + 1) / 2));
+	const uint32_t blocks = std::max(1u, std::min(uint32_t(u->num_sms * per_sm), (rows + 1) / 2));
 	if (EPI == EPI_LOSS)
 	{
 		if (blocks * 4 > u->loss_partial.bytes) return fail(u, SW_ERR_LIMIT, "loss partial buffer too small");
@@ -1658,11 +1670,10 @@ int launch_wgrad(SwUpscaler* u, const Planes (&x)[NUM_LAYERS], const Planes (&g)
 			return fail(u, SW_ERR_LIMIT, "weight-gradient partial buffer too small");
 	}
 	a.error = static_cast<int*>(u->error.ptr);
-	static bool configured = false;
-	if (!configured)
+	if (!u->wgrad_ready.load(std::memory_order_relaxed))
 	{
 		UP_CUDA(u, cudaFuncSetAttribute(wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WgradSmem::TOTAL));
-		configured = true;
+		u->wgrad_ready.store(true, std::memory_order_relaxed);
 	}
 	UP_CUDA(u, launch_dependent(wgrad_kernel, dim3(a.blocks * NUM_LAYERS), dim3(128), WgradSmem::TOTAL, s, a));
 	return SW_OK;
@@ -2029,11 +2040,10 @@ int sw_upscaler_infer(SwUpscaler* u, const uint32_t* lo, uint32_t lo_width, uint
 	int r;
 	if (u->fused)
 	{
-		static bool configured = false;
-		if (!configured)
+		if (!u->fused_ready.load(std::memory_order_relaxed))
 		{
 			UP_CUDA(u, cudaFuncSetAttribute(fused_upscale_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FusedSmem::TOTAL));
-			configured = true;
+			u->fused_ready.store(true, std::memory_order_relaxed);
 		}
 		FusedArgs f;
 		f.lo = lo;
