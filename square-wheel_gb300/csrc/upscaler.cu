@@ -1213,19 +1213,22 @@ __device__ __forceinline__ bool wgrad_rows_block(const WgradLayer& a, uint32_t b
 					float v[16];
 					tmem_ld(tmem + lane_base + (d * 2 + j) * NG + c, v);
 					tmem_ld_wait();
-					if (row >= MR) continue;
-					float4* o = reinterpret_cast<float4*>(sums + (d * MR + row) * LINE + c);
-#pragma unroll
-					for (int q = 0; q < 4; ++q)
+					if (row < MR)
 					{
-						float4 w = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-						if (j)
+						float4* o = reinterpret_cast<float4*>(sums + (d * MR + row) * LINE + c);
+#pragma unroll
+						for (int q = 0; q < 4; ++q)
 						{
-							const float4 f = o[q];
-							w = make_float4(f.x + w.x, f.y + w.y, f.z + w.z, f.w + w.w);
+							float4 w = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+							if (j)
+							{
+								const float4 f = o[q];
+								w = make_float4(f.x + w.x, f.y + w.y, f.z + w.z, f.w + w.w);
+							}
+							o[q] = w;
 						}
-						o[q] = w;
 					}
+					__syncwarp(); // the next load of accumulators is the whole warp's
 				}
 		__syncthreads();
 	}

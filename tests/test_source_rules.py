@@ -21,3 +21,30 @@ def test_no_plain_static_variable_in_a_function(path):
     bad = [(i + 1, line.strip()) for i, line in enumerate(_code(path).split("\n"))
            if re.match(r"[\t ]+static (?!const|std::atomic|__device__|_assert)", line) and "(" not in line.split("=")[0].split("{")[0]]
     assert not bad, bad
+
+
+def _enclosing_loop(code, at):
+    """Text of the innermost braced loop body around an offset, up to it and after it."""
+    depth, i = 0, at
+    while i > 0:
+        i -= 1
+        if code[i] == "}":
+            depth += 1
+        elif code[i] == "{" and depth:
+            depth -= 1
+        elif code[i] == "{" and re.search(r"\b(for|while) \([^{}]*$", code[max(0, i - 200):i]):
+            break
+    end, depth = i, 0
+    while True:
+        depth += {"{": 1, "}": -1}.get(code[end], 0)
+        end += 1
+        if depth == 0 or end >= len(code):
+            return code[i:end]
+
+
+@pytest.mark.parametrize("path", [p for p in SOURCES if p.startswith("csrc")])
+def test_accumulators_are_loaded_by_converged_warps(path):
+    """tcgen05.ld is an instruction of the whole warp: no lane may skip ahead to a loop's next load on its own."""
+    code = _code(path)
+    for m in re.finditer(r"\bcontinue;", code):
+        assert "tmem_ld(" not in _enclosing_loop(code, m.start()), f"line {code[:m.start()].count(chr(10)) + 1}"
