@@ -834,7 +834,7 @@ __device__ __forceinline__ void triangle_pixels(const RasterArgs& a, const Raste
 					++errors;
 					ua = 0;
 				}
-				tex[j] = __ldg(base + ua);
+				tex[j] = base[ua];
 			}
 		}
 #pragma unroll

@@ -693,7 +693,7 @@ __device__ __forceinline__ void f0_load_row(const FusedArgs& a, int y, bool vali
 	for (int k = 0; k < F0_PX; ++k)
 	{
 		const int j = lane + 32 * k, x = c0 - 1 + j;
-		px[k] = row_in && j < CXS && x >= 0 && x < int(a.lo_w) ? __ldg(row + x) : 0u;
+		px[k] = row_in && j < CXS && x >= 0 && x < int(a.lo_w) ? row[x] : 0u;
 	}
 }
 
@@ -828,9 +828,9 @@ static_assert(FL<1>::SLOT == FL<2>::SLOT && FL<2>::SLOT == FL<3>::SLOT, "input r
 __device__ __forceinline__ void f3_load(const FusedArgs& a, int x, int y, uint32_t (&p)[3])
 {
 	const uint32_t* row = a.lo + size_t(min(max(y, 0), int(a.lo_h) - 1)) * a.lo_pitch;
-	p[0] = __ldg(row + max(x - 1, 0));
-	p[1] = __ldg(row + x);
-	p[2] = __ldg(row + min(x + 1, int(a.lo_w) - 1));
+	p[0] = row[max(x - 1, 0)];
+	p[1] = row[x];
+	p[2] = row[min(x + 1, int(a.lo_w) - 1)];
 }
 __device__ __forceinline__ void f3_upsample(const uint32_t (&p)[3], float (&h)[2][3])
 {
@@ -1428,7 +1428,7 @@ __global__ void __launch_bounds__(REDUCE_WARPS * 32) wgrad_reduce_kernel(const _
 	{
 		const float* p = a.partial[l] + off;
 #pragma unroll 8
-		for (uint32_t c = warp; c < a.num_ctas; c += REDUCE_WARPS) s += __ldg(p + size_t(c) * stride);
+		for (uint32_t c = warp; c < a.num_ctas; c += REDUCE_WARPS) s += p[size_t(c) * stride];
 	}
 	s_sum[warp][lane] = s;
 	__syncthreads();

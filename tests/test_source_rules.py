@@ -48,3 +48,41 @@ def test_accumulators_are_loaded_by_converged_warps(path):
     code = _code(path)
     for m in re.finditer(r"\bcontinue;", code):
         assert "tmem_ld(" not in _enclosing_loop(code, m.start()), f"line {code[:m.start()].count(chr(10)) + 1}"
+
+
+def _functions(code):
+    """Bodies of the device functions and kernels of a file by name (overloads together)."""
+    out = {}
+    for m in re.finditer(r"__(?:device|global)__[^;{}]*?\{", code):
+        name = re.search(r"(\w+)\s*\(", re.sub(r"__launch_bounds__\([^)]*\)|__align__\([^)]*\)", "", m.group()))
+        if not name:
+            continue
+        end, depth = m.end(), 1
+        while depth:
+            depth += {"{": 1, "}": -1}.get(code[end], 0)
+            end += 1
+        out[name.group(1)] = out.get(name.group(1), "") + code[m.end():end]
+    return out
+
+
+@pytest.mark.parametrize("path", [p for p in SOURCES if p.endswith(".cu")])
+def test_kernels_that_start_early_read_with_plain_loads(path):
+    """A kernel launched as a programmatic dependent starts while the one before still writes: what it reads is not read-only
+    for its whole lifetime, as the loads of __ldg (ld.global.nc) require."""
+    code = _code(path)
+    functions = {}
+    for f in [path] + [p for p in SOURCES if p.endswith(".cuh")]:
+        for name, body in _functions(_code(f)).items():
+            functions[name] = functions.get(name, "") + body
+    todo = re.findall(r"launch_dependent\((\w+)", code)
+    todo = [n for n in todo if n in functions]
+    seen = set()
+    while todo:
+        n = todo.pop()
+        if n in seen:
+            continue
+        seen.add(n)
+        assert "__ldg(" not in functions[n], n
+        todo += [c for c in set(re.findall(r"\b(\w+)\s*(?:<[^;{}()]*>)?\(", functions[n])) if c in functions]
+    if "launch_dependent(" in code and path != os.path.join("csrc", "sw_device.cuh"):
+        assert seen
