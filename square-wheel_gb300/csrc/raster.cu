@@ -561,9 +561,8 @@ __device__ RasterRow row_setup(const SwDrawCmd& d, const DrawEq& e, const Raster
 // so its extremes over a part are at the part's first and last rows) and the per-draw record of the tile kernel; then
 // every thread of the group sets up rows of the draw (its row records, numbered by the host in draw order).
 // Bound by latency: with one draw per CTA 304 draws are in flight, which is what a frame of a few hundred polygons of up
-// to a screen's height needs; 4,096 draws of 90 rows took 72 us that way and take 30 with a warp each, 2,363 with
-// triangles among them 97 and 42. At 512 draws a lone pass is 8% slower with a warp each (100 us against 92), although
-// overlapped passes gain 9%; at 300 a lone frame loses 11% and overlapped ones gain nothing.
+// to a screen's height needs; thousands of draws take a warp each (warp_per_draw; 4,096 draws of 90 rows take 30 us
+// instead of 72). With the draw count on the device the host cannot choose, and it is a CTA per draw.
 struct SetupShared
 {
 	__align__(8) SwDrawCmd d;
@@ -978,10 +977,8 @@ __global__ void __launch_bounds__(256) raster_bin_kernel(RasterArgs a)
 
 // The same with BIN_GROUP_X x BIN_GROUP_Y bins per CTA, one per warp, for frames of many bins: a chunk is tested against
 // the whole group, the few boxes that meet it are compacted in order into shared memory, and every warp takes its own
-// bin's from there. A CTA per bin is bound by reading every box for every bin from L2 (5,778 bins of 4,096 draws: 568 MB
-// in 60 us; 17 us in groups of eight); with 1,020 bins of 2,363 draws all bins' CTAs are resident at once, and the
-// second step costs more than the reads (9.7 us against 12.0).
-constexpr uint32_t BIN_GROUP_X = 4, BIN_GROUP_Y = 2, BIN_GROUPS_ABOVE = 152 * 8;
+// bin's from there (bins_in_groups).
+constexpr uint32_t BIN_GROUP_X = 4, BIN_GROUP_Y = 2;
 
 __global__ void __launch_bounds__(256) raster_bin_groups_kernel(RasterArgs a)
 {
@@ -1605,14 +1602,11 @@ int launch_shadow_rebase(unsigned long long* storage, uint64_t num_texels, cudaS
 
 int launch_raster_setup(const RasterArgs& args, cudaStream_t stream)
 {
-	// A CTA per draw while the CTAs fit on the GPU a few times over, else a warp per draw (both sides measured: the
-	// kernel's comment).
-	constexpr uint32_t WARP_DRAWS_FROM = 1024;
 	if (args.counts)
 	{
 		if (args.setup_blocks > 0) raster_setup_kernel<1><<<args.setup_blocks, 256, 0, stream>>>(args);
 	}
-	else if (args.num_draws >= WARP_DRAWS_FROM)
+	else if (warp_per_draw(args.num_draws))
 		raster_setup_kernel<8><<<(args.num_draws + 7) / 8, 256, 0, stream>>>(args);
 	else if (args.num_draws > 0)
 		raster_setup_kernel<1><<<args.num_draws, 256, 0, stream>>>(args);
@@ -1709,7 +1703,7 @@ int launch_raster_bins(const RasterArgs& args, cudaStream_t stream)
 {
 	if (!args.bin_lists) return 0;
 	const uint32_t bins = args.bins_x * args.bins_y;
-	if (bins <= BIN_GROUPS_ABOVE) return int(launch_dependent(raster_bin_kernel, dim3(bins), dim3(256), 0, stream, args));
+	if (!bins_in_groups(bins, args.num_sms)) return int(launch_dependent(raster_bin_kernel, dim3(bins), dim3(256), 0, stream, args));
 	const uint32_t groups = (args.bins_x + BIN_GROUP_X - 1) / BIN_GROUP_X * ((args.bins_y + BIN_GROUP_Y - 1) / BIN_GROUP_Y);
 	return int(launch_dependent(raster_bin_groups_kernel, dim3(groups), dim3(256), 0, stream, args));
 }

@@ -253,6 +253,7 @@ struct RasterArgs
 	uint32_t num_draws;
 	const SwViewCounts* counts; // GPU-side preparation: num_draws from here (else NULL)
 	uint32_t setup_blocks;      // with counts: raster setup CTAs, each striding over the draws
+	uint32_t num_sms;
 	uint32_t total_rows; // row records of all draws
 	int32_t width, height;
 	uint32_t clear_background;

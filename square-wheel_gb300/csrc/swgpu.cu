@@ -251,6 +251,7 @@ RasterArgs raster_args(SwCtx* ctx)
 	a.height = int32_t(ctx->frame.height);
 	a.clear_background = ctx->frame.clear_background;
 	a.draw_rows = static_cast<const DrawRows*>(ctx->draw_rows.ptr);
+	a.num_sms = uint32_t(ctx->num_sms);
 	a.total_rows = uint32_t(ctx->num_rows);
 	a.tri_vertices = static_cast<const SwTriVertex*>(ctx->tri_vertices.ptr);
 	a.lite = static_cast<const uint32_t*>(ctx->lite.ptr);

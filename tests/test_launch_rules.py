@@ -16,6 +16,8 @@ extern "C" int store_frame(int device_memory, int managed, int writable, int own
 	return can_store_frame(p, device, dst, pitch, width, height, bpp) ? 1 : 0;
 }
 extern "C" uint32_t runs(uint32_t tuned, uint64_t work, int num_sms) { return surface_runs(tuned, work, num_sms); }
+extern "C" int groups(uint32_t bins, uint32_t num_sms) { return bins_in_groups(bins, num_sms) ? 1 : 0; }
+extern "C" int warp_draws(uint32_t draws) { return warp_per_draw(draws) ? 1 : 0; }
 extern "C" uint32_t num_shapes() { return NUM_TILE_SHAPES; }
 extern "C" void shape(uint32_t i, int* s) { s[0] = TILE_SHAPES[i].w, s[1] = TILE_SHAPES[i].h, s[2] = TILE_SHAPES[i].strip, s[3] = TILE_SHAPES[i].passes; }
 """
@@ -77,3 +79,12 @@ def test_tuned_surface_runs_are_what_they_say(rules):
     for work in (1, 1 << 20, 1 << 26, 1 << 40):
         assert rules.runs(1, work, 152) == 1 and rules.runs(4, work, 152) == 4
     assert [rules.runs(0, w, 152) for w in (0, 1, 622592, 2 * 622592 - 1, 2 * 622592, 8 * 622592, 1 << 50)] == [1, 1, 1, 1, 2, 8, 8]
+
+
+def test_bins_go_to_groups_where_a_cta_each_does_not_fit(rules):
+    for num_sms in (1, 76, 132, 152, 160):
+        assert [rules.groups(n, num_sms) for n in (1, 8 * num_sms - 1, 8 * num_sms, 8 * num_sms + 1, 1 << 20)] == [0, 0, 0, 1, 1]
+
+
+def test_draws_get_a_warp_each_from_a_count_on(rules):
+    assert [rules.warp_draws(n) for n in (0, 1, 300, 1023, 1024, 1 << 20)] == [0, 0, 0, 0, 1, 1]
