@@ -301,10 +301,10 @@ __global__ void __launch_bounds__(256) pp_downscale_kernel(PostArgs a)
 // over the tile, and writes the blurred cells to bloom1.
 constexpr uint32_t BL_W = 64;
 
-// Lines of a tile: the more, the less of the horizontal pass is halo; the fewer, the more CTAs there are (a 2560x1440
-// frame at scale 4 has 230 tiles of 16 lines, which took 21.6-22.3 us with the rest of the postprocess, and 450 of 8:
-// 20.2; 1920x1080 at scale 2 with 510 and 1,020: 38.4 and 37.6 us a frame). From radius 9 on a tile of 8 would be
-// two thirds halo and more.
+// Lines of a tile: the more, the less of the horizontal pass is halo; the fewer, the more CTAs there are (the
+// postprocess of a 2560x1440 frame at scale 4 takes 7-10% longer with 230 tiles of 16 lines than with 450 of 8, a
+// 1920x1080 frame at scale 2 2% longer with 510 than with 1,020). From radius 9 on a tile of 8 would be two thirds
+// halo and more.
 __host__ __device__ __forceinline__ uint32_t blur_tile_lines(uint32_t radius) { return radius <= 8 ? 8 : 16; }
 
 __host__ __device__ __forceinline__ uint32_t blur_tile_smem(uint32_t radius)
@@ -472,8 +472,8 @@ __device__ __forceinline__ void bloom_sum4(const PostArgs& a, const unsigned lon
 // pp_tonemap_bloom_kernel: the HDR frame tonemapped with its nearest or linear bloom sample
 // (postprocessor.rs:346-726, :997-1024), 4 horizontally adjacent pixels per thread over the flat pixel
 // space (one 32-byte HDR load pair and one 16-byte store when the row width is a multiple of 4). Bound by its
-// arithmetic: with three IEEE divisions and up to 8 bloom cells per pixel, 2560x1440 with linear bloom at scale 4 took
-// 31.7 us under the profiler, now 20.4 us (44 MB); 1920x1080 with nearest bloom takes 10.7 us.
+// arithmetic: 2560x1440 with linear bloom at scale 4 (44 MB) takes 20.3 us under the profiler, 31.7 with three IEEE
+// divisions and up to 8 bloom cells per pixel; 1920x1080 with nearest bloom takes 10.5 us.
 template <int S, bool LINEAR>
 __global__ void __launch_bounds__(256) pp_tonemap_bloom_kernel(PostArgs a, const uint64_t* bloom)
 {

@@ -1091,8 +1091,8 @@ static_assert(NUM_TILE_SHAPES == SW_RASTER_TILE_VARIANTS, "tile shapes");
 
 // Bound by latency: boxes -> row and draw records -> texels are three dependent round trips per tile, so what
 // counts is how many warps are in flight and that none waits for another (with the tile's draws compacted and staged
-// by the CTA between barriers, 26 KB of shared memory and four CTAs per SM, a pass over a sheet of 46.9 M colour64
-// pixels took 103 us more of 1,620, and a 1920x1080 frame 4 us more of 49). A thread has four pixels: with eight the
+// by the CTA between barriers, 26 KB of shared memory and four CTAs per SM, a pass over 4,096 surfaces and their
+// 46.6 M colour64 pixels took 103 us longer, and a 1920x1080 frame 4 us longer). A thread has four pixels: with eight the
 // sheet's frame takes 980 us where it takes 1,042, but the code of a draw, unrolled over a thread's pixels, is twice as
 // long and no longer fits the SM's first instruction cache together with other draws' modes and blends. 110 M pixel
 // writes by 4,000 overlapping draws of all modes and blends on 1920x1080 then take 1,560 us instead of 431, and 300 small
@@ -1236,8 +1236,8 @@ __global__ void __launch_bounds__(256, 4) raster_tiles_kernel(RasterArgs a)
 	}
 	if (local_errors) atomicAdd(a.error_counter, local_errors);
 	// Pixel writes (span pixels processed) for the traffic accounting, one atomic per warp, spread over counters: on a
-	// single one they follow each other at 1.5 ns apiece, which alone set the time of a 46.9 M pixel pass (366,000
-	// warps: 532-566 us with one counter, 299 us with these).
+	// single one they follow each other at 1.5 ns apiece, which alone set the time of a 46.6 M pixel pass (366,000
+	// warps: 532-566 us with one counter, 300 us with these).
 	for (int o = 16; o > 0; o >>= 1) local_writes += __shfl_xor_sync(0xFFFFFFFFu, local_writes, o);
 	if (lane == 0 && local_writes)
 		atomicAdd(a.write_counters + (blockIdx.x % SW_WRITE_COUNTERS) * SW_WRITE_COUNTER_STRIDE, (unsigned long long)local_writes);
@@ -1283,7 +1283,7 @@ __device__ __forceinline__ float depth_first_line(const RasterPart& p, float dx,
 // A part of at most this many texels (rows x widest row), or of no row this wide, is drawn by the warp that prepared it,
 // one row per lane; another goes to the chunk list: a lane's row is a serial chain of as many steps as the row has
 // texels, each an atomic on a sector of its own, and one warp would run a wall that fills a 1024 x 1024 map
-// alone. With the list a 1920x1080 frame with 4 shadowed lights and a projector takes 136 us instead of 146 us;
+// alone. With the list a 1920x1080 frame with 4 shadowed lights and a projector takes 7% less time;
 // lines at 256, 512, 2048 and 4096 texels measured the same within 1%. A chunk costs 32 columns whatever its width:
 // 900 draws of 1,000 rows take 82 us with the list and 42 without at 2 texels per row, 94 and 80 at 12, 104 and
 // 137 at 24 (5,000 of them 146 and 95, 412 and 375, 742 and 718).

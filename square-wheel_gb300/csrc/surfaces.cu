@@ -393,8 +393,8 @@ __device__ __forceinline__ CV shade_texel(const SurfaceKernelArgs& a, const Surf
 			// A factor of 0 (the texel lies outside the light's radius or in its shadow) adds zeros, unless a factor beside
 			// it is infinite or NaN. Within these bounds none is: the diffuse cosine is below 1e27, the specular one below
 			// 1e36, its intensity at most the roughness' reciprocal (127 or infinite); the light's colour is finite. Such a
-			// light is left here: of 62.4 us for 512 colour32 surfaces with six lights each 23 went into lights, most of them
-			// out of reach; now 54.6. (A bound on the texel's values alone would be hoisted out of the loop into a register
+			// light is left here: 512 colour32 surfaces with six lights each, most of them out of reach, take 62 us without
+			// this, 23 of them for lights, and 55 with it. (A bound on the texel's values alone would be hoisted out of the loop into a register
 			// too many, and so would the test before the shadow's: 1.5% of the time of batches without lights.)
 			if (sdf == 0.0f && tl_len2 > 1e-18f && tl_len2 < 1e18f && fabsf(v3dot(normal, to_light)) < 1e18f)
 			{
@@ -460,11 +460,11 @@ __device__ __forceinline__ uint32_t find_surface(const uint64_t* prefix, uint32_
 	return lo;
 }
 
-// Bound by issue (78% of the slots): exact, unfused f32 shading and integer indexing, 500 instructions per 32 texels.
-// One launch over 4,096 surfaces of 4x4 to 512x512 texels (46.9 M texels, directional lightmaps, half of the
-// materials specular, colour64): 765 us, 61 Gtexel/s; 1,119 us and 628 instructions with two lightmap entries per
+// Bound by issue (78% of the slots): exact, unfused f32 shading and integer indexing, 534 instructions per 32 texels.
+// One launch over 4,096 surfaces of 4x4 to 512x512 texels (43.9 M texels, directional lightmaps, half of the
+// materials specular, colour64): 764 us, 57 Gtexel/s; 1,119 us and 628 instructions with two lightmap entries per
 // texel from global memory and a serial search per 32 texels. Four blocks per SM (64 registers, 44 bytes spilled):
-// three measured 8% slower, five 24% (spills).
+// three are 8% slower, five 24% (spills).
 template <class P, bool DIRECTIONAL>
 __global__ void __launch_bounds__(256, 4) surf_build_kernel(SurfaceKernelArgs a, uint32_t runs)
 {

@@ -318,8 +318,8 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, const EpiOperan
 // The issuing thread's own instruction latency bounds the MMA rate, so the common case (three
 // contributions, no ring wrap) is straight-line code with compile-time descriptor offsets.
 // At a training step's sizes a CTA has three or four rows, so the kernel is bound by the latency of one row's chain
-// (load, MMAs, epilogue). A training step of 16 crops took 181 us with all eight warps on one row and the operands
-// loaded after the accumulators, and takes 163 this way.
+// (load, MMAs, epilogue). With all eight warps on one row and the operands loaded after the accumulators a training
+// step of 16 crops (150 us) takes 18 us longer.
 // Every wait is bounded: on expiry the role stops, the error flag is set, and the CTA still waits for
 // its own MMAs and copies before freeing TMEM.
 constexpr int CONV_THREADS = 320;
@@ -1248,8 +1248,8 @@ __device__ __forceinline__ bool wgrad_rows_block(const WgradLayer& a, uint32_t b
 // The weight gradients of all four layers, ROWS rows of a crop and one layer per CTA, last layer first. Bound by the
 // rate of the MMAs (52 cycles each for 2 * NG <= 64 columns, whatever their number, so two gradient rows share one:
 // 48 per CTA instead of 96) and by loading, multiplying and storing one after the other in the two CTAs of an SM.
-// A training step of 16 crops took 163 us with a launch per layer between the input gradients and a copy per row
-// and chunk, 157 with one launch and whole rows, and takes 145 with two gradient rows per MMA.
+// 32 us for 16 crops, of a training step of 150; with a launch per layer between the input gradients and a copy per
+// row and chunk the step takes 6 us longer, and with one gradient row per MMA another 12.
 __global__ void __launch_bounds__(128, 2) wgrad_kernel(const __grid_constant__ WgradArgs a)
 {
 	extern __shared__ __align__(1024) unsigned char smem[];
@@ -1379,8 +1379,8 @@ __global__ void adam_pack_kernel(AdamArgs a)
 // a.update Adam and the repacking right after, one launch for the four layers. A block takes 32 neighbouring
 // accumulator columns, so a warp reads whole 128-byte lines of a partial; its eight warps take every eighth
 // partial and their sums are added in order, so the result does not depend on the run. Bound by reading the
-// partials from L2 (28 MB at 16 crops). The four sums with one thread per parameter, 256 dependent reads of 4
-// bytes from lines of their own, took 121 us of a 334 us step.
+// partials from L2 (28 MB at 16 crops): 10 us. With one thread per parameter, 256 dependent reads of 4 bytes
+// from lines of their own, the four sums took 121 us.
 struct ReduceArgs
 {
 	const float* partial[NUM_LAYERS];
